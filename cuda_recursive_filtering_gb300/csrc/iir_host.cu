@@ -30,6 +30,8 @@
 #include "iir_host_internal.h"
 #include "iir_params.h"
 #include "iir_registry.h"
+#include "iir_sweep.cuh"
+#include "iir_sweep.h"
 
 using namespace iirgb;
 
@@ -436,6 +438,14 @@ void host_staging_free(HostStaging* h) {
 
 }  // namespace iirhost
 
+// A sweep kernel of a plan: its tables on the device, decay and resident blocks.
+struct SweepPart {
+    const SweepKernel* k = nullptr;
+    float* d_tab = nullptr;
+    int lanes = 0;  // lanes that a state reaches
+    int resident = 0;
+};
+
 struct iir_plan {
     int device = 0;
     int kind = 0;
@@ -473,6 +483,10 @@ struct iir_plan {
     float4* d_tables_tiny = nullptr;
     int tiny_pieces = 0;
     size_t tiny_max_n = 0;
+    // State-sweep kernels (iir_sweep.cuh) of a filter that decays within a tile, the one for large
+    // signals first; empty: the lookback kernels above filter every signal.
+    std::vector<SweepPart> sweeps;
+    IirSweepParams sweep{};
 };
 
 namespace {
@@ -620,6 +634,8 @@ void plan_free(iir_plan* p) {
     if (p->d_tables_small) cudaFree(p->d_tables_small);
     if (p->d_tables_tiny) cudaFree(p->d_tables_tiny);
     if (p->d_fac) cudaFree(p->d_fac);
+    for (SweepPart& s : p->sweeps)
+        if (s.d_tab) cudaFree(s.d_tab);
     delete p;
 }
 
@@ -735,6 +751,43 @@ int plan_create_plr(iir_plan** out, const double* b, const double* a, int order,
         q.a[j] = static_cast<float>(a[j]);
     }
     *out = p;
+    return IIR_OK;
+}
+
+// Adds the plan's state-sweep kernels: those whose tiles cover the filter's decay.
+int plan_add_sweeps(iir_plan* p, const std::vector<SectionF32>& secs, double gain) {
+    if (tail_max_pieces() <= 0) return IIR_OK;  // the lookback everywhere
+    if (p->n_sections == 1 && (!pipeline_enabled() || std::getenv("IIR_GB300_SMALL_N"))) return IIR_OK;
+    const SweepFilter f = sweep_filter(secs.data(), p->n_sections, gain);
+    for (const SweepKernel* k : sweep_kernels(p->kind, p->n_sections)) {
+        SweepPart s;
+        s.k = k;
+        s.lanes = sweep_decay(f, k->span(), SWEEP_LANES);
+        if (s.lanes == 0) continue;
+        const std::vector<float> tab = sweep_tables(f, k->N, k->R);
+        int st = cuda_status(
+            cudaFuncSetAttribute(k->fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(k->smem)));
+        if (!st) st = cuda_status(cudaFuncSetAttribute(k->fn, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
+        int nb = 0;
+        if (!st) st = cuda_status(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k->fn, 32 * (k->warps + 1), k->smem));
+        if (!st && nb <= 0) st = IIR_ERR_UNSUPPORTED;
+        if (!st) st = cuda_status(cudaMalloc(&s.d_tab, tab.size() * sizeof(float)));
+        if (!st) st = cuda_status(cudaMemcpy(s.d_tab, tab.data(), tab.size() * sizeof(float), cudaMemcpyHostToDevice));
+        if (st) {
+            if (s.d_tab) cudaFree(s.d_tab);
+            return st;
+        }
+        s.resident = nb * p->sms;
+        p->sweeps.push_back(s);
+    }
+    IirSweepParams& q = p->sweep;
+    q.state = p->d_state;
+    q.gain = static_cast<float>(gain);
+    for (int s = 0; s < p->n_sections; ++s)
+        q.sec[s] = SweepSection{secs[s].b1, secs[s].b2, secs[s].a1, secs[s].a2};
+    // the first section's input is the raw sample: its FIR taps carry the gain
+    q.sec[0].b1 = static_cast<float>(gain * secs[0].b1);
+    q.sec[0].b2 = static_cast<float>(gain * secs[0].b2);
     return IIR_OK;
 }
 
@@ -903,6 +956,11 @@ int iir_plan_create(iir_plan** out, const float* sos, int n_sections, int kernel
     q.n_sections = n_sections;
     q.gain = static_cast<float>(gain);
     q.tail_pieces = pieces;
+    st = plan_add_sweeps(p, secs, gain);
+    if (st) {
+        plan_free(p);
+        return st;
+    }
     *out = p;
     return IIR_OK;
 }
@@ -918,6 +976,68 @@ int iir_plan_create_plr_ba(iir_plan** out, const double* b, const double* a, int
 
 namespace {
 
+// Tiles of a sweep kernel over n samples.
+size_t sweep_tile_count(const SweepPart& s, size_t n) {
+    const size_t tile = 32 * static_cast<size_t>(s.k->span());
+    return (n + tile - 1) / tile;
+}
+
+// From this many samples per SM on, a signal takes the large-signal sweep kernel (GB300, CUDA graph
+// replays, large / small kernel: order 8 11.3 / 8.9 us at 2^20 samples, 12.4 / 12.8 at 3e6, 20.1 / 22.7
+// at 2^23; order 16 17.7 / 13.2, 18.5 / 22.4, 32 / 39). Single sections below it keep their
+// one-block-per-chunk kernels (order 2: 8.7 us against 6.9 at 2^20, 9.5 against 10.7 at 3e6).
+constexpr size_t SWEEP_LARGE_PER_SM = 16384;
+
+// The sweep kernel for a signal of n samples, or null for a single section's small signal.
+const SweepPart* sweep_pick(const iir_plan* p, size_t n) {
+    if (n >= SWEEP_LARGE_PER_SM * static_cast<size_t>(p->sms)) return &p->sweeps.front();
+    return p->n_sections > 1 ? &p->sweeps.back() : nullptr;
+}
+
+int sweep_launch(iir_plan* p, const SweepPart& s, const float* x, float* y, size_t n, cudaStream_t stream) {
+    const size_t tiles = sweep_tile_count(s, n);
+    if (tiles > 0x7fffffffull) return IIR_ERR_TOO_LARGE;
+    IirSweepParams& q = p->sweep;
+    const int span = s.k->span();
+    const size_t rows = n / static_cast<size_t>(span);
+    q.x = x;
+    q.y = y;
+    q.n = static_cast<long long>(n);
+    q.tables = s.d_tab;
+    q.timeout_ns = p->timeout_ns;
+    q.ntiles = static_cast<unsigned>(tiles);
+    q.lanes = s.lanes;
+    q.rounds = 0;
+    while ((1 << q.rounds) < s.lanes) ++q.rounds;
+    const bool aligned = ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) & 15u) == 0;
+    q.use_tma = (aligned && rows < 0x7fffff00ull &&
+                 encode_rows_map(&q.tmap_x, x, static_cast<long long>(rows), span, 32, 32) &&
+                 encode_rows_map(&q.tmap_y, y, static_cast<long long>(rows), span, 32, 32))
+                    ? 1
+                    : 0;
+    // a block's first run takes its warps one tile each, after the tile ahead of the run
+    const size_t per = static_cast<size_t>(std::max(1, s.k->warps - 1));
+    const size_t grid = std::min((tiles + per - 1) / per, static_cast<size_t>(s.resident));
+    const size_t share = tiles / grid;
+    if (share < 16) {
+        q.run0 = static_cast<unsigned>((tiles + grid - 1) / grid);  // dealt out whole
+        q.run1 = 1;
+    } else if (p->n_sections <= 2) {
+        // Memory-bound: half is drawn, in short runs (order 2 at 2^27: 157.8 us; 3/4 of it dealt out
+        // 158.5; runs of 12: 160.6).
+        q.run0 = static_cast<unsigned>(share / 2);
+        q.run1 = 4;
+    } else {
+        // Bound by arithmetic, every run costing a tile's pass A: an eighth is drawn, in longer runs
+        // (order 8 at 2^25: 51.6 us; half drawn in runs of 4: 55.4; order 16: 95.6 against 106.1).
+        q.run0 = static_cast<unsigned>(share - share / 8);
+        q.run1 = 8;
+    }
+    void* args[] = {&q};
+    return cuda_status(cudaLaunchKernel(s.k->fn, dim3(static_cast<unsigned>(grid)), dim3(32 * (s.k->warps + 1)), args,
+                                        s.k->smem, stream));
+}
+
 // One launch of the plan over device buffers (arguments checked by the caller). zi: initial
 // state of a single-section pipeline plan (x[-2], x[-1], y[-2], y[-1]), or null for rest.
 int plan_launch(iir_plan* p, const float* x, float* y, size_t n, const float* zi, cudaStream_t stream) {
@@ -926,6 +1046,10 @@ int plan_launch(iir_plan* p, const float* x, float* y, size_t n, const float* zi
         p->withhold = -1;
         return st;
     }
+    // filters that decay within a tile's halo (a launch with an injected fault takes the lookback,
+    // whose carries it withholds)
+    if (!p->sweeps.empty() && !zi && p->withhold < 0)
+        if (const SweepPart* s = sweep_pick(p, n)) return sweep_launch(p, *s, x, y, n, stream);
     // the kernel for this signal: a single-section plan's small-signal kernel up to its limit
     // (a piece that starts from a carried state always takes the persistent schedule)
     const bool use_tiny = p->tiny && !zi && n <= p->tiny_max_n;

@@ -54,10 +54,10 @@ struct IirLaunchState {
     unsigned long long ticket;       // (epoch << 32) | ticket
     unsigned long long error;        // (epoch << 32) | status code of the first failure
     unsigned int done;               // persistent kernels: blocks of the launch that have exited
-    unsigned int pad0;
+    unsigned int runs;               // state-sweep kernels: runs drawn in this launch (iir_sweep.cuh)
     unsigned long long* host_error;  // host-mapped error word, or null
 };
-#define IIR_STATE_RESET_BYTES 24  // ticket, error, done, pad0
+#define IIR_STATE_RESET_BYTES 24  // ticket, error, done, runs
 
 struct IirSection {
     float b1, b2;           // FIR taps after b0 normalisation (b0 = 1)

@@ -1,0 +1,230 @@
+// iir_sweep.cu — PH kernels on the state-sweep schedule (iir_sweep.cuh) and the host's side of
+// that schedule: the tables of a filter, computed in FP64 from its float32 sections.
+#include "iir_sweep.cuh"
+
+#include <algorithm>
+#include <cmath>
+#include <mutex>
+
+#include "iir_sweep.h"
+
+namespace iirgb {
+
+template <int K, int N, int R, int W, int NB>
+__global__ void __launch_bounds__((W + 1) * 32) iir_ph_sweep_kernel(const __grid_constant__ IirSweepParams p) {
+    extern __shared__ __align__(1024) unsigned char smem[];
+    using G = SweepGeom<K, N, R>;
+    sweep_tiles<G, W, NB>(p, smem, [&](float* buf, int lane, auto& st, auto& xh) {
+        sweep_run_ph<G>(buf, p.sec, p.gain, lane, st, xh);
+    });
+}
+
+}  // namespace iirgb
+
+using namespace iirgb;
+
+namespace iirhost {
+
+namespace {
+
+template <int K, int N, int R, int W, int NB>
+void add(std::vector<SweepKernel>& v) {
+    v.push_back(SweepKernel{IIR_KIND_PH, K, N, R, W, reinterpret_cast<const void*>(iir_ph_sweep_kernel<K, N, R, W, NB>),
+                            sweep_smem<K, N, R>(NB, sizeof(SweepAux<NB, 2 * K>))});
+}
+
+template <int K>
+void add_sections(std::vector<SweepKernel>& v) {
+    // Large signals: 16 KB tiles, two warps per scheduler (7, 9 or 10 warps leave the schedulers uneven
+    // and 12 leave one buffer to load ahead: 5-10% slower), as many buffers as shared memory holds.
+    // Four sub-rows per lane give pass B two independent chains; from 5 sections on the registers and
+    // the joins of four sub-rows cost more than that (order 16 at 2^27: 337 us with two, 395 with four).
+    if constexpr (K <= 4) add<K, 32, 4, 8, 13>(v);
+    else add<K, 64, 2, 8, (K <= 6 ? 13 : 12)>(v);
+    // Small signals: short lane rows, so that the signal spreads over more SMs. (Single sections have
+    // their 32-row kernel there, which is faster up to 2^20 samples.)
+    if constexpr (K > 1) add<K, 32, 2, 4, 6>(v);
+}
+
+const std::vector<SweepKernel>& kernels() {
+    static const std::vector<SweepKernel> all = [] {
+        std::vector<SweepKernel> v;
+        add_sections<1>(v);
+        add_sections<2>(v);
+        add_sections<3>(v);
+        add_sections<4>(v);
+        add_sections<5>(v);
+        add_sections<6>(v);
+        add_sections<7>(v);
+        add_sections<8>(v);
+        return v;
+    }();
+    return all;
+}
+
+using Mat = std::vector<double>;  // D x D, row-major
+
+Mat mat_mul(const Mat& a, const Mat& b, int D) {
+    Mat r(static_cast<size_t>(D) * D, 0.0);
+    for (int i = 0; i < D; ++i)
+        for (int k = 0; k < D; ++k) {
+            const double aik = a[static_cast<size_t>(i) * D + k];
+            if (aik == 0.0) continue;
+            for (int j = 0; j < D; ++j) r[static_cast<size_t>(i) * D + j] += aik * b[static_cast<size_t>(k) * D + j];
+        }
+    return r;
+}
+
+Mat mat_pow(Mat x, int e, int D) {
+    Mat r(static_cast<size_t>(D) * D, 0.0);
+    for (int i = 0; i < D; ++i) r[static_cast<size_t>(i) * D + i] = 1.0;
+    for (; e; e >>= 1) {
+        if (e & 1) r = mat_mul(r, x, D);
+        if (e > 1) x = mat_mul(x, x, D);
+    }
+    return r;
+}
+
+// The kernels carry a section's state as (y[-1] - y[-2], y[-1]): a low cutoff's two outputs differ
+// by little, and it is the difference that the recurrence amplifies. 2x2 block (s, q) of a transition
+// of (y[-2], y[-1]) pairs, in that basis and in the kernels' column order.
+void put_block(std::vector<float>& t, size_t at, const Mat& m, int D, int s, int q) {
+    const double* r0 = m.data() + static_cast<size_t>(2 * s) * D + 2 * q;
+    const double* r1 = r0 + D;
+    // columns: a unit difference is (y[-2], y[-1]) = (-1, 0), a unit y[-1] is (1, 1)
+    const double d0 = -r0[0], d1 = -r1[0], u0 = r0[0] + r0[1], u1 = r1[0] + r1[1];
+    t[at] = static_cast<float>(d1 - d0);
+    t[at + 1] = static_cast<float>(d1);
+    t[at + 2] = static_cast<float>(u1 - u0);
+    t[at + 3] = static_cast<float>(u1);
+}
+
+// Response of every section's output to a unit sample entering section 0 after its FIR taps.
+std::vector<std::vector<double>> impulse_states(const std::vector<SectionF32>& secs, int len) {
+    const size_t K = secs.size();
+    std::vector<std::vector<double>> p(K, std::vector<double>(static_cast<size_t>(len), 0.0));
+    for (size_t s = 0; s < K; ++s) {
+        double y1 = 0.0, y2 = 0.0;
+        for (int n = 0; n < len; ++n) {
+            double w;
+            if (s == 0) {
+                w = n == 0 ? 1.0 : 0.0;
+            } else {
+                const std::vector<double>& x = p[s - 1];
+                w = x[n] + (n >= 1 ? secs[s].b1 * x[n - 1] : 0.0) + (n >= 2 ? secs[s].b2 * x[n - 2] : 0.0);
+            }
+            const double y = w + secs[s].a1 * y1 + secs[s].a2 * y2;
+            p[s][static_cast<size_t>(n)] = y;
+            y2 = y1;
+            y1 = y;
+        }
+    }
+    return p;
+}
+
+}  // namespace
+
+std::vector<const SweepKernel*> sweep_kernels(int kind, int K) {
+    std::vector<const SweepKernel*> r;
+    for (const SweepKernel& k : kernels())
+        if (k.kind == kind && k.K == K) r.push_back(&k);
+    return r;
+}
+
+SweepFilter sweep_filter(const SectionF32* secs, int K, double gain) {
+    SweepFilter f;
+    f.K = K;
+    f.gain = gain;
+    f.secs.assign(secs, secs + K);
+    const int D = 2 * K;
+    // state (y_s[n-2], y_s[n-1]) of every section, zero input: section s > 0 sees its predecessor's
+    // new output and history through its FIR taps
+    f.phi.assign(static_cast<size_t>(D) * D, 0.0);
+    std::vector<double> row(static_cast<size_t>(D)), prev(static_cast<size_t>(D), 0.0);
+    for (int s = 0; s < K; ++s) {
+        std::fill(row.begin(), row.end(), 0.0);
+        row[2 * s + 1] += secs[s].a1;
+        row[2 * s] += secs[s].a2;
+        if (s > 0) {
+            for (int j = 0; j < D; ++j) row[j] += prev[j];
+            row[2 * (s - 1) + 1] += secs[s].b1;
+            row[2 * (s - 1)] += secs[s].b2;
+        }
+        f.phi[static_cast<size_t>(2 * s) * D + 2 * s + 1] = 1.0;
+        for (int j = 0; j < D; ++j) f.phi[static_cast<size_t>(2 * s + 1) * D + j] = row[j];
+        prev = row;
+    }
+    // energy of every section's impulse response over the longest halo considered
+    const std::vector<std::vector<double>> p = impulse_states(f.secs, 4096);
+    f.scale.assign(static_cast<size_t>(K), 1.0);
+    for (int s = 0; s < K; ++s) {
+        double e = 0.0;
+        for (double v : p[static_cast<size_t>(s)]) e += v * v;
+        f.scale[static_cast<size_t>(s)] = std::sqrt(e);
+    }
+    return f;
+}
+
+int sweep_decay(const SweepFilter& f, int unit, int most) {
+    const int D = 2 * f.K;
+    for (double s : f.scale)
+        if (!std::isfinite(s) || !(s > 0.0)) return 0;
+    const Mat step = mat_pow(f.phi, unit, D);
+    Mat m = step;
+    for (int h = 1; h <= most; ++h) {
+        double norm = 0.0;
+        for (int i = 0; i < D; ++i) {
+            double r = 0.0;
+            for (int j = 0; j < D; ++j)
+                r += std::fabs(m[static_cast<size_t>(i) * D + j]) * f.scale[j / 2] / f.scale[i / 2];
+            norm = std::max(norm, r);
+        }
+        if (!std::isfinite(norm)) return 0;
+        if (norm <= 1e-10) return h;
+        m = mat_mul(m, step, D);
+    }
+    return 0;
+}
+
+std::vector<float> sweep_tables(const SweepFilter& f, int N, int R) {
+    const int K = f.K, D = 2 * K, span = N * R;
+    const std::vector<std::vector<double>> p = impulse_states(f.secs, N);
+    auto ps = [&](int s, int n) { return n >= 0 ? p[static_cast<size_t>(s)][static_cast<size_t>(n)] : 0.0; };
+    const double b1 = f.secs[0].b1, b2 = f.secs[0].b2, g = f.gain;
+    const int blocks = K * (K + 1) / 2;
+    const size_t t_h = static_cast<size_t>(D) * N, t_pn = (t_h + 2 * D + 3) & ~size_t(3),
+                 t_pl = t_pn + 4 * static_cast<size_t>(blocks);
+    std::vector<float> t(t_pl + 4 * static_cast<size_t>(SWEEP_LANES) * blocks, 0.f);
+    for (int s = 0; s < K; ++s) {
+        float* t0 = t.data() + static_cast<size_t>(2 * s) * N;  // y[N-1] - y[N-2]
+        float* t1 = t0 + N;                                      // y[N-1]
+        auto h = [&](int m) { return g * (ps(s, m) + b1 * ps(s, m - 1) + b2 * ps(s, m - 2)); };  // impulse response
+        for (int n = 0; n < N; ++n) {
+            const double y1 = h(N - 1 - n), y2 = h(N - 2 - n);
+            t0[n] = static_cast<float>(y1 - y2);
+            t1[n] = static_cast<float>(y1);
+        }
+        // (x[-2], x[-1]) reach the sub-row through section 0's FIR taps
+        auto h2 = [&](int m) { return g * b2 * ps(s, m); };
+        auto h1 = [&](int m) { return g * (b1 * ps(s, m) + b2 * ps(s, m - 1)); };
+        float* th = t.data() + t_h + 4 * s;
+        th[0] = static_cast<float>(h2(N - 1) - h2(N - 2));
+        th[1] = static_cast<float>(h1(N - 1) - h1(N - 2));
+        th[2] = static_cast<float>(h2(N - 1));
+        th[3] = static_cast<float>(h1(N - 1));
+    }
+    auto put = [&](size_t at, const Mat& m) {
+        for (int s = 0; s < K; ++s)
+            for (int q = 0; q <= s; ++q) put_block(t, at + 4 * static_cast<size_t>(s * (s + 1) / 2 + q), m, D, s, q);
+    };
+    put(t_pn, mat_pow(f.phi, N, D));
+    const Mat step = mat_pow(f.phi, span, D);
+    Mat pl = mat_pow(f.phi, 0, D);
+    for (int l = 0; l < SWEEP_LANES; ++l) {
+        put(t_pl + 4 * static_cast<size_t>(l) * blocks, pl);
+        pl = mat_mul(pl, step, D);
+    }
+    return t;
+}
+
+}  // namespace iirhost

@@ -1,0 +1,558 @@
+// iir_sweep.cuh — the state-sweep schedule: cascades whose state decays within a tile (a few
+// thousand samples), one warp per tile.
+//
+// A warp owns a tile of 32 lane rows, SPAN = R x N consecutive samples per lane, staged in shared
+// memory by TMA. The signal is swept twice:
+//   pass A  every lane computes, for each of its R sub-rows of N samples, the state of all K sections
+//           that the sub-row leaves behind when it starts from rest: 2K dot products of the N samples
+//           with impulse-response tables (2K multiply-adds per sample, no recurrence);
+//   scan    the sub-rows' states are joined inside the lane with Phi^N (Phi is the cascade's state
+//           transition, block lower triangular), then across the lanes with powers of Phi^SPAN;
+//   pass B  every sub-row runs the whole cascade once from its true state, all K sections in
+//           registers (4K multiply-adds per sample), and its output replaces the input.
+// One pass per section (iir_ph.cuh: zero-state filter, scan, correction folded into the next pass)
+// takes 7K operations per sample and a read and a write of shared memory per section; this takes
+// 6K, two reads and one write.
+//
+// The state before a tile is the end state of the tile before it, from rest: the planner takes this
+// schedule only if older state is by then below 1e-10 of the states' own scale (FP64). So there is
+// no lookback: blocks exchange nothing, the tiles of a block pass their end states through shared
+// memory. Filters that decay more slowly keep the lookback schedules.
+//
+// Arithmetic is packed: fma.rn.f32x2 issues two multiply-adds per lane, which leaves half of the
+// issue slots to the shared-memory accesses and shuffles (the FP32 rate is the same: 36 TFMA/s
+// measured either way). Pass A packs neighbouring samples (x and the tables come as pairs from
+// 16-byte loads), pass B two sub-rows.
+//
+// Bound by: memory up to 2 sections; above, by issue (27 instructions per sample at 4 sections, 17 of
+// them on the FMA pipe, which is 55% busy). Measured on GB300, butter(order, 0.1), CUDA graph replays,
+// against the kernels that this replaces (us, before -> after):
+//   order        2              4              8              16
+//   2^20     (small kernel kept) 8.8 -> 7.4   12.7 -> 8.9    21.0 -> 13.2
+//   2^23      18.2 -> 15.8   22.7 -> 16.9   31.4 -> 20.2   56.2 -> 34.4
+//   2^25      48.4 -> 44.4   59.3 -> 45.7   83.4 -> 51.6  152.1 -> 95.6
+//   2^27     163 -> 157.8   193 -> 158.2   284 -> 177.9   565 -> 345
+#pragma once
+#include "iir_pipe.cuh"
+
+namespace iirgb {
+
+// ------------------------------------------------------------------------------------
+// packed float pairs
+// ------------------------------------------------------------------------------------
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pack2(float a, float b) {
+    f32x2 d;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(a), "f"(b));
+    return d;
+}
+__device__ __forceinline__ void unpack2(f32x2 v, float& a, float& b) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+    f32x2 d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+
+// ------------------------------------------------------------------------------------
+// geometry and tables of one kernel: K sections, R sub-rows of N samples per lane
+// ------------------------------------------------------------------------------------
+// Most lanes that a state reaches: filters that take longer to decay keep the lookback schedules.
+constexpr int SWEEP_LANES = 32;
+
+template <int K_, int N_, int R_>
+struct SweepGeom {
+    static constexpr int K = K_, N = N_, R = R_, D = 2 * K_;
+    static constexpr int SPAN = N * R;
+    static constexpr int TILE = 32 * SPAN;
+    static constexpr uint32_t TILE_BYTES = TILE * 4u;
+    static_assert(N % 32 == 0 && R % 2 == 0, "sub-rows of whole 128-byte lines, in packed pairs");
+    static constexpr int BLOCKS = K * (K + 1) / 2;  // 2x2 blocks of a block lower triangular matrix
+    // table offsets in floats (iir_sweep.h: the host's copy of this layout)
+    static constexpr int T_A = 0;                     // [D][N] pass A
+    static constexpr int T_H = T_A + D * N;           // [D][2] response to (x[-2], x[-1])
+    static constexpr int T_PN = (T_H + 2 * D + 3) & ~3;  // [BLOCKS] Phi^N, columns (m00, m10, m01, m11)
+    static constexpr int T_PL = T_PN + 4 * BLOCKS;       // [SWEEP_LANES][BLOCKS] Phi^(SPAN l)
+    static constexpr int T_LEN = T_PL + 4 * SWEEP_LANES * BLOCKS;
+    static_assert(T_LEN % 4 == 0 && T_PN % 4 == 0, "16-byte table rows");
+};
+
+// Float index of sample n of lane row l in the tile buffer: SPAN / 32 planes of 32-sample columns,
+// a 128-byte line per lane, 16-byte units swizzled by the lane (the 128-byte TMA swizzle), so that
+// a warp's 16-byte accesses at one column fall on all banks.
+__device__ __forceinline__ int tile_at(int l, int n) {
+    return ((n >> 5) << 10) + (l << 5) + ((((n >> 2) & 7) ^ (l & 7)) << 2) + (n & 3);
+}
+
+// o += M v for one 2x2 block in column order: (o0, o1) += (m00, m10) v0 + (m01, m11) v1
+__device__ __forceinline__ f32x2 block_mad(const float* m, float v0, float v1, f32x2 o) {
+    const ulonglong2 c = *reinterpret_cast<const ulonglong2*>(m);
+    return fma2(c.y, pack2(v1, v1), fma2(c.x, pack2(v0, v0), o));
+}
+
+// y = M v + e for a block lower triangular matrix (blocks in row order, s = 0..K-1, q = 0..s)
+template <int K>
+__device__ __forceinline__ void tri_mad(const float* m, const float (&v)[2 * K], const float (&e)[2 * K],
+                                        float (&y)[2 * K]) {
+    float o[2 * K];
+#pragma unroll
+    for (int s = 0; s < K; ++s) {
+        f32x2 a = pack2(e[2 * s], e[2 * s + 1]);
+#pragma unroll
+        for (int q = 0; q <= s; ++q) a = block_mad(m + 4 * (s * (s + 1) / 2 + q), v[2 * q], v[2 * q + 1], a);
+        unpack2(a, o[2 * s], o[2 * s + 1]);
+    }
+#pragma unroll
+    for (int i = 0; i < 2 * K; ++i) y[i] = o[i];
+}
+
+// ------------------------------------------------------------------------------------
+// pass A: zero-state end states of the lane's R sub-rows, components [C0, C0 + C) of 2K
+// ------------------------------------------------------------------------------------
+template <class G, int C0, int C>
+__device__ __forceinline__ void sweep_dots(const float* buf, const float* tab, int lane, float (&e)[G::R][G::D]) {
+    constexpr int N = G::N, R = G::R;
+    f32x2 acc[R][C];
+#pragma unroll
+    for (int i = 0; i < R; ++i)
+#pragma unroll
+        for (int c = 0; c < C; ++c) acc[i][c] = 0ull;
+    const float* row = buf + (lane << 5);
+    const float* ta = tab + G::T_A + C0 * N;
+    const int l7 = lane & 7;
+#pragma unroll 4
+    for (int j = 0; j < N / 4; ++j) {
+        const float* at = row + ((j >> 3) << 10) + (((j & 7) ^ l7) << 2);
+        ulonglong2 x[R];
+#pragma unroll
+        for (int i = 0; i < R; ++i) x[i] = *reinterpret_cast<const ulonglong2*>(at + i * (N / 32) * 1024);
+#pragma unroll
+        for (int c = 0; c < C; ++c) {
+            const ulonglong2 t = *reinterpret_cast<const ulonglong2*>(ta + c * N + 4 * j);
+#pragma unroll
+            for (int i = 0; i < R; ++i) acc[i][c] = fma2(t.y, x[i].y, fma2(t.x, x[i].x, acc[i][c]));
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < R; ++i)
+#pragma unroll
+        for (int c = 0; c < C; ++c) {
+            float a, b;
+            unpack2(acc[i][c], a, b);
+            e[i][C0 + c] = a + b;
+        }
+}
+
+// Pass A of the whole tile: e[i] = zero-state end state of sub-row i, xh[i] = its input history
+// (x[-2], x[-1]); lane 0's history before the tile is (g2, g1).
+template <class G>
+__device__ __forceinline__ void sweep_ends(const float* buf, const float* tab, int lane, float g2, float g1,
+                                           float (&e)[G::R][G::D], float (&xh)[G::R][2]) {
+    constexpr int N = G::N, R = G::R, D = G::D;
+    if constexpr (D <= 8) {
+        sweep_dots<G, 0, D>(buf, tab, lane, e);
+    } else {
+        sweep_dots<G, 0, 8>(buf, tab, lane, e);
+        sweep_dots<G, 8, D - 8>(buf, tab, lane, e);
+    }
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+        if (i > 0 || lane > 0) {
+            const int at = i > 0 ? tile_at(lane, i * N - 2) : tile_at(lane - 1, G::SPAN - 2);
+            const float2 h = *reinterpret_cast<const float2*>(buf + at);
+            xh[i][0] = h.x;
+            xh[i][1] = h.y;
+        } else {
+            xh[i][0] = g2;
+            xh[i][1] = g1;
+        }
+#pragma unroll
+        for (int c = 0; c < D; ++c) {
+            const float2 t = *reinterpret_cast<const float2*>(tab + G::T_H + 2 * c);
+            e[i][c] = fmaf(t.y, xh[i][1], fmaf(t.x, xh[i][0], e[i][c]));
+        }
+    }
+}
+
+// The lane's end state from rest: its sub-rows joined with Phi^N.
+template <class G>
+__device__ __forceinline__ void sweep_join(const float* tab, const float (&e)[G::R][G::D], float (&f)[G::D]) {
+#pragma unroll
+    for (int c = 0; c < G::D; ++c) f[c] = e[0][c];
+#pragma unroll
+    for (int i = 1; i < G::R; ++i) tri_mad<G::K>(tab + G::T_PN, f, e[i], f);
+}
+
+// Scan across the lanes from rest before the tile: S = the state before the lane, last = the state
+// after it (lane 31: the tile's end state), from the lanes' zero-state end states f. Kogge-Stone with
+// the whole state vector per step: a section-by-section scan takes K times as many dependent
+// shuffles. `rounds` steps reach 2^rounds lanes back, beyond which nothing is left.
+template <class G>
+__device__ __forceinline__ void sweep_scan(const float* tab, int rounds, int lane, const float (&f)[G::D],
+                                           float (&S)[G::D], float (&last)[G::D]) {
+    constexpr int D = G::D;
+#pragma unroll
+    for (int c = 0; c < D; ++c) last[c] = f[c];
+#pragma unroll
+    for (int k = 0; (1 << k) < SWEEP_LANES; ++k) {
+        if (k >= rounds) break;
+        float o[D];
+#pragma unroll
+        for (int c = 0; c < D; ++c) {
+            o[c] = __shfl_up_sync(FULL_MASK, last[c], 1u << k);
+            if (lane < (1 << k)) o[c] = 0.f;
+        }
+        tri_mad<G::K>(tab + G::T_PL + 4 * (1 << k) * G::BLOCKS, o, last, last);
+    }
+#pragma unroll
+    for (int c = 0; c < D; ++c) {
+        S[c] = __shfl_up_sync(FULL_MASK, last[c], 1);
+        if (lane == 0) S[c] = 0.f;
+    }
+}
+
+// ------------------------------------------------------------------------------------
+// pass B, PH form: the cascade's own recurrences, sub-rows in packed pairs
+// ------------------------------------------------------------------------------------
+struct SweepSection {
+    float b1, b2, a1, a2;  // section 0: b1, b2 carry the input gain (its input is the raw sample)
+};
+
+template <class G>
+__device__ __forceinline__ void sweep_run_ph(float* buf, const SweepSection* sec, float gain, int lane,
+                                             const float (&st)[G::R][G::D], const float (&xh)[G::R][2]) {
+    constexpr int K = G::K, N = G::N, R = G::R, P = R / 2;
+    f32x2 b1[K], b2[K], a1[K], a2[K];
+#pragma unroll
+    for (int s = 0; s < K; ++s) {
+        b1[s] = pack2(sec[s].b1, sec[s].b1);
+        b2[s] = pack2(sec[s].b2, sec[s].b2);
+        a1[s] = pack2(sec[s].a1, sec[s].a1);
+        a2[s] = pack2(sec[s].a2, sec[s].a2);
+    }
+    const f32x2 g = pack2(gain, gain);
+    // h[p][0]: input history; h[p][s + 1]: section s's output history; [..][0] = n - 2, [..][1] = n - 1
+    f32x2 h[P][K + 1][2];
+#pragma unroll
+    for (int p = 0; p < P; ++p)
+#pragma unroll
+        for (int t = 0; t < 2; ++t) {
+            h[p][0][t] = pack2(xh[2 * p][t], xh[2 * p + 1][t]);
+#pragma unroll
+            for (int s = 0; s < K; ++s) {
+                // state pairs are (y[-1] - y[-2], y[-1])
+                const float* u = st[2 * p] + 2 * s;
+                const float* v = st[2 * p + 1] + 2 * s;
+                h[p][s + 1][t] = t == 0 ? pack2(u[1] - u[0], v[1] - v[0]) : pack2(u[1], v[1]);
+            }
+        }
+    float* row = buf + (lane << 5);
+    const int l7 = lane & 7;
+#pragma unroll 2
+    for (int j = 0; j < N / 4; ++j) {
+        float* at = row + ((j >> 3) << 10) + (((j & 7) ^ l7) << 2);
+        float4 x[R];
+#pragma unroll
+        for (int i = 0; i < R; ++i) x[i] = *reinterpret_cast<const float4*>(at + i * (N / 32) * 1024);
+        // v[p][s][t]: section s's input (s = K: the output) at samples t - 2, t = 0..5. Four samples go
+        // through the sections along the diagonals (sample + section), whose steps do not depend on
+        // one another.
+        f32x2 v[P][K + 1][6];
+#pragma unroll
+        for (int p = 0; p < P; ++p) {
+#pragma unroll
+            for (int s = 0; s <= K; ++s) {
+                v[p][s][0] = h[p][s][0];
+                v[p][s][1] = h[p][s][1];
+            }
+            v[p][0][2] = pack2(x[2 * p].x, x[2 * p + 1].x);
+            v[p][0][3] = pack2(x[2 * p].y, x[2 * p + 1].y);
+            v[p][0][4] = pack2(x[2 * p].z, x[2 * p + 1].z);
+            v[p][0][5] = pack2(x[2 * p].w, x[2 * p + 1].w);
+        }
+#pragma unroll
+        for (int d = 0; d < K + 3; ++d) {
+#pragma unroll
+            for (int s = 0; s < K; ++s) {
+                const int t = d - s + 2;
+                if (t < 2 || t > 5) continue;
+#pragma unroll
+                for (int p = 0; p < P; ++p) {
+                    const f32x2 in = s == 0 ? mul2(g, v[p][0][t]) : v[p][s][t];
+                    const f32x2 w = fma2(b2[s], v[p][s][t - 2], fma2(b1[s], v[p][s][t - 1], in));
+                    v[p][s + 1][t] = fma2(a1[s], v[p][s + 1][t - 1], fma2(a2[s], v[p][s + 1][t - 2], w));
+                }
+            }
+        }
+#pragma unroll
+        for (int p = 0; p < P; ++p) {
+#pragma unroll
+            for (int s = 0; s <= K; ++s) {
+                h[p][s][0] = v[p][s][4];
+                h[p][s][1] = v[p][s][5];
+            }
+            unpack2(v[p][K][2], x[2 * p].x, x[2 * p + 1].x);
+            unpack2(v[p][K][3], x[2 * p].y, x[2 * p + 1].y);
+            unpack2(v[p][K][4], x[2 * p].z, x[2 * p + 1].z);
+            unpack2(v[p][K][5], x[2 * p].w, x[2 * p + 1].w);
+        }
+#pragma unroll
+        for (int i = 0; i < R; ++i) *reinterpret_cast<float4*>(at + i * (N / 32) * 1024) = x[i];
+    }
+}
+
+// ------------------------------------------------------------------------------------
+// launch parameters and the tile loop
+// ------------------------------------------------------------------------------------
+struct IirSweepParams {
+    CUtensorMap tmap_x;  // x as rows of SPAN samples, box {32, 32}, 128-byte swizzle
+    CUtensorMap tmap_y;  // y likewise
+    const float* x;
+    float* y;
+    long long n;
+    const float* tables;  // SweepGeom's layout
+    IirLaunchState* state;
+    long long timeout_ns;
+    unsigned int ntiles;
+    unsigned int run0, run1;  // tiles of a block's first run, and of the runs drawn after it
+    int lanes, rounds;        // lanes that a state reaches; scan steps that cover them
+    int use_tma;              // tensor maps valid (x, y 16-byte aligned, at least one row)
+    float gain;
+    SweepSection sec[IIR_MAX_SECTIONS];
+};
+
+constexpr unsigned SWEEP_RING = 64;  // item records and end states kept of the last items
+constexpr unsigned SWEEP_WARM = 0x80000000u;
+
+template <int NB, int D>
+struct SweepAux {
+    unsigned long long full[NB], empty[NB];
+    float ends[SWEEP_RING][D];           // items' end states
+    unsigned int item[SWEEP_RING];       // the item's tile, SWEEP_WARM if only its end state is wanted
+    volatile unsigned int ready[SWEEP_RING];  // i + 1 once item i's end state is in `ends`
+    volatile unsigned int issued[NB];    // items put into the buffer so far
+    volatile unsigned int total;         // items of the block, once known
+    volatile unsigned int abandon;       // a wait ran out: everybody leaves
+    unsigned int next;                   // next item for a free warp
+};
+
+// Blocks of W filter warps and a loader warp. The signal's tiles (32 lane rows each) are dealt out in
+// runs of consecutive tiles: block b starts with run b of run0 tiles, then draws runs of run1 tiles
+// from a ticket counter until they are gone. SMs differ in the bandwidth they get (a copy kernel
+// that splits a signal evenly among blocks reaches 6.2 TB/s, one that draws its tiles 7.0), so the
+// last part is drawn. Ahead of a run goes the tile before it, of which only the end state is
+// computed: no block needs anything from another.
+//
+// Inside a block the items (tiles of its runs, one after another) are taken by the warps in order,
+// and item i's end state goes to item i + 1 through shared memory. It is the end state from rest:
+// older state has decayed inside the tile, so the items form no chain, and a warp waits for no more
+// than the pass A of the item before its own, which another warp began earlier. Its first lanes add
+// the response to it, Phi^(SPAN l) for lane l.
+//
+// Item i lies in buffer i % NB: the loader keeps NB - W items ahead of the warps. A warp gives its
+// buffer back when the store of its output has read it, which it looks after during its next item
+// (after pass A), or before it would wait itself.
+template <class G, int W, int NB, class Run>
+__device__ __forceinline__ void sweep_tiles(const IirSweepParams& p, unsigned char* smem, Run&& run) {
+    constexpr int SPAN = G::SPAN, R = G::R, K = G::K, D = G::D;
+    using Aux = SweepAux<NB, D>;
+    static_assert(NB >= W && NB + W <= static_cast<int>(SWEEP_RING), "a buffer per warp, a record per item in flight");
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    float* bufs = reinterpret_cast<float*>(smem);
+    Aux& aux = *reinterpret_cast<Aux*>(smem + NB * size_t(G::TILE_BYTES));
+    float* tab = reinterpret_cast<float*>(smem + NB * size_t(G::TILE_BYTES) + ((sizeof(Aux) + 15) & ~size_t(15)));
+    if (threadIdx.x == W * 32) {
+        for (int b = 0; b < NB; ++b) {
+            mbar_init(aux.full + b, 1);
+            mbar_init(aux.empty + b, 1);
+            aux.issued[b] = 0u;
+        }
+        for (unsigned i = 0; i < SWEEP_RING; ++i) aux.ready[i] = 0u;
+        aux.next = 0u;
+        aux.total = 0xffffffffu;
+        aux.abandon = 0u;
+        fence_mbar_init();
+    }
+    // (of Phi^(SPAN l), the powers that the lanes and the scan steps use)
+    const int reach = p.lanes > (1 << p.rounds) / 2 + 1 ? p.lanes : (1 << p.rounds) / 2 + 1;
+    for (int i = threadIdx.x; i < G::T_PL / 4 + reach * G::BLOCKS; i += (W + 1) * 32)
+        reinterpret_cast<float4*>(tab)[i] = __ldg(reinterpret_cast<const float4*>(p.tables) + i);
+    __syncthreads();
+    // every wait is bounded; the first to run out sends the whole block home
+    auto wait_for = [&](auto&& cond) {
+        if (cond()) return true;
+        const uint64_t start = globaltimer_ns();
+        uint32_t spins = 0;
+        while (!cond()) {
+            if ((++spins & 63u) != 0u) continue;
+            if (aux.abandon) return false;
+            if (globaltimer_ns() - start > static_cast<uint64_t>(p.timeout_ns)) {
+                aux.abandon = 1u;
+                raise_error(p.state, 0xffffffffu, IIR_DEV_ERR_MBARRIER);
+                return false;
+            }
+        }
+        return true;
+    };
+    if (warp == W) {
+        if (lane == 0) {
+            unsigned i = 0;
+            unsigned long long first = static_cast<unsigned long long>(blockIdx.x) * p.run0;
+            unsigned len = p.run0;
+            bool ok = true;
+            while (ok && first < p.ntiles) {
+                const unsigned a = static_cast<unsigned>(first);
+                const unsigned e = p.ntiles - a < len ? p.ntiles : a + len;
+                for (unsigned t = a > 0 ? a - 1 : 0; t < e; ++t, ++i) {
+                    const unsigned b = i % NB;
+                    if (i >= NB) ok = wait_for([&] { return mbar_try_wait(aux.empty + b, (i / NB - 1u) & 1u); });
+                    if (!ok) break;
+                    aux.item[i % SWEEP_RING] = t < a ? (t | SWEEP_WARM) : t;
+                    if (p.use_tma) {
+                        float* buf = bufs + static_cast<size_t>(b) * G::TILE;
+                        mbar_arrive_expect_tx(aux.full + b, G::TILE_BYTES);
+#pragma unroll
+                        for (int h = 0; h < SPAN / 32; ++h)
+                            tma_load_2d(buf + h * 1024, &p.tmap_x, 32 * h, static_cast<int>(t * 32u), aux.full + b);
+                    } else {
+                        mbar_arrive(aux.full + b);
+                    }
+                    aux.issued[b] = i / NB + 1u;
+                }
+                if (!ok) break;
+                len = p.run1;
+                first = static_cast<unsigned long long>(gridDim.x) * p.run0 +
+                        static_cast<unsigned long long>(atomicAdd(&p.state->runs, 1u)) * p.run1;
+            }
+            aux.total = i;
+        }
+    } else {
+        const long long rows = p.n / SPAN;  // whole lane rows of the signal
+        const int rest = static_cast<int>(p.n - rows * SPAN);
+        int back = -1;  // lane 0: the buffer to give back
+        auto give_back = [&] {
+            bulk_wait_read_all();  // the store has read it
+            mbar_arrive(aux.empty + back);
+            back = -1;
+        };
+        while (true) {
+            unsigned i = 0;
+            if (lane == 0) i = atomicAdd(&aux.next, 1u);
+            i = __shfl_sync(FULL_MASK, i, 0);
+            const unsigned b = i % NB;
+            // Item i is in its buffer. Its barrier is looked at only once the item's own load has been
+            // issued: until then the barrier may be two phases back, and a parity cannot tell those apart.
+            auto arrived = [&] { return aux.issued[b] == i / NB + 1u && mbar_try_wait(aux.full + b, (i / NB) & 1u); };
+            if (back >= 0 && !arrived()) give_back();
+            __syncwarp();
+            const bool in = wait_for([&] { return aux.total <= i || arrived(); });
+            if (__any_sync(FULL_MASK, !in) || aux.total <= i) break;
+            const unsigned rec = aux.item[i % SWEEP_RING];
+            const bool warm = (rec & SWEEP_WARM) != 0u;
+            const unsigned t = rec & ~SWEEP_WARM;
+            float* buf = bufs + static_cast<size_t>(b) * G::TILE;
+            const long long row0 = static_cast<long long>(t) * 32, base = row0 * SPAN;
+            float g2 = 0.f, g1 = 0.f;  // the two samples before the tile
+            if (lane == 0 && t > 0) {
+                g2 = __ldg(p.x + base - 2);
+                g1 = __ldg(p.x + base - 1);
+            }
+            // the signal's last, partial lane row (the tensor maps hold whole rows), if it is here
+            const int part = (rest > 0 && rows >= row0 && rows < row0 + 32) ? static_cast<int>(rows - row0) : -1;
+            if (p.use_tma) {
+                if (part >= 0) {
+                    for (int j = lane; j < rest; j += 32) buf[tile_at(part, j)] = __ldg(p.x + rows * SPAN + j);
+                    __syncwarp();
+                }
+            } else {
+#pragma unroll 8
+                for (int j = lane; j < G::TILE; j += 32) {
+                    const bool have = base + j < p.n;
+                    cp_async4(buf + tile_at(j / SPAN, j % SPAN), have ? p.x + base + j : p.x, have ? 4 : 0);
+                }
+                cp_async_commit();
+                cp_async_wait<0>();
+                __syncwarp();
+            }
+            float e[R][D], st[R][D], xh[R][2];
+            sweep_ends<G>(buf, tab, lane, g2, g1, e, xh);
+            if (back >= 0) give_back();
+            {
+                float f[D], last[D];
+                sweep_join<G>(tab, e, f);
+                sweep_scan<G>(tab, p.rounds, lane, f, st[0], last);
+                if (lane == 31) {
+#pragma unroll
+                    for (int c = 0; c < D; c += 2)
+                        *reinterpret_cast<float2*>(&aux.ends[i % SWEEP_RING][c]) = make_float2(last[c], last[c + 1]);
+                    __threadfence_block();
+                    aux.ready[i % SWEEP_RING] = i + 1u;
+                }
+            }
+            if (!warm && t > 0) {
+                const bool got = wait_for([&] { return aux.ready[(i - 1u) % SWEEP_RING] == i; });
+                if (__any_sync(FULL_MASK, !got)) break;
+                __threadfence_block();
+                if (lane < p.lanes) {
+                    float X[D];
+#pragma unroll
+                    for (int c = 0; c < D; c += 2) {
+                        const float2 v = *reinterpret_cast<const float2*>(&aux.ends[(i - 1u) % SWEEP_RING][c]);
+                        X[c] = v.x;
+                        X[c + 1] = v.y;
+                    }
+                    tri_mad<K>(tab + G::T_PL + 4 * lane * G::BLOCKS, X, st[0], st[0]);
+                }
+            }
+            if (!warm) {
+#pragma unroll
+                for (int j = 1; j < R; ++j) tri_mad<K>(tab + G::T_PN, st[j - 1], e[j - 1], st[j]);
+                __syncwarp();  // every lane has read its neighbour's last samples
+                run(buf, lane, st, xh);
+            }
+            if (p.use_tma) {
+                fence_proxy_async_smem();  // generic accesses of the buffer before the async ones to come
+                __syncwarp();
+                if (lane == 0 && !warm) {
+#pragma unroll
+                    for (int h = 0; h < SPAN / 32; ++h)
+                        tma_store_2d(&p.tmap_y, 32 * h, static_cast<int>(row0), buf + h * 1024);
+                    bulk_commit();
+                }
+                if (!warm && part >= 0)
+                    for (int j = lane; j < rest; j += 32) p.y[rows * SPAN + j] = buf[tile_at(part, j)];
+            } else if (!warm) {
+                __syncwarp();
+#pragma unroll 8
+                for (int j = lane; j < G::TILE; j += 32)
+                    if (base + j < p.n) p.y[base + j] = buf[tile_at(j / SPAN, j % SPAN)];
+            }
+            __syncwarp();
+            if (lane == 0) back = static_cast<int>(b);
+        }
+        if (lane == 0) bulk_wait_read_all();  // shared memory outlives the copies' reads
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        // the last block out re-arms the run counter
+        __threadfence();
+        if (atomicAdd(&p.state->done, 1u) == gridDim.x - 1u) {
+            p.state->runs = 0u;
+            p.state->done = 0u;
+            __threadfence();
+        }
+    }
+}
+
+template <int K, int N, int R>
+constexpr size_t sweep_smem(int NBv, size_t aux) {
+    return NBv * size_t(SweepGeom<K, N, R>::TILE_BYTES) + ((aux + 15) & ~size_t(15)) + SweepGeom<K, N, R>::T_LEN * 4u;
+}
+
+}  // namespace iirgb
