@@ -1,8 +1,13 @@
-// iir_batch.cu — batched segments: many independent signals in one persistent launch.
+// iir_batch.cu — batched segments: many independent signals in one launch.
 //
 // A segment is one signal (a channel, or the next chunk of a live stream) with its own
 // cascade (any number of sections up to IIR_MAX_SECTIONS), an optional state in (zi) and an
-// optional state out (zf). The launch's chunks are the concatenation of every segment's
+// optional state out (zf). Two kernels share a call's segments:
+//   * the state sweep (iir_batch_sweep.cuh) takes every segment whose filter decays within a tile;
+//   * the lookback kernel below takes the others, and all of them when a fault is injected or the
+//     environment asks for its schedules. Where both have segments they run side by side.
+//
+// Lookback kernel: the launch's chunks are the concatenation of every segment's
 // chunks; that list is the launch's work queue. A persistent grid (every block resident: the
 // occupancy of the chosen kernel times the SMs) draws chunks from it in ticket order, one atomic
 // per chunk, finds each chunk's segment with a 32-way search of the segment start table, and
@@ -11,7 +16,7 @@
 // segment. The block that holds a segment's last sample writes zf. A chunk only ever waits for
 // a chunk drawn before it, which a running block holds, so the queue cannot deadlock.
 //
-// Two schedules:
+// It has two schedules:
 //   * per-section lookback (the default): each section publishes the chunk's zero-state
 //     aggregate and waits for its predecessor's (control(); two block barriers per section);
 //   * tail aggregate (iir_tail.cuh), for segments of at least IIR_GB300_BATCH_TAIL_CHUNKS chunks
@@ -19,10 +24,10 @@
 //     section comes from its last pieces, published at once; the chunk reads its predecessor's
 //     and the row warps run every section with one barrier each.
 //
-// The chunk shape (rows x samples per row) is a run-time choice among compiled instantiations
+// Its chunk shape (rows x samples per row) is a run-time choice among compiled instantiations
 // (iir_batch_set_shape): long channels favour big chunks (fewer lookbacks per sample), short ones
 // small chunks (less padding past a segment's end). The tuner in autotune.py picks it, seeded
-// by an occupancy model of GB300.
+// by an occupancy model of GB300. It has no say in the sweep's tiles.
 //
 // The reference filters one signal with one compile-time filter per launch
 // (ph_kernels.cuh:151-200, src/test_accuracy.cu:146); this is the batching form that design
@@ -37,6 +42,7 @@
 #include <vector>
 
 #include "../../include/iir_gb300.h"
+#include "iir_batch_sweep.h"
 #include "iir_host_internal.h"
 #include "iir_ph.cuh"
 #include "iir_registry.h"
@@ -525,12 +531,33 @@ const std::vector<ShapeDef>& shapes() {
 // row) and the filters (with each filter's schedule for this shape), built when the shape is
 // first used; the occupancy of its kernel.
 struct ShapeData {
-    bool ready = false;
+    bool ready = false;    // tables and filters on the device
+    bool measured = false;  // footprint and residency known
+    bool tails = false;     // the filters carry their tail pieces
+    bool all = false;       // every filter's tables, not the slow ones' only
     IirSection* d_secs = nullptr;
     float4* d_tables = nullptr;
     IirBatchFilter* d_filters = nullptr;
     int blocks_per_sm = 0;
     int regs = 0;  // registers per thread of the shape's kernel
+};
+
+// The state sweep's tiles: 4096 samples, or 1024 for short segments.
+constexpr int SWEEP_SIZES = 2;
+
+// Device tables of one tile size, and what a segment of each filter needs.
+struct SweepData {
+    bool ready = false;
+    const BatchSweepKernel* kern = nullptr;
+    float4* d_tables = nullptr;
+    int resident = 0;  // blocks
+    struct Filter {
+        unsigned int table;  // 16-byte units from d_tables
+        int rounds;
+        bool fast;  // decays within a tile
+    };
+    std::vector<Filter> filters;
+    bool covers = false;  // every filter does
 };
 
 }  // namespace
@@ -543,9 +570,11 @@ struct iir_batch {
     // filters on the host: normalised sections, gains, sections per filter, tail pieces needed
     std::vector<SectionF32> sec32;
     std::vector<IirBatchFilter> filters;
+    std::vector<double> gains;
     std::vector<int> tail_need;  // least number of tail pieces for the filter's state to decay (0: > 8)
     float* d_phi = nullptr;
     std::vector<ShapeData> shape_data;
+    std::vector<void*> retired;  // device tables that later ones replaced
     int shape = 0;  // index into shapes()
     IirLaunchState* d_state = nullptr;
     unsigned long long* d_carry = nullptr;
@@ -557,6 +586,15 @@ struct iir_batch {
     unsigned char* h_stage[2] = {nullptr, nullptr};
     cudaEvent_t stage_done[2] = {nullptr, nullptr};
     int stage_turn = 0;
+    SweepData sweep[SWEEP_SIZES];
+    BatchRun* d_runs = nullptr;
+    size_t run_cap = 0;
+    BatchRun* h_runs[2] = {nullptr, nullptr};  // pinned, used in turn (an event guards reuse)
+    cudaEvent_t run_done[2] = {nullptr, nullptr};
+    int run_turn = 0;
+    IirLaunchState* d_sweep_state = nullptr;  // the sweep's own: it may run beside the lookback kernel
+    cudaStream_t side = nullptr;              // ... which then runs here, between these two events
+    cudaEvent_t fork = nullptr, join = nullptr;
     std::vector<int> filter_sections;
     long long timeout_ns = 1000000000ll;
     long long withhold = -1;
@@ -590,6 +628,20 @@ int batch_alloc_segments(iir_batch* b, size_t segs) {
     return IIR_OK;
 }
 
+int batch_alloc_runs(iir_batch* b, size_t runs) {
+    if (b->d_runs) cudaFree(b->d_runs);
+    b->d_runs = nullptr;
+    for (int i = 0; i < 2; ++i) {
+        if (b->h_runs[i]) cudaFreeHost(b->h_runs[i]);
+        b->h_runs[i] = nullptr;
+    }
+    b->run_cap = 0;
+    int st = cuda_status(cudaMalloc(&b->d_runs, runs * sizeof(BatchRun)));
+    for (int i = 0; i < 2 && !st; ++i) st = cuda_status(cudaMallocHost(&b->h_runs[i], runs * sizeof(BatchRun)));
+    if (!st) b->run_cap = runs;
+    return st;
+}
+
 int batch_alloc_carry(iir_batch* b, size_t chunks, size_t segs) {
     if (b->d_carry) cudaFree(b->d_carry);
     b->d_carry = nullptr;
@@ -613,12 +665,25 @@ void batch_free(iir_batch* b) {
     cudaDeviceSynchronize();
     batch_free_segments(b);
     for (int i = 0; i < 2; ++i)
+    {
         if (b->stage_done[i]) cudaEventDestroy(b->stage_done[i]);
+        if (b->run_done[i]) cudaEventDestroy(b->run_done[i]);
+    }
+    for (SweepData& d : b->sweep)
+        if (d.d_tables) cudaFree(d.d_tables);
+    if (b->d_runs) cudaFree(b->d_runs);
+    for (int i = 0; i < 2; ++i)
+        if (b->h_runs[i]) cudaFreeHost(b->h_runs[i]);
+    if (b->d_sweep_state) cudaFree(b->d_sweep_state);
+    if (b->fork) cudaEventDestroy(b->fork);
+    if (b->join) cudaEventDestroy(b->join);
+    if (b->side) cudaStreamDestroy(b->side);
     for (ShapeData& d : b->shape_data) {
         if (d.d_secs) cudaFree(d.d_secs);
         if (d.d_tables) cudaFree(d.d_tables);
         if (d.d_filters) cudaFree(d.d_filters);
     }
+    for (void* q : b->retired) cudaFree(q);
     if (b->d_phi) cudaFree(b->d_phi);
     if (b->d_state) cudaFree(b->d_state);
     if (b->d_carry) cudaFree(b->d_carry);
@@ -645,15 +710,68 @@ size_t batch_tail_min_chunks() {
     return v > 0 ? static_cast<size_t>(v) : 1;
 }
 
-// Builds shape k's lane tables and filter records (once) and its occupancy.
-int shape_prepare(iir_batch* b, int k) {
+// Footprint and residency of shape k's kernel (once).
+int shape_measure(iir_batch* b, int k) {
     ShapeData& d = b->shape_data[static_cast<size_t>(k)];
-    if (d.ready) return IIR_OK;
+    if (d.measured) return IIR_OK;
+    const ShapeDef& sd = shapes()[static_cast<size_t>(k)];
+    int st = cuda_status(
+        cudaFuncSetAttribute(sd.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sd.smem)));
+    if (!st) st = cuda_status(cudaFuncSetAttribute(sd.fn, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
+    int nb = 0;
+    if (!st) st = cuda_status(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, sd.fn, sd.threads, sd.smem));
+    cudaFuncAttributes fa{};
+    if (!st) st = cuda_status(cudaFuncGetAttributes(&fa, sd.fn));
+    if (st) return st;
+    if (nb <= 0) return IIR_ERR_UNSUPPORTED;
+    d.blocks_per_sm = nb;
+    d.regs = fa.numRegs;
+    d.measured = true;
+    return IIR_OK;
+}
+
+// Tail-aggregate schedule, an option (IIR_GB300_BATCH_TAIL_CHUNKS): pieces for every filter's state to
+// decay, and Phi^512.
+int batch_tail_tables(iir_batch* b) {
+    std::vector<float> phi(b->filters.size() * IIR_BT_PHI_FLOATS, 0.f);
+    for (size_t f = 0; f < b->filters.size(); ++f) {
+        std::vector<float> pf;
+        const IirBatchFilter& q = b->filters[f];
+        b->tail_need[f] = tail_pieces(b->sec32.data() + q.sec0, q.n_sections, IIR_TAIL_MAX_PIECES, pf);
+        std::copy(pf.begin(), pf.end(), phi.begin() + static_cast<long>(f) * IIR_BT_PHI_FLOATS);
+    }
+    int st = cuda_status(cudaMalloc(&b->d_phi, phi.size() * sizeof(float)));
+    if (!st) st = cuda_status(cudaMemcpy(b->d_phi, phi.data(), phi.size() * sizeof(float), cudaMemcpyHostToDevice));
+    return st;
+}
+
+// Builds shape k's lane tables and filter records (once) and its occupancy.
+// (all: of every filter; else of those that the sweep does not take).
+int shape_prepare(iir_batch* b, int k, bool all) {
+    ShapeData& d = b->shape_data[static_cast<size_t>(k)];
+    const bool tails = std::getenv("IIR_GB300_BATCH_TAIL_CHUNKS") != nullptr;
+    if (d.ready && (d.tails || !tails) && (d.all || !all)) return IIR_OK;
+    if (tails && !b->d_phi)
+        if (const int r = batch_tail_tables(b)) return r;
+    if (d.ready) {  // again, with more of them: bound launches (and graphs of them) keep the earlier ones
+        for (void* q : {static_cast<void*>(d.d_secs), static_cast<void*>(d.d_tables), static_cast<void*>(d.d_filters)})
+            b->retired.push_back(q);
+        d = ShapeData{};
+    }
+    d.tails = tails;
+    d.all = all;
     const ShapeDef& sd = shapes()[static_cast<size_t>(k)];
     std::vector<float4> tabs(b->sec32.size() * IIR_BT_STRIDE, make_float4(0, 0, 0, 0));
     std::vector<IirSection> secs(b->sec32.size());
     std::vector<float4> full(IIR_TAB_STRIDE);
+    std::vector<char> wanted(b->sec32.size(), all ? 1 : 0);
+    for (size_t f = 0; f < b->filters.size() && !all; ++f) {
+        bool fast = true;
+        for (const SweepData& v : b->sweep) fast = fast && (!v.ready || v.filters[f].fast);
+        std::fill_n(wanted.begin() + b->filters[f].sec0, b->filters[f].n_sections, fast ? 0 : 1);
+    }
     for (size_t s = 0; s < b->sec32.size(); ++s) {
+        if (!wanted[s]) continue;
         IirSection& q = secs[s];
         const int st = precompute_section(b->sec32[s], IIR_KIND_PH, sd.rows, sd.n, q, full.data());
         if (st) return st;
@@ -670,7 +788,7 @@ int shape_prepare(iir_batch* b, int k) {
     std::vector<IirBatchFilter> flt = b->filters;
     const bool tail_on = batch_tail_enabled();
     for (size_t f = 0; f < flt.size(); ++f) {
-        const int need = b->tail_need[f];
+        const int need = b->tail_need[f];  // 0 unless the option is set
         flt[f].tail = (tail_on && need > 0 && need <= sd.max_pieces) ? need : 0;
     }
     int st = cuda_status(cudaMalloc(&d.d_secs, secs.size() * sizeof(IirSection)));
@@ -680,20 +798,208 @@ int shape_prepare(iir_batch* b, int k) {
     if (!st) st = cuda_status(cudaMalloc(&d.d_filters, flt.size() * sizeof(IirBatchFilter)));
     if (!st)
         st = cuda_status(cudaMemcpy(d.d_filters, flt.data(), flt.size() * sizeof(IirBatchFilter), cudaMemcpyHostToDevice));
-    if (!st)
-        st = cuda_status(
-            cudaFuncSetAttribute(sd.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sd.smem)));
-    if (!st) st = cuda_status(cudaFuncSetAttribute(sd.fn, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
-    int nb = 0;
-    if (!st) st = cuda_status(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, sd.fn, sd.threads, sd.smem));
-    cudaFuncAttributes fa{};
-    if (!st) st = cuda_status(cudaFuncGetAttributes(&fa, sd.fn));
+    if (!st) st = shape_measure(b, k);
     if (st) return st;
-    if (nb <= 0) return IIR_ERR_UNSUPPORTED;
-    d.blocks_per_sm = nb;
-    d.regs = fa.numRegs;
     d.ready = true;
     return IIR_OK;
+}
+
+// ---- state sweep ----
+const std::vector<BatchSweepKernel>& sweep_kernel_list() {
+    static const std::vector<BatchSweepKernel> v = [] {
+        std::vector<BatchSweepKernel> r;
+        bsweep_kernels2(r);
+        bsweep_kernels4(r);
+        bsweep_kernels8(r);
+        return r;
+    }();
+    return v;
+}
+
+// Tile size v's tables (once): the kernel for the batch's largest cascade.
+int sweep_prepare(iir_batch* b, int v) {
+    SweepData& d = b->sweep[v];
+    if (d.ready) return IIR_OK;
+    const BatchSweepKernel* kern = nullptr;
+    for (const BatchSweepKernel& k : sweep_kernel_list())
+        if (k.max_k >= b->max_sections && k.tile() == (v == 0 ? 4096 : 1024) && (!kern || k.max_k < kern->max_k)) kern = &k;
+    if (!kern) return IIR_ERR_UNSUPPORTED;
+    std::vector<float> all;
+    d.filters.clear();
+    d.covers = true;
+    for (size_t f = 0; f < b->filters.size(); ++f) {
+        const IirBatchFilter& q = b->filters[f];
+        const BatchSweepFilter s =
+            bsweep_filter(b->sec32.data() + q.sec0, q.n_sections, b->gains[f], kern->span);
+        d.filters.push_back(SweepData::Filter{static_cast<unsigned>(all.size() / 4), s.rounds, s.fast});
+        d.covers = d.covers && s.fast;
+        all.insert(all.end(), s.table.begin(), s.table.end());
+    }
+    if (all.size() / 4 > 0xffffffffull) return IIR_ERR_TOO_LARGE;
+    int nb = 0;
+    int st = cuda_status(
+        cudaFuncSetAttribute(kern->fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kern->smem)));
+    if (!st) st = cuda_status(cudaFuncSetAttribute(kern->fn, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
+    if (!st)
+        st = cuda_status(
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kern->fn, kern->threads, kern->smem));
+    if (!st && nb <= 0) st = IIR_ERR_UNSUPPORTED;
+    if (!st) st = cuda_status(cudaMalloc(&d.d_tables, all.size() * sizeof(float)));
+    if (!st) st = cuda_status(cudaMemcpy(d.d_tables, all.data(), all.size() * sizeof(float), cudaMemcpyHostToDevice));
+    if (st) return st;
+    d.kern = kern;
+    d.resident = nb * b->sms;
+    d.ready = true;
+    return IIR_OK;
+}
+
+// Samples of a segment before the first 16-byte boundary of its input (0..3).
+int sweep_peel_of(const iir_segment& s) {
+    const size_t k = (4 - ((reinterpret_cast<uintptr_t>(s.x) >> 2) & 3u)) & 3u;
+    return static_cast<int>(k < s.n ? k : s.n);
+}
+
+size_t sweep_tiles(const iir_segment& s, int tile) {
+    if (s.n == 0) return 0;
+    const size_t n = s.n - static_cast<size_t>(sweep_peel_of(s));
+    return n == 0 ? 1 : (n + static_cast<size_t>(tile) - 1) / static_cast<size_t>(tile);
+}
+
+// How a call's segments are filtered: those on the state sweep, with the tile size and the length and
+// number of their runs, and those on the lookback kernel.
+struct Schedule {
+    bool sweep = false;  // some may be swept
+    int v = 0;
+    size_t len = 0;      // tiles per run
+    size_t longest = 0;  // of the runs there are
+    size_t runs = 0;
+    std::vector<int> swept;
+    std::vector<iir_segment> rest;
+};
+
+bool sweep_enabled() { return batch_tail_enabled() && !std::getenv("IIR_GB300_BATCH_TAIL_CHUNKS"); }
+
+// Runs of calls of up to `segs` segments and `chunks` (the largest) chunks: by the runs' length below.
+size_t sweep_run_capacity(const iir_batch* b, size_t segs, size_t chunks) {
+    return 2 * segs + 6 * static_cast<size_t>(b->sms) + chunks / 2 + 8;
+}
+
+// The sweep takes every segment whose filter decays within a tile, unless a fault is to be injected (it
+// has no carries to withhold) or the environment asks for a lookback schedule.
+int make_schedule(iir_batch* b, const iir_segment* segs, int n_segs, bool inject, cudaStream_t stream, Schedule& c) {
+    const bool sweep = c.sweep = !inject && sweep_enabled();
+    // 4096-sample tiles unless padding costs more than the shorter tiles' overhead (a 1024-sample tile
+    // scans as many lanes for a quarter of the samples)
+    size_t large = 0, small = 0;
+    if (sweep) {
+        for (int i = 0; i < n_segs; ++i) {
+            large += 4096 * sweep_tiles(segs[i], 4096);
+            small += 1024 * sweep_tiles(segs[i], 1024);
+        }
+        c.v = 2 * large > 3 * small ? 1 : 0;
+        if (c.v == 1 && !(b->sweep[1].ready && (b->sweep[1].covers || b->shape_data[static_cast<size_t>(b->shape)].all))) {
+            // tables to build, which no capture allows: it gets the tiles that are there
+            cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+            if (const int st = cuda_status(cudaStreamIsCapturing(stream, &cap))) return st;
+            if (cap != cudaStreamCaptureStatusNone) c.v = 0;
+        }
+        if (const int st = sweep_prepare(b, c.v)) return st;
+    }
+    const SweepData& d = b->sweep[c.v];
+    const int tile = sweep ? d.kern->tile() : 1;
+    // A run costs the pass A of the tile ahead of it, so it is long, but every block should see several.
+    const size_t total = (c.v == 0 ? large : small) / static_cast<size_t>(tile);
+    c.len = std::min<size_t>(16, std::max<size_t>(4, total / static_cast<size_t>(6 * b->sms)));
+    for (int i = 0; i < n_segs; ++i) {
+        const iir_segment& s = segs[i];
+        if (s.n == 0) continue;
+        const size_t tiles = sweep ? sweep_tiles(s, tile) : 0;
+        if (!sweep || !d.filters[static_cast<size_t>(s.filter)].fast || tiles >= (1ull << 30)) {
+            c.rest.push_back(s);
+        } else {
+            c.swept.push_back(i);
+            c.runs += (tiles + c.len - 1) / c.len;
+            c.longest = std::max(c.longest, std::min(tiles, c.len));
+        }
+    }
+    return c.runs > 0x7fffffffull ? IIR_ERR_TOO_LARGE : IIR_OK;
+}
+
+void sweep_runs(const iir_batch* b, const Schedule& c, const iir_segment* segs, BatchRun* out) {
+    const SweepData& d = b->sweep[c.v];
+    for (const int i : c.swept) {
+        const iir_segment& s = segs[i];
+        const size_t tiles = sweep_tiles(s, d.kern->tile());
+        const SweepData::Filter& f = d.filters[static_cast<size_t>(s.filter)];
+        const int peel = sweep_peel_of(s);
+        BatchRun r{};
+        r.x = s.x + peel;
+        r.y = s.y + peel;
+        r.zi = s.zi;
+        r.zf = s.zf;
+        r.n = static_cast<long long>(s.n) - peel;
+        r.table = f.table;
+        r.K = static_cast<unsigned char>(b->filter_sections[static_cast<size_t>(s.filter)]);
+        r.rounds = static_cast<unsigned char>(f.rounds);
+        r.peel = static_cast<unsigned char>(peel);
+        for (size_t t = 0; t < tiles; t += c.len) {
+            r.tile0 = static_cast<unsigned>(t);
+            r.count = static_cast<unsigned>(std::min(c.len, tiles - t));
+            r.warm = t > 0 ? 1 : 0;
+            *out++ = r;
+        }
+    }
+}
+
+// One tensor map over [lo, hi) for tiles that start at any 16-byte granule (IirBatchSweepParams). false: the
+// range is too long for it.
+bool encode_granule_map(CUtensorMap* map, uintptr_t lo, uintptr_t hi, int span) {
+    PFN_cuTensorMapEncodeTiled_v12000 enc = tensor_map_encoder();
+    const cuuint64_t granules = (hi - lo) / 16;
+    if (!enc || granules < 1 || granules > 0x7fffffffull) return false;
+    const cuuint64_t dims[3] = {32ull, granules, 32ull};
+    const cuuint64_t strides[2] = {16ull, static_cast<cuuint64_t>(span) * 4};
+    const cuuint32_t box[3] = {32u, 1u, 32u};
+    const cuuint32_t estr[3] = {1u, 1u, 1u};
+    return enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, reinterpret_cast<void*>(lo), dims, strides, box, estr,
+               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// Launch parameters of a schedule's sweep, but for the runs.
+IirBatchSweepParams sweep_params(const iir_batch* b, const Schedule& c, const iir_segment* segs) {
+    IirBatchSweepParams q{};
+    const SweepData& d = b->sweep[c.v];
+    uintptr_t lo[2] = {~uintptr_t(0), ~uintptr_t(0)}, hi[2] = {0, 0};
+    for (const int i : c.swept) {
+        const uintptr_t p[2] = {reinterpret_cast<uintptr_t>(segs[i].x), reinterpret_cast<uintptr_t>(segs[i].y)};
+        for (int k = 0; k < 2; ++k) {
+            lo[k] = std::min(lo[k], p[k]);
+            hi[k] = std::max(hi[k], p[k] + segs[i].n * sizeof(float));
+        }
+    }
+    for (int k = 0; k < 2; ++k) lo[k] &= ~uintptr_t(15);
+    q.x0 = reinterpret_cast<const float*>(lo[0]);
+    q.y0 = reinterpret_cast<float*>(lo[1]);
+    q.use_tma = (encode_granule_map(&q.tmap_x, lo[0], hi[0], d.kern->span) &&
+                 encode_granule_map(&q.tmap_y, lo[1], hi[1], d.kern->span))
+                    ? 1
+                    : 0;
+    q.tables = d.d_tables;
+    q.state = b->d_sweep_state;
+    q.nruns = static_cast<unsigned>(c.runs);
+    q.unit = c.longest >= 8 ? 1 : 2;  // short runs are drawn in pairs: a draw takes about a microsecond
+    return q;
+}
+
+int sweep_launch(const iir_batch* b, int v, IirBatchSweepParams& q, const BatchRun* d_runs, cudaStream_t stream) {
+    const SweepData& d = b->sweep[v];
+    q.runs = d_runs;
+    q.timeout_ns = b->timeout_ns;
+    const unsigned draws = (q.nruns + q.unit - 1) / q.unit, grid = std::min(draws, static_cast<unsigned>(d.resident));
+    void* args[] = {&q};
+    return cuda_status(
+        cudaLaunchKernel(d.kern->fn, dim3(grid), dim3(d.kern->threads), args, d.kern->smem, stream));
 }
 
 // Parameters of a launch over `nchunks` chunks with shape k (segment tables already on the device).
@@ -746,97 +1052,29 @@ size_t seg_chunks(const iir_segment& s, int k) {
 
 }  // namespace
 
-extern "C" {
+namespace {
 
-int iir_batch_create(iir_batch** out, const float* sos, const int* n_sections, int n_filters, size_t max_segments,
-                     size_t max_chunks) {
-    if (!out || !sos || !n_sections || n_filters < 1) return IIR_ERR_INVALID_ARGUMENT;
-    *out = nullptr;
-    iir_batch* b = new iir_batch();
-    b->n_filters = n_filters;
-    b->filters.resize(static_cast<size_t>(n_filters));
-    b->tail_need.assign(static_cast<size_t>(n_filters), 0);
-    std::vector<float> phi(static_cast<size_t>(n_filters) * IIR_BT_PHI_FLOATS, 0.f);
-    int max_sec = 1;
-    size_t off = 0;
-    for (int f = 0; f < n_filters; ++f) {
-        const int ns = n_sections[f];
-        if (ns < 1 || ns > IIR_MAX_SECTIONS) {
-            delete b;
-            return IIR_ERR_INVALID_ARGUMENT;
-        }
-        SectionF32 s32[IIR_MAX_SECTIONS];
-        double gain = 1.0;
-        int st = normalise_sos(sos + 6 * off, ns, s32, gain);
-        if (st) {
-            delete b;
-            return st;
-        }
-        // the sections' scalars and lane tables depend on the chunk shape: shape_prepare builds them
-        b->filters[static_cast<size_t>(f)] =
-            IirBatchFilter{static_cast<float>(gain), ns, static_cast<int>(b->sec32.size()), 0};
-        for (int k = 0; k < ns; ++k) b->sec32.push_back(s32[k]);
-        // tail-aggregate schedule: pieces for the cascade's state to decay, and Phi^512
-        std::vector<float> pf;
-        b->tail_need[static_cast<size_t>(f)] = tail_pieces(s32, ns, IIR_TAIL_MAX_PIECES, pf);
-        std::copy(pf.begin(), pf.end(), phi.begin() + static_cast<size_t>(f) * IIR_BT_PHI_FLOATS);
-        max_sec = std::max(max_sec, ns);
-        off += static_cast<size_t>(ns);
+// Runs `lookback` (launches on the given stream) and `sweep` of one call. Where there are both, the lookback
+// kernel goes first and on the side stream: its last chunks leave most SMs idle, and the sweep's blocks
+// start on them. The caller's stream goes on when both are done.
+template <class Lookback, class Sweep>
+int launch_both(iir_batch* b, cudaStream_t stream, bool both, Lookback&& lookback, Sweep&& sweep) {
+    if (!both) {
+        const int st = lookback(stream);
+        return st ? st : sweep(stream);
     }
-    b->max_sections = max_sec;
-    b->filter_sections.assign(n_sections, n_sections + n_filters);
-    b->shape_data.resize(shapes().size());
-    int st = cuda_status(cudaGetDevice(&b->device));
-    if (!st) st = cuda_status(cudaDeviceGetAttribute(&b->sms, cudaDevAttrMultiProcessorCount, b->device));
-    if (!st) st = cuda_status(cudaMalloc(&b->d_phi, phi.size() * sizeof(float)));
-    if (!st) st = cuda_status(cudaMemcpy(b->d_phi, phi.data(), phi.size() * sizeof(float), cudaMemcpyHostToDevice));
-    if (!st) st = cuda_status(cudaMalloc(&b->d_state, sizeof(IirLaunchState)));
-    if (!st) st = cuda_status(cudaMemset(b->d_state, 0, sizeof(IirLaunchState)));
-    if (!st) st = batch_alloc_segments(b, max_segments);
-    if (!st) st = batch_alloc_carry(b, max_chunks, b->seg_cap);
-    for (int i = 0; i < 2 && !st; ++i) st = cuda_status(cudaEventCreateWithFlags(&b->stage_done[i], cudaEventDisableTiming));
-    if (!st) st = shape_prepare(b, 0);
-    if (st) {
-        batch_free(b);
-        return st;
-    }
-    *out = b;
-    return IIR_OK;
+    int st = cuda_status(cudaEventRecord(b->fork, stream));
+    if (!st) st = cuda_status(cudaStreamWaitEvent(b->side, b->fork, 0));
+    if (!st) st = lookback(b->side);
+    const int side = cuda_status(cudaEventRecord(b->join, b->side));
+    if (!st) st = sweep(stream);
+    if (!side) cudaStreamWaitEvent(stream, b->join, 0);
+    return st ? st : side;
 }
 
-int iir_batch_set_shape(iir_batch* b, int rows, int samples_per_row) {
-    if (!b) return IIR_ERR_INVALID_ARGUMENT;
-    for (size_t k = 0; k < shapes().size(); ++k) {
-        if (shapes()[k].rows == rows && shapes()[k].n == samples_per_row) {
-            const int st = shape_prepare(b, static_cast<int>(k));
-            if (st) return st;
-            b->shape = static_cast<int>(k);
-            return IIR_OK;
-        }
-    }
-    return IIR_ERR_UNSUPPORTED;
-}
-
-int iir_batch_get_shape(const iir_batch* b, int* rows, int* samples_per_row, int* threads, int* regs_per_thread,
-                        int* smem_bytes, int* blocks_per_sm) {
-    if (!b) return IIR_ERR_INVALID_ARGUMENT;
-    const ShapeDef& sd = shapes()[static_cast<size_t>(b->shape)];
-    const ShapeData& d = b->shape_data[static_cast<size_t>(b->shape)];
-    if (rows) *rows = sd.rows;
-    if (samples_per_row) *samples_per_row = sd.n;
-    if (threads) *threads = sd.threads;
-    if (regs_per_thread) *regs_per_thread = d.regs;
-    if (smem_bytes) *smem_bytes = static_cast<int>(sd.smem);
-    if (blocks_per_sm) *blocks_per_sm = d.blocks_per_sm;
-    return IIR_OK;
-}
-
-int iir_batch_execute(iir_batch* b, const iir_segment* segs, int n_segs, void* stream_) {
-    if (!b || n_segs < 0 || (n_segs > 0 && !segs)) return IIR_ERR_INVALID_ARGUMENT;
-    cudaStream_t stream = static_cast<cudaStream_t>(stream_);
-    const int k = b->shape;
-    // validate and count chunks
-    size_t total = 0, groups = 0;
+// Arguments of every segment, and the number of chunks (of the current shape) within bounds.
+int check_segments(const iir_batch* b, const iir_segment* segs, int n_segs) {
+    size_t total = 0;
     for (int i = 0; i < n_segs; ++i) {
         const iir_segment& s = segs[i];
         if (s.filter < 0 || s.filter >= b->n_filters) return IIR_ERR_INVALID_ARGUMENT;
@@ -845,12 +1083,22 @@ int iir_batch_execute(iir_batch* b, const iir_segment* segs, int n_segs, void* s
         const char* xb = reinterpret_cast<const char*>(s.x);
         const char* yb = reinterpret_cast<const char*>(s.y);
         if (s.n > 0 && xb < yb + s.n * sizeof(float) && yb < xb + s.n * sizeof(float)) return IIR_ERR_INVALID_ARGUMENT;
-        const size_t ch = seg_chunks(s, k);
+        total += seg_chunks(s, b->shape);
+        if (total > 0x7fffffffull) return IIR_ERR_TOO_LARGE;
+    }
+    return IIR_OK;
+}
+
+// Segments (checked) on the lookback kernel: their table to the device, and the launch.
+int lookback_execute(iir_batch* b, const iir_segment* segs, int n_segs, bool all, cudaStream_t stream) {
+    const int k = b->shape;
+    if (const int st = shape_prepare(b, k, all)) return st;
+    size_t total = 0, groups = 0;
+    for (int i = 0; i < n_segs; ++i) {
+        const size_t ch = seg_chunks(segs[i], k);
         total += ch;
         groups += (ch + IIR_GROUP - 1) / IIR_GROUP;
     }
-    if (total == 0) return IIR_OK;
-    if (total > 0x7fffffffull) return IIR_ERR_TOO_LARGE;
     if (static_cast<size_t>(n_segs) > b->seg_cap) {
         cudaStreamSynchronize(stream);
         const int st = batch_alloc_segments(b, static_cast<size_t>(n_segs) * 2);
@@ -898,6 +1146,132 @@ int iir_batch_execute(iir_batch* b, const iir_segment* segs, int n_segs, void* s
     return batch_launch(b, k, q, stream);
 }
 
+}  // namespace
+
+extern "C" {
+
+int iir_batch_create(iir_batch** out, const float* sos, const int* n_sections, int n_filters, size_t max_segments,
+                     size_t max_chunks) {
+    if (!out || !sos || !n_sections || n_filters < 1) return IIR_ERR_INVALID_ARGUMENT;
+    *out = nullptr;
+    iir_batch* b = new iir_batch();
+    b->n_filters = n_filters;
+    b->filters.resize(static_cast<size_t>(n_filters));
+    b->tail_need.assign(static_cast<size_t>(n_filters), 0);
+    int max_sec = 1;
+    size_t off = 0;
+    for (int f = 0; f < n_filters; ++f) {
+        const int ns = n_sections[f];
+        if (ns < 1 || ns > IIR_MAX_SECTIONS) {
+            delete b;
+            return IIR_ERR_INVALID_ARGUMENT;
+        }
+        SectionF32 s32[IIR_MAX_SECTIONS];
+        double gain = 1.0;
+        int st = normalise_sos(sos + 6 * off, ns, s32, gain);
+        if (st) {
+            delete b;
+            return st;
+        }
+        // the sections' scalars and lane tables depend on the chunk shape: shape_prepare builds them
+        b->filters[static_cast<size_t>(f)] =
+            IirBatchFilter{static_cast<float>(gain), ns, static_cast<int>(b->sec32.size()), 0};
+        b->gains.push_back(gain);
+        for (int k = 0; k < ns; ++k) b->sec32.push_back(s32[k]);
+        max_sec = std::max(max_sec, ns);
+        off += static_cast<size_t>(ns);
+    }
+    b->max_sections = max_sec;
+    b->filter_sections.assign(n_sections, n_sections + n_filters);
+    b->shape_data.resize(shapes().size());
+    int st = cuda_status(cudaGetDevice(&b->device));
+    if (!st) st = cuda_status(cudaDeviceGetAttribute(&b->sms, cudaDevAttrMultiProcessorCount, b->device));
+    if (!st) st = cuda_status(cudaMalloc(&b->d_state, sizeof(IirLaunchState)));
+    if (!st) st = cuda_status(cudaMemset(b->d_state, 0, sizeof(IirLaunchState)));
+    if (!st) st = cuda_status(cudaMalloc(&b->d_sweep_state, sizeof(IirLaunchState)));
+    if (!st) st = cuda_status(cudaMemset(b->d_sweep_state, 0, sizeof(IirLaunchState)));
+    if (!st) st = cuda_status(cudaStreamCreateWithFlags(&b->side, cudaStreamNonBlocking));
+    if (!st) st = cuda_status(cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming));
+    if (!st) st = cuda_status(cudaEventCreateWithFlags(&b->join, cudaEventDisableTiming));
+    if (!st) st = batch_alloc_segments(b, max_segments);
+    if (!st) st = batch_alloc_runs(b, sweep_run_capacity(b, b->seg_cap, max_chunks));
+    if (!st) st = batch_alloc_carry(b, max_chunks, b->seg_cap);
+    for (int i = 0; i < 2 && !st; ++i) {
+        st = cuda_status(cudaEventCreateWithFlags(&b->stage_done[i], cudaEventDisableTiming));
+        if (!st) st = cuda_status(cudaEventCreateWithFlags(&b->run_done[i], cudaEventDisableTiming));
+    }
+    if (!st) st = shape_measure(b, 0);
+    if (!st) st = sweep_prepare(b, 0);
+    // the lookback kernel's tables at once where a segment may need it, else at its first launch
+    if (!st && !(b->sweep[0].covers && sweep_enabled())) st = shape_prepare(b, 0, !sweep_enabled());
+    if (st) {
+        batch_free(b);
+        return st;
+    }
+    *out = b;
+    return IIR_OK;
+}
+
+int iir_batch_set_shape(iir_batch* b, int rows, int samples_per_row) {
+    if (!b) return IIR_ERR_INVALID_ARGUMENT;
+    for (size_t k = 0; k < shapes().size(); ++k) {
+        if (shapes()[k].rows == rows && shapes()[k].n == samples_per_row) {
+            const int st = b->sweep[0].covers && sweep_enabled()
+                               ? shape_measure(b, static_cast<int>(k))
+                               : shape_prepare(b, static_cast<int>(k), !sweep_enabled());
+            if (st) return st;
+            b->shape = static_cast<int>(k);
+            return IIR_OK;
+        }
+    }
+    return IIR_ERR_UNSUPPORTED;
+}
+
+int iir_batch_get_shape(const iir_batch* b, int* rows, int* samples_per_row, int* threads, int* regs_per_thread,
+                        int* smem_bytes, int* blocks_per_sm) {
+    if (!b) return IIR_ERR_INVALID_ARGUMENT;
+    const ShapeDef& sd = shapes()[static_cast<size_t>(b->shape)];
+    const ShapeData& d = b->shape_data[static_cast<size_t>(b->shape)];
+    if (rows) *rows = sd.rows;
+    if (samples_per_row) *samples_per_row = sd.n;
+    if (threads) *threads = sd.threads;
+    if (regs_per_thread) *regs_per_thread = d.regs;
+    if (smem_bytes) *smem_bytes = static_cast<int>(sd.smem);
+    if (blocks_per_sm) *blocks_per_sm = d.blocks_per_sm;
+    return IIR_OK;
+}
+
+int iir_batch_execute(iir_batch* b, const iir_segment* segs, int n_segs, void* stream_) {
+    if (!b || n_segs < 0 || (n_segs > 0 && !segs)) return IIR_ERR_INVALID_ARGUMENT;
+    cudaStream_t stream = static_cast<cudaStream_t>(stream_);
+    if (const int st = check_segments(b, segs, n_segs)) return st;
+    Schedule c;
+    int st = make_schedule(b, segs, n_segs, b->withhold >= 0, stream, c);
+    if (st) return st;
+    if (c.runs > b->run_cap) {
+        cudaStreamSynchronize(stream);
+        st = batch_alloc_runs(b, 2 * c.runs);
+        if (st) return st;
+    }
+    auto lookback = [&](cudaStream_t s) {
+        return c.rest.empty() ? IIR_OK : lookback_execute(b, c.rest.data(), static_cast<int>(c.rest.size()), !c.sweep || c.v != 0, s);
+    };
+    auto sweep = [&](cudaStream_t s) {
+        if (c.runs == 0) return static_cast<int>(IIR_OK);
+        const int turn = b->run_turn;
+        b->run_turn ^= 1;
+        int r = cuda_status(cudaEventSynchronize(b->run_done[turn]));
+        if (r) return r;
+        sweep_runs(b, c, segs, b->h_runs[turn]);
+        r = cuda_status(cudaMemcpyAsync(b->d_runs, b->h_runs[turn], c.runs * sizeof(BatchRun), cudaMemcpyHostToDevice, s));
+        if (!r) r = cuda_status(cudaEventRecord(b->run_done[turn], s));
+        if (r) return r;
+        IirBatchSweepParams q = sweep_params(b, c, segs);
+        return sweep_launch(b, c.v, q, b->d_runs, s);
+    };
+    return launch_both(b, stream, c.runs > 0 && !c.rest.empty(), lookback, sweep);
+}
+
 struct iir_batch_bound {
     iir_batch* b = nullptr;
     int shape = 0;
@@ -906,85 +1280,109 @@ struct iir_batch_bound {
     unsigned int* d_chunk_seg = nullptr;  // each chunk's segment: no search in the launch
     IirBatchParams params{};
     unsigned int nchunks = 0;
+    // the segments on the state sweep (the fields above: those on the lookback kernel)
+    int v = 0;
+    BatchRun* d_runs = nullptr;
+    size_t runs = 0;
+    IirBatchSweepParams sweep{};
 };
 
-int iir_batch_bind(iir_batch* b, const iir_segment* segs, int n_segs, iir_batch_bound** out) {
-    if (!b || !out || n_segs < 0 || (n_segs > 0 && !segs)) return IIR_ERR_INVALID_ARGUMENT;
+int iir_batch_bind(iir_batch* b, const iir_segment* all, int n_all, iir_batch_bound** out) {
+    if (!b || !out || n_all < 0 || (n_all > 0 && !all)) return IIR_ERR_INVALID_ARGUMENT;
     *out = nullptr;
     const int k = b->shape;
-    std::vector<IirBatchSegment> hs(static_cast<size_t>(std::max(n_segs, 1)));
-    std::vector<unsigned int> starts(static_cast<size_t>(n_segs) + 1);
-    size_t chunk0 = 0, group0 = 0;
-    const size_t tail_min = batch_tail_min_chunks();
-    for (int i = 0; i < n_segs; ++i) {
-        const iir_segment& s = segs[i];
-        if (s.filter < 0 || s.filter >= b->n_filters) return IIR_ERR_INVALID_ARGUMENT;
-        if (s.n > 0 && (!s.x || !s.y)) return IIR_ERR_INVALID_ARGUMENT;
-        if (s.n > (1ull << 40)) return IIR_ERR_TOO_LARGE;
-        const char* xb = reinterpret_cast<const char*>(s.x);
-        const char* yb = reinterpret_cast<const char*>(s.y);
-        if (s.n > 0 && xb < yb + s.n * sizeof(float) && yb < xb + s.n * sizeof(float)) return IIR_ERR_INVALID_ARGUMENT;
-        const size_t ch = seg_chunks(s, k);
-        hs[i] = IirBatchSegment{s.x, s.y, static_cast<long long>(s.n), s.zi, s.zf, static_cast<unsigned int>(chunk0),
-                                static_cast<unsigned int>(group0), s.filter, ch >= tail_min ? 1 : 0, seg_lead(s), 0};
-        starts[i] = static_cast<unsigned int>(chunk0);
-        chunk0 += ch;
-        group0 += (ch + IIR_GROUP - 1) / IIR_GROUP;
-        if (chunk0 > 0x7fffffffull) return IIR_ERR_TOO_LARGE;
-    }
-    starts[n_segs] = static_cast<unsigned int>(chunk0);
-    // each chunk's segment (the last of equal starts: empty segments have no chunks)
-    std::vector<unsigned int> cseg(std::max<size_t>(chunk0, 1), 0u);
-    for (int i = 0; i < n_segs; ++i)
-        for (unsigned int c = starts[i]; c < starts[i + 1]; ++c) cseg[c] = static_cast<unsigned int>(i);
-    int st = cuda_status(cudaDeviceSynchronize());
+    if (const int st = check_segments(b, all, n_all)) return st;
+    Schedule c;
+    int st = make_schedule(b, all, n_all, false, nullptr, c);  // (a bound launch takes no injected fault)
     if (st) return st;
-    if (chunk0 > b->carry_cap || group0 > b->gcap) {
-        st = batch_alloc_carry(b, std::max(chunk0, b->carry_cap * 2), std::max<size_t>(n_segs, group0));
-        if (st) return st;
-    }
+    const iir_segment* segs = c.rest.data();
+    const int n_segs = static_cast<int>(c.rest.size());
+    if (n_segs > 0) st = shape_prepare(b, k, !c.sweep || c.v != 0);
+    if (!st) st = cuda_status(cudaDeviceSynchronize());
+    if (st) return st;
     iir_batch_bound* h = new iir_batch_bound();
     h->b = b;
     h->shape = k;
-    h->nchunks = static_cast<unsigned int>(chunk0);
-    st = cuda_status(cudaMalloc(&h->d_segs, hs.size() * sizeof(IirBatchSegment)));
-    if (!st) st = cuda_status(cudaMalloc(&h->d_starts, starts.size() * sizeof(unsigned int)));
-    if (!st) st = cuda_status(cudaMalloc(&h->d_chunk_seg, cseg.size() * sizeof(unsigned int)));
-    if (!st)
-        st = cuda_status(
-            cudaMemcpy(h->d_chunk_seg, cseg.data(), cseg.size() * sizeof(unsigned int), cudaMemcpyHostToDevice));
-    if (!st)
-        st = cuda_status(cudaMemcpy(h->d_segs, hs.data(), hs.size() * sizeof(IirBatchSegment), cudaMemcpyHostToDevice));
-    if (!st)
-        st = cuda_status(
-            cudaMemcpy(h->d_starts, starts.data(), starts.size() * sizeof(unsigned int), cudaMemcpyHostToDevice));
+    h->v = c.v;
+    h->runs = c.runs;
+    if (c.runs > 0) {
+        std::vector<BatchRun> runs(c.runs);
+        sweep_runs(b, c, all, runs.data());
+        h->sweep = sweep_params(b, c, all);
+        // the costly runs first: they set when the launch ends
+        std::stable_sort(runs.begin(), runs.end(), [](const BatchRun& p, const BatchRun& q) {
+            return static_cast<size_t>(p.K) * p.count > static_cast<size_t>(q.K) * q.count;
+        });
+        st = cuda_status(cudaMalloc(&h->d_runs, runs.size() * sizeof(BatchRun)));
+        if (!st)
+            st = cuda_status(cudaMemcpy(h->d_runs, runs.data(), runs.size() * sizeof(BatchRun), cudaMemcpyHostToDevice));
+    }
+    if (!st && n_segs > 0) {
+        std::vector<IirBatchSegment> hs(static_cast<size_t>(n_segs));
+        std::vector<unsigned int> starts(static_cast<size_t>(n_segs) + 1);
+        size_t chunk0 = 0, group0 = 0;
+        const size_t tail_min = batch_tail_min_chunks();
+        for (int i = 0; i < n_segs; ++i) {
+            const iir_segment& s = segs[i];
+            const size_t ch = seg_chunks(s, k);
+            hs[i] =
+                IirBatchSegment{s.x, s.y, static_cast<long long>(s.n), s.zi, s.zf, static_cast<unsigned int>(chunk0),
+                                static_cast<unsigned int>(group0), s.filter, ch >= tail_min ? 1 : 0, seg_lead(s), 0};
+            starts[i] = static_cast<unsigned int>(chunk0);
+            chunk0 += ch;
+            group0 += (ch + IIR_GROUP - 1) / IIR_GROUP;
+        }
+        starts[n_segs] = static_cast<unsigned int>(chunk0);
+        // each chunk's segment (the last of equal starts: empty segments have no chunks)
+        std::vector<unsigned int> cseg(std::max<size_t>(chunk0, 1), 0u);
+        for (int i = 0; i < n_segs; ++i)
+            for (unsigned int q = starts[i]; q < starts[i + 1]; ++q) cseg[q] = static_cast<unsigned int>(i);
+        if (chunk0 > b->carry_cap || group0 > b->gcap)
+            st = batch_alloc_carry(b, std::max(chunk0, b->carry_cap * 2), std::max<size_t>(n_segs, group0));
+        h->nchunks = static_cast<unsigned int>(chunk0);
+        if (!st) st = cuda_status(cudaMalloc(&h->d_segs, hs.size() * sizeof(IirBatchSegment)));
+        if (!st) st = cuda_status(cudaMalloc(&h->d_starts, starts.size() * sizeof(unsigned int)));
+        if (!st) st = cuda_status(cudaMalloc(&h->d_chunk_seg, cseg.size() * sizeof(unsigned int)));
+        if (!st)
+            st = cuda_status(
+                cudaMemcpy(h->d_chunk_seg, cseg.data(), cseg.size() * sizeof(unsigned int), cudaMemcpyHostToDevice));
+        if (!st)
+            st = cuda_status(cudaMemcpy(h->d_segs, hs.data(), hs.size() * sizeof(IirBatchSegment), cudaMemcpyHostToDevice));
+        if (!st)
+            st = cuda_status(
+                cudaMemcpy(h->d_starts, starts.data(), starts.size() * sizeof(unsigned int), cudaMemcpyHostToDevice));
+    }
     if (st) {
-        if (h->d_segs) cudaFree(h->d_segs);
-        if (h->d_starts) cudaFree(h->d_starts);
-        if (h->d_chunk_seg) cudaFree(h->d_chunk_seg);
-        delete h;
+        iir_batch_unbind(h);
         return st;
     }
-    h->params = batch_params(b, k, h->d_segs, h->d_starts, static_cast<unsigned int>(n_segs), h->nchunks, -1);
-    h->params.chunk_seg = h->d_chunk_seg;
+    if (n_segs > 0) {
+        h->params = batch_params(b, k, h->d_segs, h->d_starts, static_cast<unsigned int>(n_segs), h->nchunks, -1);
+        h->params.chunk_seg = h->d_chunk_seg;
+    }
     *out = h;
     return IIR_OK;
 }
 
 int iir_batch_launch_bound(iir_batch_bound* h, void* stream_) {
     if (!h) return IIR_ERR_INVALID_ARGUMENT;
-    if (h->nchunks == 0) return IIR_OK;
     iir_batch* b = h->b;
     // the carry slots must still be the ones bound (a later execute that grew them rebinds)
-    if (h->params.carry != b->d_carry) return IIR_ERR_INVALID_ARGUMENT;
-    cudaStream_t stream = static_cast<cudaStream_t>(stream_);
-    if (++b->launches >= (1ull << 30)) {
-        int st = cuda_status(cudaMemsetAsync(b->d_carry, 0, b->carry_bytes, stream));
-        if (!st) st = cuda_status(cudaMemsetAsync(b->d_state, 0, IIR_STATE_RESET_BYTES, stream));
-        if (st) return st;
-        b->launches = 1;
-    }
-    return batch_launch(b, h->shape, h->params, stream);
+    if (h->nchunks > 0 && h->params.carry != b->d_carry) return IIR_ERR_INVALID_ARGUMENT;
+    auto lookback = [&](cudaStream_t s) {
+        if (h->nchunks == 0) return static_cast<int>(IIR_OK);
+        if (++b->launches >= (1ull << 30)) {
+            int st = cuda_status(cudaMemsetAsync(b->d_carry, 0, b->carry_bytes, s));
+            if (!st) st = cuda_status(cudaMemsetAsync(b->d_state, 0, IIR_STATE_RESET_BYTES, s));
+            if (st) return st;
+            b->launches = 1;
+        }
+        return batch_launch(b, h->shape, h->params, s);
+    };
+    auto sweep = [&](cudaStream_t s) {
+        return h->runs > 0 ? sweep_launch(b, h->v, h->sweep, h->d_runs, s) : static_cast<int>(IIR_OK);
+    };
+    return launch_both(b, static_cast<cudaStream_t>(stream_), h->runs > 0 && h->nchunks > 0, lookback, sweep);
 }
 
 int iir_batch_unbind(iir_batch_bound* h) {
@@ -993,6 +1391,7 @@ int iir_batch_unbind(iir_batch_bound* h) {
     cudaFree(h->d_segs);
     cudaFree(h->d_starts);
     cudaFree(h->d_chunk_seg);
+    cudaFree(h->d_runs);
     delete h;
     return IIR_OK;
 }
@@ -1002,14 +1401,18 @@ int iir_batch_check(iir_batch* b, void* stream_) {
     cudaStream_t stream = static_cast<cudaStream_t>(stream_);
     int st = cuda_status(cudaStreamSynchronize(stream));
     if (st) return st;
-    IirLaunchState hs;
-    st = cuda_status(cudaMemcpy(&hs, b->d_state, sizeof(hs), cudaMemcpyDeviceToHost));
-    if (st) return st;
-    if (hs.error == 0ull) return IIR_OK;
-    const unsigned long long zero = 0ull;
-    cudaMemcpy(reinterpret_cast<char*>(b->d_state) + offsetof(IirLaunchState, error), &zero, sizeof(zero),
-               cudaMemcpyHostToDevice);
-    return device_error_status(hs.error);
+    int found = IIR_OK;
+    for (IirLaunchState* state : {b->d_state, b->d_sweep_state}) {
+        IirLaunchState hs;
+        st = cuda_status(cudaMemcpy(&hs, state, sizeof(hs), cudaMemcpyDeviceToHost));
+        if (st) return st;
+        if (hs.error == 0ull) continue;
+        const unsigned long long zero = 0ull;
+        cudaMemcpy(reinterpret_cast<char*>(state) + offsetof(IirLaunchState, error), &zero, sizeof(zero),
+                   cudaMemcpyHostToDevice);
+        if (!found) found = device_error_status(hs.error);
+    }
+    return found;
 }
 
 int iir_batch_set_timeout_ns(iir_batch* b, long long timeout_ns) {

@@ -1,0 +1,15 @@
+// iir_batch_sweep2.cu — batch kernels on the state sweep for filters of up to 2 sections.
+#include "iir_batch_sweep.cuh"
+#include "iir_batch_sweep.h"
+namespace iirhost {
+
+void bsweep_kernels2(std::vector<BatchSweepKernel>& v) {
+    using namespace iirgb;
+    // tiles of 4096 samples, as many buffers as shared memory holds with a table each; 1024 for short segments
+    v.push_back({2, 128, 32 * (8 + 1 + BSWEEP_COPIERS),
+                 reinterpret_cast<const void*>(iir_batch_sweep_kernel<2, 128, 8, 12>), bsweep_smem<2, 128, 12>()});
+    v.push_back({2, 32, 32 * (8 + 1 + BSWEEP_COPIERS),
+                 reinterpret_cast<const void*>(iir_batch_sweep_kernel<2, 32, 8, 15>), bsweep_smem<2, 32, 15>()});
+}
+
+}  // namespace iirhost

@@ -2,6 +2,7 @@
 // translation units of the library (not part of the C ABI).
 #pragma once
 #include <cuda.h>
+#include <cudaTypedefs.h>
 #include <cuda_runtime.h>
 
 #include <vector>
@@ -29,6 +30,8 @@ int normalise_sos(const float* sos, int n_sections, SectionF32* out, double& gai
 int tail_pieces(const SectionF32* secs, int K, int max_pieces, std::vector<float>& piece_phi);
 // One section's kernel coefficients and its IIR_TAB_STRIDE lane-table entries.
 int precompute_section(const SectionF32& s, int kind, int rows, int N, IirSection& q, float4* tab);
+// cuTensorMapEncodeTiled through the runtime (null if the driver lacks it).
+PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder();
 // 2D tensor map over a float32 signal viewed as 128-byte lines, box = lines_per_block lines.
 bool encode_lines_map(CUtensorMap* map, const float* base, long long n, int lines_per_block);
 // 2D tensor map over rows of row_len floats, box {box_inner, box_rows}, 128-byte swizzle.

@@ -6,6 +6,7 @@
 #include <cmath>
 #include <mutex>
 
+#include "iir_batch_sweep.h"
 #include "iir_sweep.h"
 
 namespace iirgb {
@@ -122,6 +123,32 @@ std::vector<std::vector<double>> impulse_states(const std::vector<SectionF32>& s
     return p;
 }
 
+// Pass A's tables, [2K][N] dot products at 0 and the response to the input history at t_h.
+void put_dots(std::vector<float>& t, const SweepFilter& f, int N, size_t t_h) {
+    const int K = f.K;
+    const std::vector<std::vector<double>> p = impulse_states(f.secs, N);
+    auto ps = [&](int s, int n) { return n >= 0 ? p[static_cast<size_t>(s)][static_cast<size_t>(n)] : 0.0; };
+    const double b1 = f.secs[0].b1, b2 = f.secs[0].b2, g = f.gain;
+    for (int s = 0; s < K; ++s) {
+        float* t0 = t.data() + static_cast<size_t>(2 * s) * N;  // y[N-1] - y[N-2]
+        float* t1 = t0 + N;                                      // y[N-1]
+        auto h = [&](int m) { return g * (ps(s, m) + b1 * ps(s, m - 1) + b2 * ps(s, m - 2)); };  // impulse response
+        for (int n = 0; n < N; ++n) {
+            const double y1 = h(N - 1 - n), y2 = h(N - 2 - n);
+            t0[n] = static_cast<float>(y1 - y2);
+            t1[n] = static_cast<float>(y1);
+        }
+        // (x[-2], x[-1]) reach the sub-row through section 0's FIR taps
+        auto h2 = [&](int m) { return g * b2 * ps(s, m); };
+        auto h1 = [&](int m) { return g * (b1 * ps(s, m) + b2 * ps(s, m - 1)); };
+        float* th = t.data() + t_h + 4 * s;
+        th[0] = static_cast<float>(h2(N - 1) - h2(N - 2));
+        th[1] = static_cast<float>(h1(N - 1) - h1(N - 2));
+        th[2] = static_cast<float>(h2(N - 1));
+        th[3] = static_cast<float>(h1(N - 1));
+    }
+}
+
 }  // namespace
 
 std::vector<const SweepKernel*> sweep_kernels(int kind, int K) {
@@ -154,8 +181,17 @@ SweepFilter sweep_filter(const SectionF32* secs, int K, double gain) {
         for (int j = 0; j < D; ++j) f.phi[static_cast<size_t>(2 * s + 1) * D + j] = row[j];
         prev = row;
     }
-    // energy of every section's impulse response over the longest halo considered
-    const std::vector<std::vector<double>> p = impulse_states(f.secs, 4096);
+    // energy of every section's impulse response, over as many samples as most of it takes
+    std::vector<std::vector<double>> p;
+    for (const int len : {512, 4096, 65536}) {
+        p = impulse_states(f.secs, len);
+        double peak = 0.0, tail = 0.0;
+        for (int n = 0; n < len; ++n) {
+            const double v = std::fabs(p.back()[static_cast<size_t>(n)]);
+            (8 * n < 7 * len ? peak : tail) = std::max(8 * n < 7 * len ? peak : tail, v);
+        }
+        if (!(tail > 1e-3 * peak)) break;
+    }
     f.scale.assign(static_cast<size_t>(K), 1.0);
     for (int s = 0; s < K; ++s) {
         double e = 0.0;
@@ -188,31 +224,11 @@ int sweep_decay(const SweepFilter& f, int unit, int most) {
 
 std::vector<float> sweep_tables(const SweepFilter& f, int N, int R) {
     const int K = f.K, D = 2 * K, span = N * R;
-    const std::vector<std::vector<double>> p = impulse_states(f.secs, N);
-    auto ps = [&](int s, int n) { return n >= 0 ? p[static_cast<size_t>(s)][static_cast<size_t>(n)] : 0.0; };
-    const double b1 = f.secs[0].b1, b2 = f.secs[0].b2, g = f.gain;
     const int blocks = K * (K + 1) / 2;
     const size_t t_h = static_cast<size_t>(D) * N, t_pn = (t_h + 2 * D + 3) & ~size_t(3),
                  t_pl = t_pn + 4 * static_cast<size_t>(blocks);
     std::vector<float> t(t_pl + 4 * static_cast<size_t>(SWEEP_LANES) * blocks, 0.f);
-    for (int s = 0; s < K; ++s) {
-        float* t0 = t.data() + static_cast<size_t>(2 * s) * N;  // y[N-1] - y[N-2]
-        float* t1 = t0 + N;                                      // y[N-1]
-        auto h = [&](int m) { return g * (ps(s, m) + b1 * ps(s, m - 1) + b2 * ps(s, m - 2)); };  // impulse response
-        for (int n = 0; n < N; ++n) {
-            const double y1 = h(N - 1 - n), y2 = h(N - 2 - n);
-            t0[n] = static_cast<float>(y1 - y2);
-            t1[n] = static_cast<float>(y1);
-        }
-        // (x[-2], x[-1]) reach the sub-row through section 0's FIR taps
-        auto h2 = [&](int m) { return g * b2 * ps(s, m); };
-        auto h1 = [&](int m) { return g * (b1 * ps(s, m) + b2 * ps(s, m - 1)); };
-        float* th = t.data() + t_h + 4 * s;
-        th[0] = static_cast<float>(h2(N - 1) - h2(N - 2));
-        th[1] = static_cast<float>(h1(N - 1) - h1(N - 2));
-        th[2] = static_cast<float>(h2(N - 1));
-        th[3] = static_cast<float>(h1(N - 1));
-    }
+    put_dots(t, f, N, t_h);
     auto put = [&](size_t at, const Mat& m) {
         for (int s = 0; s < K; ++s)
             for (int q = 0; q <= s; ++q) put_block(t, at + 4 * static_cast<size_t>(s * (s + 1) / 2 + q), m, D, s, q);
@@ -225,6 +241,82 @@ std::vector<float> sweep_tables(const SweepFilter& f, int N, int R) {
         pl = mat_mul(pl, step, D);
     }
     return t;
+}
+
+BatchSweepFilter bsweep_filter(const SectionF32* secs, int K, double gain, int span) {
+    // the compiled number of sections: those past the filter's own pass their input on
+    const int KP = bsweep_sections(K);
+    std::vector<SectionF32> padded(secs, secs + K);
+    padded.resize(static_cast<size_t>(KP), SectionF32{0.f, 0.f, 0.f, 0.f});
+    const SweepFilter f = sweep_filter(padded.data(), KP, gain);
+    const int D = 2 * KP, N = bsweep_subrow(KP, span), blocks = KP * (KP + 1) / 2;
+    auto log2i = [](int v) {
+        int l = 0;
+        while ((1 << l) < v) ++l;
+        return l;
+    };
+    // squares of the one-sample transition (block lower triangular)
+    std::vector<Mat> sq{f.phi};
+    auto power = [&](int k) -> const Mat& {  // Phi^(2^k)
+        while (static_cast<int>(sq.size()) <= k) {
+            const Mat& a = sq.back();
+            Mat r(static_cast<size_t>(D) * D, 0.0);
+            for (int i = 0; i < D; ++i)
+                for (int m = 0; m <= (i | 1); ++m) {
+                    const double v = a[static_cast<size_t>(i) * D + m];
+                    for (int j = 0; j <= (m | 1); ++j)
+                        r[static_cast<size_t>(i) * D + j] += v * a[static_cast<size_t>(m) * D + j];
+                }
+            sq.push_back(std::move(r));
+        }
+        return sq[static_cast<size_t>(k)];
+    };
+    auto decayed = [&](const Mat& m) {
+        for (int i = 0; i < D; ++i) {
+            double r = 0.0;
+            for (int j = 0; j <= (i | 1); ++j)
+                r += std::fabs(m[static_cast<size_t>(i) * D + j]) * f.scale[static_cast<size_t>(j / 2)] /
+                     f.scale[static_cast<size_t>(i / 2)];
+            if (!(r <= 1e-10)) return false;
+        }
+        return true;
+    };
+    BatchSweepFilter out;
+    const int ls = log2i(span);
+    int k = 0;
+    while (k <= 5 && !decayed(power(ls + k))) ++k;
+    if (k > 5) return out;
+    out.rounds = k;
+    out.fast = true;
+    const size_t t_h = static_cast<size_t>(D) * N, t_c = t_h + 2 * D, t_pn = t_c + 4 * KP + 4,
+                 t_ps = t_pn + 4 * static_cast<size_t>(blocks);
+    std::vector<float>& t = out.table;
+    t.assign(static_cast<size_t>(bsweep_table_floats(KP, span)), 0.f);
+    put_dots(t, f, N, t_h);
+    for (int s = 0; s < KP; ++s) {
+        // the first section's input is the raw sample: its FIR taps carry the gain
+        float* c = t.data() + t_c + 4 * s;
+        c[0] = static_cast<float>(s == 0 ? gain * padded[0].b1 : padded[static_cast<size_t>(s)].b1);
+        c[1] = static_cast<float>(s == 0 ? gain * padded[0].b2 : padded[static_cast<size_t>(s)].b2);
+        c[2] = padded[static_cast<size_t>(s)].a1;
+        c[3] = padded[static_cast<size_t>(s)].a2;
+    }
+    t[t_c + 4 * static_cast<size_t>(KP)] = static_cast<float>(gain);
+    auto put = [&](size_t at, const Mat& m) {
+        for (int s = 0; s < KP; ++s)
+            for (int q = 0; q <= s; ++q) put_block(t, at + 4 * static_cast<size_t>(s * (s + 1) / 2 + q), m, D, s, q);
+    };
+    put(t_pn, power(log2i(N)));
+    for (int j = 0; j < BSWEEP_STEPS; ++j) put(t_ps + 4 * static_cast<size_t>(j) * blocks, power(ls + j));
+    if (!bsweep_chained(KP)) {
+        const size_t t_pl = t_ps + 4 * static_cast<size_t>(BSWEEP_STEPS) * blocks;
+        Mat pl = mat_pow(f.phi, 0, D);
+        for (int l = 0; l < BSWEEP_NEAR; ++l) {
+            put(t_pl + 4 * static_cast<size_t>(l) * blocks, pl);
+            if (l + 1 < BSWEEP_NEAR) pl = mat_mul(pl, power(ls), D);
+        }
+    }
+    return out;
 }
 
 }  // namespace iirhost

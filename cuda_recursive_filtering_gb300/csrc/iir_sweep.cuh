@@ -90,6 +90,14 @@ __device__ __forceinline__ int tile_at(int l, int n) {
     return ((n >> 5) << 10) + (l << 5) + ((((n >> 2) & 7) ^ (l & 7)) << 2) + (n & 3);
 }
 
+// Float offset of granule j (samples 4j .. 4j + 3) of sub-row i (N samples) from the lane's line, l7 =
+// lane & 7: one address per j serves every sub-row.
+template <int N>
+__device__ __forceinline__ int sub_granule_at(int i, int j, int l7) {
+    if constexpr (N % 32 == 0) return ((j >> 3) << 10) + (((j & 7) ^ l7) << 2) + i * (N / 32) * 1024;
+    else return (((j ^ l7) ^ ((i & 1) << 2)) << 2) + (i >> 1) * 1024;  // N = 16: two sub-rows to a line
+}
+
 // o += M v for one 2x2 block in column order: (o0, o1) += (m00, m10) v0 + (m01, m11) v1
 __device__ __forceinline__ f32x2 block_mad(const float* m, float v0, float v1, f32x2 o) {
     const ulonglong2 c = *reinterpret_cast<const ulonglong2*>(m);
@@ -128,10 +136,9 @@ __device__ __forceinline__ void sweep_dots(const float* buf, const float* tab, i
     const int l7 = lane & 7;
 #pragma unroll 4
     for (int j = 0; j < N / 4; ++j) {
-        const float* at = row + ((j >> 3) << 10) + (((j & 7) ^ l7) << 2);
         ulonglong2 x[R];
 #pragma unroll
-        for (int i = 0; i < R; ++i) x[i] = *reinterpret_cast<const ulonglong2*>(at + i * (N / 32) * 1024);
+        for (int i = 0; i < R; ++i) x[i] = *reinterpret_cast<const ulonglong2*>(row + sub_granule_at<N>(i, j, l7));
 #pragma unroll
         for (int c = 0; c < C; ++c) {
             const ulonglong2 t = *reinterpret_cast<const ulonglong2*>(ta + c * N + 4 * j);

@@ -197,18 +197,21 @@ typedef struct iir_batch iir_batch;
  * (sum of n_sections[f] rows of 6), n_sections[f] in 1..8. Capacities grow on demand. */
 int iir_batch_create(iir_batch** batch, const float* sos, const int* n_sections, int n_filters,
                      size_t max_segments, size_t max_chunks);
-/* Filters every segment in one launch on `stream`: a persistent grid draws the segments' chunks
- * from one work queue (PH solve; the decoupled lookback restricted to each segment, one carry
- * per section; with IIR_GB300_BATCH_TAIL_CHUNKS=n, segments of n chunks or more whose filter's
- * state decays within half a chunk publish one aggregate per chunk from its tail instead).
+/* Filters every segment on `stream`: a persistent grid draws runs of each segment's tiles from one
+ * work queue (state sweep). Segments whose filter takes longer than a tile to decay go to a second
+ * kernel beside it, which draws chunks (PH solve; the decoupled lookback restricted to each segment,
+ * one carry per section). That kernel takes all of them with IIR_GB300_TAIL=0 or
+ * IIR_GB300_BATCH_TAIL_CHUNKS=n (then segments of n chunks or more whose filter's state decays within
+ * half a chunk publish one aggregate per chunk from its tail).
  * Stream-ordered; launches of one batch plan must be ordered on one stream. */
 int iir_batch_execute(iir_batch* batch, const iir_segment* segs, int n_segs, void* stream);
 int iir_batch_check(iir_batch* batch, void* stream);
 /* A fixed segment table uploaded once (synchronously) for repeated launches: each
- * iir_batch_launch_bound is one kernel launch and nothing else, so it can be captured into a
- * CUDA graph and replayed. The segments' buffers must stay valid while the handle is used; an
- * iir_batch_execute that has to grow the batch's carry slots invalidates earlier handles
- * (iir_batch_launch_bound then returns IIR_ERR_INVALID_ARGUMENT). */
+ * iir_batch_launch_bound is one kernel launch, or two joined by events where both kernels have
+ * segments, and nothing else, so it can be captured into a CUDA graph and replayed. The segments'
+ * buffers must stay valid while the handle is used; an iir_batch_execute that has to grow the
+ * batch's carry slots invalidates earlier handles (iir_batch_launch_bound then returns
+ * IIR_ERR_INVALID_ARGUMENT). */
 typedef struct iir_batch_bound iir_batch_bound;
 int iir_batch_bind(iir_batch* batch, const iir_segment* segs, int n_segs, iir_batch_bound** bound);
 int iir_batch_launch_bound(iir_batch_bound* bound, void* stream);
