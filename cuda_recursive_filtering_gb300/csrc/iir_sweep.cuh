@@ -31,8 +31,8 @@
 //   order        2              4              8              16
 //   2^20     (small kernel kept) 8.8 -> 7.4   12.7 -> 8.9    21.0 -> 13.2
 //   2^23      18.2 -> 15.8   22.7 -> 16.9   31.4 -> 20.2   56.2 -> 34.4
-//   2^25      48.4 -> 44.4   59.3 -> 45.7   83.4 -> 51.6  152.1 -> 95.6
-//   2^27     163 -> 157.8   193 -> 158.2   284 -> 177.9   565 -> 345
+//   2^25      48.4 -> 44.4   59.3 -> 45.7   83.4 -> 51.5  152.1 -> 91.9
+//   2^27     163 -> 157.8   193 -> 158.2   284 -> 175.5   565 -> 333
 #pragma once
 #include "iir_pipe.cuh"
 
@@ -334,7 +334,7 @@ __device__ __forceinline__ void sweep_run_ph(float* buf, const SweepSection* sec
 //   order            2              4              8               16
 //   STCR  3e6   10.1 ->  9.4   12.4 -> 11.2   18.2 -> 14.1    31.7 ->  21.8
 //   STCR  2^25  55.9 -> 44.0   82.0 -> 47.1  128.6 -> 63.0   240.6 -> 117.2
-//   STCR  2^27 189.1 ->157.8  292.6 ->160.9  473.2 ->218.8   909.3 -> 428.0
+//   STCR  2^27 189.1 ->157.8  292.6 ->160.9  473.2 ->216.9   909.3 -> 428.0
 //   DTCR  2^25  57.0 -> 44.0  107.6 -> 47.1  187.1 -> 63.0   367.4 -> 117.2
 //   DTCR  2^27 200.1 ->157.8  403.1 ->160.9  719.8 ->219.0  1428   -> 428.1
 struct SweepCr {
@@ -502,8 +502,10 @@ struct SweepAux {
 // the response to it, Phi^(SPAN l) for lane l.
 //
 // Item i lies in buffer i % NB: the loader keeps NB - W items ahead of the warps. A warp gives its
-// buffer back when the store of its output has read it, which it looks after during its next item
-// (after pass A), or before it would wait itself.
+// buffer back when the store of its output has read it. From 3 sections on it waits for that at once,
+// so that the loads run further ahead (2^27, order 8: 177.9 -> 175.5 us, order 16: 345 -> 332.6); at 1 and
+// 2 sections, bound by memory, it looks after it during its next item (after pass A), or before it would
+// wait itself (order 4: 158.2 us, 158.7 at once).
 template <class G, int W, int NB, class Run>
 __device__ __forceinline__ void sweep_tiles(const IirSweepParams& p, unsigned char* smem, Run&& run) {
     constexpr int SPAN = G::SPAN, R = G::R, K = G::K, D = G::D;
@@ -680,7 +682,10 @@ __device__ __forceinline__ void sweep_tiles(const IirSweepParams& p, unsigned ch
                     if (base + j < p.n) p.y[base + j] = buf[tile_at(j / SPAN, j % SPAN)];
             }
             __syncwarp();
-            if (lane == 0) back = static_cast<int>(b);
+            if (lane == 0) {
+                back = static_cast<int>(b);
+                if constexpr (K >= 3) give_back();
+            }
         }
         if (lane == 0) bulk_wait_read_all();  // shared memory outlives the copies' reads
     }
