@@ -486,6 +486,7 @@ struct iir_plan {
     // State-sweep kernels (iir_sweep.cuh) of a filter that decays within a tile, the one for large
     // signals first; empty: the lookback kernels above filter every signal.
     std::vector<SweepPart> sweeps;
+    int sweep_kind = 0;  // which of the sweep kernels: the plan's kind, or SWEEP_KIND_PH_DIFF
     IirSweepParams sweep{};
 };
 
@@ -503,14 +504,27 @@ int default_geometry(int kind, int n_sections, int& B, int& N) {
     return IIR_OK;
 }
 
-// Fastest realization by order, measured on GB300 at 2^28 samples (butter(order, 0.05), N(0,1)
-// noise plus tones): PH up to order 10 (473 / 376 GS/s at orders 8 / 10; the precision form gives
-// 438 / 307); the precision form from order 12, its cost nearly flat in the order while PH's grows
-// with the sections (orders 12 / 14 / 16: 307 / 311 / 342 against 302 / 266 / 237 GS/s, with a
-// quarter of the error).
-int resolve_auto(int kernel, int n_sections) {
-    if (kernel != IIR_KERNEL_AUTO) return kernel;
-    return n_sections >= 6 ? IIR_KERNEL_TC : IIR_KERNEL_PH;
+// The realization that AUTO stands for: PH up to 5 sections (at 6 and more PH's direct form rounds more than
+// the precision form for many filters). From 6 on, PH on the state sweep, in the direct form or on
+// differences (`sweep_kind`), for filters whose float32 error there is below the precision form's: it is
+// found by doing the sweep's arithmetic on the host (within a fifth of the device's error for 40 designs of
+// orders 12 and 16), and the precision form's is 3.7e-7 to 7.4e-7 for all of them. Orders 12 / 16 at 2^27
+// samples: direct 259 / 330 us, differences 291 / 357, precision form 443 / 399; at 2^20: 11 / 13, 12 / 14,
+// 15 / 15. Low passes up to half of the band qualify, the direct form from a cutoff of about 0.2 on;
+// Chebyshev filters, high passes near zero and filters that do not decay within a tile do not.
+int resolve_auto(const std::vector<SectionF32>& secs, double gain, int& sweep_kind) {
+    const int K = static_cast<int>(secs.size());
+    sweep_kind = IIR_KIND_PH;
+    if (K < SWEEP_DIFF_MIN_SECTIONS) return IIR_KERNEL_PH;
+    if (tail_max_pieces() <= 0) return IIR_KERNEL_TC;  // the lookback schedules are asked for
+    const SweepFilter f = sweep_filter(secs.data(), K, gain);
+    const SweepKernel* k = sweep_kernels(SWEEP_KIND_PH_DIFF, K).front();
+    if (sweep_decay(f, k->span(), SWEEP_LANES) == 0) return IIR_KERNEL_TC;
+    constexpr double limit = 3e-7;
+    const std::vector<float> tables = sweep_tables(f, k->N, k->R);
+    if (sweep_error(f, tables, k->N, false) <= limit) return IIR_KERNEL_PH;
+    sweep_kind = SWEEP_KIND_PH_DIFF;
+    return sweep_error(f, tables, k->N, true) <= limit ? IIR_KERNEL_PH : IIR_KERNEL_TC;
 }
 
 // samples per block (= per lookback unit) of the plan's large-signal kernel, or of kernel e
@@ -759,7 +773,7 @@ int plan_add_sweeps(iir_plan* p, const std::vector<SectionF32>& secs, double gai
     if (tail_max_pieces() <= 0) return IIR_OK;  // the lookback everywhere
     if (p->n_sections == 1 && (!pipeline_enabled() || std::getenv("IIR_GB300_SMALL_N"))) return IIR_OK;
     const SweepFilter f = sweep_filter(secs.data(), p->n_sections, gain);
-    for (const SweepKernel* k : sweep_kernels(p->kind, p->n_sections)) {
+    for (const SweepKernel* k : sweep_kernels(p->sweep_kind, p->n_sections)) {
         SweepPart s;
         s.k = k;
         s.lanes = sweep_decay(f, k->span(), SWEEP_LANES);
@@ -784,7 +798,8 @@ int plan_add_sweeps(iir_plan* p, const std::vector<SectionF32>& secs, double gai
     q.state = p->d_state;
     q.gain = static_cast<float>(gain);
     for (int s = 0; s < p->n_sections; ++s)
-        q.sec[s] = SweepSection{secs[s].b1, secs[s].b2, secs[s].a1, secs[s].a2};
+        q.sec[s] = SweepSection{secs[s].b1, secs[s].b2, secs[s].a1, secs[s].a2,
+                                static_cast<float>(static_cast<double>(secs[s].a1) + secs[s].a2 - 1.0)};
     // the first section's input is the raw sample: its FIR taps carry the gain
     q.sec[0].b1 = static_cast<float>(gain * secs[0].b1);
     q.sec[0].b2 = static_cast<float>(gain * secs[0].b2);
@@ -841,12 +856,17 @@ int iir_plan_create(iir_plan** out, const float* sos, int n_sections, int kernel
     if (!out || !sos) return IIR_ERR_INVALID_ARGUMENT;
     *out = nullptr;
     if (n_sections < 1 || n_sections > IIR_MAX_SECTIONS) return IIR_ERR_INVALID_ARGUMENT;
-    kernel = resolve_auto(kernel, n_sections);
-    if (kernel < IIR_KERNEL_PH || kernel > IIR_KERNEL_TC) return IIR_ERR_INVALID_ARGUMENT;
+    if (kernel != IIR_KERNEL_AUTO && (kernel < IIR_KERNEL_PH || kernel > IIR_KERNEL_TC)) return IIR_ERR_INVALID_ARGUMENT;
     std::vector<SectionF32> secs;
     double gain = 1.0;
     int st = normalise_sos(sos, n_sections, secs, gain);
     if (st) return st;
+    int sweep_kind = kernel;
+    if (kernel == IIR_KERNEL_AUTO) {
+        kernel = resolve_auto(secs, gain, sweep_kind);
+        // (the precision form takes no geometry, so from 6 sections on AUTO takes none)
+        if (n_sections >= SWEEP_DIFF_MIN_SECTIONS) block_size = n_blocks = 0;
+    }
     if (kernel == IIR_KERNEL_PLR) {
         std::vector<double> bt, at;
         merge_sections(secs, bt, at);
@@ -963,6 +983,7 @@ int iir_plan_create(iir_plan** out, const float* sos, int n_sections, int kernel
     q.n_sections = n_sections;
     q.gain = static_cast<float>(gain);
     q.tail_pieces = pieces;
+    p->sweep_kind = sweep_kind;
     st = plan_add_sweeps(p, secs, gain);
     if (st) {
         plan_free(p);

@@ -16,7 +16,17 @@ __global__ void __launch_bounds__((W + 1) * 32) iir_ph_sweep_kernel(const __grid
     extern __shared__ __align__(1024) unsigned char smem[];
     using G = SweepGeom<K, N, R>;
     sweep_tiles<G, W, NB>(p, smem, [&](float* buf, int lane, auto& st, auto& xh) {
-        sweep_run_ph<G>(buf, p.sec, p.gain, lane, st, xh);
+        sweep_run_ph<G, false>(buf, p.sec, p.gain, lane, st, xh);
+    });
+}
+
+// The recurrence on differences: AUTO's, from 6 sections on, where the direct form rounds too much.
+template <int K, int N, int R, int W, int NB>
+__global__ void __launch_bounds__((W + 1) * 32) iir_ph_diff_sweep_kernel(const __grid_constant__ IirSweepParams p) {
+    extern __shared__ __align__(1024) unsigned char smem[];
+    using G = SweepGeom<K, N, R>;
+    sweep_tiles<G, W, NB>(p, smem, [&](float* buf, int lane, auto& st, auto& xh) {
+        sweep_run_ph<G, true>(buf, p.sec, p.gain, lane, st, xh);
     });
 }
 
@@ -50,6 +60,10 @@ template <int K, int N, int R, int W, int NB>
 void add(std::vector<SweepKernel>& v) {
     v.push_back(SweepKernel{IIR_KIND_PH, K, N, R, W, reinterpret_cast<const void*>(iir_ph_sweep_kernel<K, N, R, W, NB>),
                             sweep_smem<K, N, R>(NB, sizeof(SweepAux<NB, 2 * K>))});
+    if constexpr (K >= SWEEP_DIFF_MIN_SECTIONS)
+        v.push_back(SweepKernel{SWEEP_KIND_PH_DIFF, K, N, R, W,
+                                reinterpret_cast<const void*>(iir_ph_diff_sweep_kernel<K, N, R, W, NB>),
+                                sweep_smem<K, N, R>(NB, sizeof(SweepAux<NB, 2 * K>))});
     v.push_back(SweepKernel{IIR_KIND_STCR, K, N, R, W, reinterpret_cast<const void*>(iir_cr_sweep_kernel<K, N, R, W, NB>),
                             sweep_smem<K, N, R>(NB, sizeof(SweepAux<NB, 2 * K>)) + 10 * K * sizeof(f32x2)});
 }
@@ -245,10 +259,10 @@ int sweep_decay(const SweepFilter& f, int unit, int most) {
 
 std::vector<float> sweep_tables(const SweepFilter& f, int N, int R) {
     const int K = f.K, D = 2 * K, span = N * R;
-    const int blocks = K * (K + 1) / 2;
+    const int blocks = K * (K + 1) / 2, row = blocks | 1;
     const size_t t_h = static_cast<size_t>(D) * N, t_pn = (t_h + 2 * D + 3) & ~size_t(3),
                  t_pl = t_pn + 4 * static_cast<size_t>(blocks);
-    std::vector<float> t(t_pl + 4 * static_cast<size_t>(SWEEP_LANES) * blocks, 0.f);
+    std::vector<float> t(t_pl + 4 * static_cast<size_t>(SWEEP_LANES) * row, 0.f);
     put_dots(t, f, N, t_h);
     auto put = [&](size_t at, const Mat& m) {
         for (int s = 0; s < K; ++s)
@@ -258,10 +272,87 @@ std::vector<float> sweep_tables(const SweepFilter& f, int N, int R) {
     const Mat step = mat_pow(f.phi, span, D);
     Mat pl = mat_pow(f.phi, 0, D);
     for (int l = 0; l < SWEEP_LANES; ++l) {
-        put(t_pl + 4 * static_cast<size_t>(l) * blocks, pl);
+        put(t_pl + 4 * static_cast<size_t>(l) * row, pl);
         pl = mat_mul(pl, step, D);
     }
     return t;
+}
+
+double sweep_error(const SweepFilter& f, const std::vector<float>& t, int N, bool diff) {
+    const int K = f.K, D = 2 * K, rows = 40;
+    const float* th = t.data() + static_cast<size_t>(D) * N;
+    const float* pn = t.data() + ((static_cast<size_t>(D) * N + 2 * D + 3) & ~size_t(3));
+    std::vector<float> st(static_cast<size_t>(D), 0.f), e(st), next(st);
+    std::vector<float> h(static_cast<size_t>(2 * (K + 1)));   // pass B's histories: (n - 2, n - 1) of each stage
+    std::vector<double> r(static_cast<size_t>(2 * (K + 1)), 0.0);  // the same in 64 bits
+    std::vector<float> x(static_cast<size_t>(N)), dl(static_cast<size_t>(K));
+    const float g = static_cast<float>(f.gain);
+    float x2 = 0.f, x1 = 0.f;
+    double err = 0.0, ref = 0.0;
+    unsigned int lcg = 12345u;
+    for (int i = 0; i < rows; ++i) {
+        for (float& v : x) v = static_cast<float>(static_cast<int>((lcg = 1664525u * lcg + 1013904223u) >> 8)) * 0x1p-23f - 1.f;
+        for (int c = 0; c < D; ++c) {
+            float a[2] = {0.f, 0.f};
+            for (int n = 0; n < N; ++n) a[n & 1] = std::fmaf(t[static_cast<size_t>(c) * N + n], x[n], a[n & 1]);
+            e[c] = std::fmaf(th[2 * c + 1], x1, std::fmaf(th[2 * c], x2, a[0] + a[1]));
+        }
+        h[0] = x2;
+        h[1] = x1;
+        for (int s = 0; s < K; ++s) {
+            dl[s] = st[2 * s];
+            h[2 * s + 2] = st[2 * s + 1] - st[2 * s];
+            h[2 * s + 3] = st[2 * s + 1];
+        }
+        for (int n = 0; n < N; ++n) {
+            float in = x[n];
+            double rin = in;
+            for (int s = 0; s < K; ++s) {
+                const SectionF32& q = f.secs[s];
+                const float b1 = s == 0 ? static_cast<float>(f.gain * q.b1) : q.b1;
+                const float b2 = s == 0 ? static_cast<float>(f.gain * q.b2) : q.b2;
+                const float w = std::fmaf(b2, h[2 * s], std::fmaf(b1, h[2 * s + 1], s == 0 ? g * in : in));
+                float y;
+                if (diff) {
+                    const float k = static_cast<float>(static_cast<double>(q.a1) + q.a2 - 1.0);
+                    dl[s] = std::fmaf(k, h[2 * s + 3], std::fmaf(-q.a2, dl[s], w));
+                    y = h[2 * s + 3] + dl[s];
+                } else {
+                    y = std::fmaf(q.a1, h[2 * s + 3], std::fmaf(q.a2, h[2 * s + 2], w));
+                }
+                h[2 * s] = h[2 * s + 1];
+                h[2 * s + 1] = in;
+                in = y;
+                const double gs = s == 0 ? f.gain : 1.0;
+                const double rw = gs * (rin + q.b1 * r[2 * s + 1] + q.b2 * r[2 * s]);
+                const double ry = rw + q.a1 * r[2 * s + 3] + q.a2 * r[2 * s + 2];
+                r[2 * s] = r[2 * s + 1];
+                r[2 * s + 1] = rin;
+                rin = ry;
+            }
+            h[2 * K] = h[2 * K + 1];
+            h[2 * K + 1] = in;
+            r[2 * K] = r[2 * K + 1];
+            r[2 * K + 1] = rin;
+            err += (in - rin) * (in - rin);
+            ref += rin * rin;
+        }
+        for (int s = 0; s < K; ++s) {
+            float a0 = e[2 * s], a1 = e[2 * s + 1];
+            for (int q = 0; q <= s; ++q) {
+                const float* m = pn + 4 * (s * (s + 1) / 2 + q);
+                a0 = std::fmaf(m[2], st[2 * q + 1], std::fmaf(m[0], st[2 * q], a0));
+                a1 = std::fmaf(m[3], st[2 * q + 1], std::fmaf(m[1], st[2 * q], a1));
+            }
+            next[2 * s] = a0;
+            next[2 * s + 1] = a1;
+        }
+        st = next;
+        x2 = x[N - 2];
+        x1 = x[N - 1];
+    }
+    const double e2 = std::sqrt(err / ref);
+    return std::isfinite(e2) ? e2 : INFINITY;
 }
 
 BatchSweepFilter bsweep_filter(const SectionF32* secs, int K, double gain, int span) {

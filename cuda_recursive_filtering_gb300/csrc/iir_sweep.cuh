@@ -55,6 +55,11 @@ __device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
     return d;
 }
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+    f32x2 d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
 __device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
     f32x2 d;
     asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
@@ -79,8 +84,10 @@ struct SweepGeom {
     static constexpr int T_A = 0;                     // [D][N] pass A
     static constexpr int T_H = T_A + D * N;           // [D][2] response to (x[-2], x[-1])
     static constexpr int T_PN = (T_H + 2 * D + 3) & ~3;  // [BLOCKS] Phi^N, columns (m00, m10, m01, m11)
-    static constexpr int T_PL = T_PN + 4 * BLOCKS;       // [SWEEP_LANES][BLOCKS] Phi^(SPAN l)
-    static constexpr int T_LEN = T_PL + 4 * SWEEP_LANES * BLOCKS;
+    // a lane's power, in rows of an odd number of 16-byte units: lanes read their rows side by side
+    static constexpr int ROW = BLOCKS | 1;
+    static constexpr int T_PL = T_PN + 4 * BLOCKS;       // [SWEEP_LANES][ROW] Phi^(SPAN l)
+    static constexpr int T_LEN = T_PL + 4 * SWEEP_LANES * ROW;
     static_assert(T_LEN % 4 == 0 && T_PN % 4 == 0, "16-byte table rows");
 };
 
@@ -216,7 +223,7 @@ __device__ __forceinline__ void sweep_scan(const float* tab, int rounds, int lan
             o[c] = __shfl_up_sync(FULL_MASK, last[c], 1u << k);
             if (lane < (1 << k)) o[c] = 0.f;
         }
-        tri_mad<G::K>(tab + G::T_PL + 4 * (1 << k) * G::BLOCKS, o, last, last);
+        tri_mad<G::K>(tab + G::T_PL + 4 * (1 << k) * G::ROW, o, last, last);
     }
 #pragma unroll
     for (int c = 0; c < D; ++c) {
@@ -228,11 +235,27 @@ __device__ __forceinline__ void sweep_scan(const float* tab, int rounds, int lan
 // ------------------------------------------------------------------------------------
 // pass B, PH form: the cascade's own recurrences, sub-rows in packed pairs
 // ------------------------------------------------------------------------------------
+// Granules of 4 samples that go through the cascade together. More of them give longer diagonals (steps
+// that do not depend on one another) and more code; measured with 1 / 2 / 4: order 2 at 2^23 samples
+// 15.4 / 15.0 / 14.7 us, order 4 16.9 / 16.6 / 16.2; at 2^27 order 8 174.7 / 175.0 / 184.7, order 10
+// 237.5 / 234.3 / 230.6, order 12 259 / 267 / 273, order 16 330.7 / 329.8 / 330.7 (on differences 376 / 367
+// / 380).
+__host__ __device__ constexpr int sweep_step_granules(int K) { return K <= 2 || K == 5 ? 4 : K == 8 ? 2 : 1; }
+
 struct SweepSection {
     float b1, b2, a1, a2;  // section 0: b1, b2 carry the input gain (its input is the raw sample)
+    float k;               // a1 + a2 - 1, rounded once: the difference form's coefficient
 };
 
-template <class G>
+// DIFF: the recurrence on the outputs' differences,
+//     d[n] = w[n] + (a1 + a2 - 1) y[n-1] - a2 d[n-1],   y[n] = y[n-1] + d[n],
+// one addition more per sample and section. A rounding of y[n] in the direct form enters its recurrence at
+// full gain, 1 / A(z), which a low cutoff makes large; here the rounding of y[n] is the only one of y's own
+// size, and it meets (1 + a2 z^-1) / A(z), smaller by the cutoff's angle. Error against 64 bits (2-norm,
+// butter(16, .)): cutoff 0.05 3.0e-7 (direct form 1.11e-6, precision form 7.4e-7), 0.1 2.6e-7 (5.8e-7,
+// 6.5e-7), 0.4 3.0e-7 (2.3e-7, 5.3e-7). Time at 2^27 samples, cutoff 0.1, orders 12 / 16: 291 / 357 us
+// against 259 / 330 direct and 443 / 399 in the precision form.
+template <class G, bool DIFF>
 __device__ __forceinline__ void sweep_run_ph(float* buf, const SweepSection* sec, float gain, int lane,
                                              const float (&st)[G::R][G::D], const float (&xh)[G::R][2]) {
     constexpr int K = G::K, N = G::N, R = G::R, P = R / 2;
@@ -241,9 +264,14 @@ __device__ __forceinline__ void sweep_run_ph(float* buf, const SweepSection* sec
     for (int s = 0; s < K; ++s) {
         b1[s] = pack2(sec[s].b1, sec[s].b1);
         b2[s] = pack2(sec[s].b2, sec[s].b2);
-        a1[s] = pack2(sec[s].a1, sec[s].a1);
-        a2[s] = pack2(sec[s].a2, sec[s].a2);
+        a1[s] = DIFF ? pack2(sec[s].k, sec[s].k) : pack2(sec[s].a1, sec[s].a1);
+        a2[s] = DIFF ? pack2(-sec[s].a2, -sec[s].a2) : pack2(sec[s].a2, sec[s].a2);
     }
+    f32x2 dl[P][K];  // DIFF: the sections' last differences
+#pragma unroll
+    for (int p = 0; p < P; ++p)
+#pragma unroll
+        for (int s = 0; s < K; ++s) dl[p][s] = pack2(st[2 * p][2 * s], st[2 * p + 1][2 * s]);
     const f32x2 g = pack2(gain, gain);
     // h[p][0]: input history; h[p][s + 1]: section s's output history; [..][0] = n - 2, [..][1] = n - 1
     f32x2 h[P][K + 1][2];
@@ -262,16 +290,20 @@ __device__ __forceinline__ void sweep_run_ph(float* buf, const SweepSection* sec
         }
     float* row = buf + (lane << 5);
     const int l7 = lane & 7;
-#pragma unroll 2
-    for (int j = 0; j < N / 4; ++j) {
-        float* at = row + ((j >> 3) << 10) + (((j & 7) ^ l7) << 2);
-        float4 x[R];
+    constexpr int GB = sweep_step_granules(K), S = 4 * GB;  // granules and samples per step
+#pragma unroll (GB == 1 ? 2 : 1)
+    for (int j = 0; j < N / 4; j += GB) {
+        float4 x[GB][R];
+        float* at[GB];
 #pragma unroll
-        for (int i = 0; i < R; ++i) x[i] = *reinterpret_cast<const float4*>(at + i * (N / 32) * 1024);
-        // v[p][s][t]: section s's input (s = K: the output) at samples t - 2, t = 0..5. Four samples go
-        // through the sections along the diagonals (sample + section), whose steps do not depend on
-        // one another.
-        f32x2 v[P][K + 1][6];
+        for (int b = 0; b < GB; ++b) {
+            at[b] = row + ((j >> 3) << 10) + ((((j & 7) + b) ^ l7) << 2);
+#pragma unroll
+            for (int i = 0; i < R; ++i) x[b][i] = *reinterpret_cast<const float4*>(at[b] + i * (N / 32) * 1024);
+        }
+        // v[p][s][t]: section s's input (s = K: the output) at samples t - 2. The samples go through the
+        // sections along the diagonals (sample + section), whose steps do not depend on one another.
+        f32x2 v[P][K + 1][S + 2];
 #pragma unroll
         for (int p = 0; p < P; ++p) {
 #pragma unroll
@@ -279,22 +311,30 @@ __device__ __forceinline__ void sweep_run_ph(float* buf, const SweepSection* sec
                 v[p][s][0] = h[p][s][0];
                 v[p][s][1] = h[p][s][1];
             }
-            v[p][0][2] = pack2(x[2 * p].x, x[2 * p + 1].x);
-            v[p][0][3] = pack2(x[2 * p].y, x[2 * p + 1].y);
-            v[p][0][4] = pack2(x[2 * p].z, x[2 * p + 1].z);
-            v[p][0][5] = pack2(x[2 * p].w, x[2 * p + 1].w);
+#pragma unroll
+            for (int b = 0; b < GB; ++b) {
+                v[p][0][4 * b + 2] = pack2(x[b][2 * p].x, x[b][2 * p + 1].x);
+                v[p][0][4 * b + 3] = pack2(x[b][2 * p].y, x[b][2 * p + 1].y);
+                v[p][0][4 * b + 4] = pack2(x[b][2 * p].z, x[b][2 * p + 1].z);
+                v[p][0][4 * b + 5] = pack2(x[b][2 * p].w, x[b][2 * p + 1].w);
+            }
         }
 #pragma unroll
-        for (int d = 0; d < K + 3; ++d) {
+        for (int d = 0; d < K + S - 1; ++d) {
 #pragma unroll
             for (int s = 0; s < K; ++s) {
                 const int t = d - s + 2;
-                if (t < 2 || t > 5) continue;
+                if (t < 2 || t > S + 1) continue;
 #pragma unroll
                 for (int p = 0; p < P; ++p) {
                     const f32x2 in = s == 0 ? mul2(g, v[p][0][t]) : v[p][s][t];
                     const f32x2 w = fma2(b2[s], v[p][s][t - 2], fma2(b1[s], v[p][s][t - 1], in));
-                    v[p][s + 1][t] = fma2(a1[s], v[p][s + 1][t - 1], fma2(a2[s], v[p][s + 1][t - 2], w));
+                    if constexpr (DIFF) {
+                        dl[p][s] = fma2(a1[s], v[p][s + 1][t - 1], fma2(a2[s], dl[p][s], w));
+                        v[p][s + 1][t] = add2(v[p][s + 1][t - 1], dl[p][s]);
+                    } else {
+                        v[p][s + 1][t] = fma2(a1[s], v[p][s + 1][t - 1], fma2(a2[s], v[p][s + 1][t - 2], w));
+                    }
                 }
             }
         }
@@ -302,16 +342,21 @@ __device__ __forceinline__ void sweep_run_ph(float* buf, const SweepSection* sec
         for (int p = 0; p < P; ++p) {
 #pragma unroll
             for (int s = 0; s <= K; ++s) {
-                h[p][s][0] = v[p][s][4];
-                h[p][s][1] = v[p][s][5];
+                h[p][s][0] = v[p][s][S];
+                h[p][s][1] = v[p][s][S + 1];
             }
-            unpack2(v[p][K][2], x[2 * p].x, x[2 * p + 1].x);
-            unpack2(v[p][K][3], x[2 * p].y, x[2 * p + 1].y);
-            unpack2(v[p][K][4], x[2 * p].z, x[2 * p + 1].z);
-            unpack2(v[p][K][5], x[2 * p].w, x[2 * p + 1].w);
+#pragma unroll
+            for (int b = 0; b < GB; ++b) {
+                unpack2(v[p][K][4 * b + 2], x[b][2 * p].x, x[b][2 * p + 1].x);
+                unpack2(v[p][K][4 * b + 3], x[b][2 * p].y, x[b][2 * p + 1].y);
+                unpack2(v[p][K][4 * b + 4], x[b][2 * p].z, x[b][2 * p + 1].z);
+                unpack2(v[p][K][4 * b + 5], x[b][2 * p].w, x[b][2 * p + 1].w);
+            }
         }
 #pragma unroll
-        for (int i = 0; i < R; ++i) *reinterpret_cast<float4*>(at + i * (N / 32) * 1024) = x[i];
+        for (int b = 0; b < GB; ++b)
+#pragma unroll
+            for (int i = 0; i < R; ++i) *reinterpret_cast<float4*>(at[b] + i * (N / 32) * 1024) = x[b][i];
     }
 }
 
@@ -529,7 +574,7 @@ __device__ __forceinline__ void sweep_tiles(const IirSweepParams& p, unsigned ch
     }
     // (of Phi^(SPAN l), the powers that the lanes and the scan steps use)
     const int reach = p.lanes > (1 << p.rounds) / 2 + 1 ? p.lanes : (1 << p.rounds) / 2 + 1;
-    for (int i = threadIdx.x; i < G::T_PL / 4 + reach * G::BLOCKS; i += (W + 1) * 32)
+    for (int i = threadIdx.x; i < G::T_PL / 4 + reach * G::ROW; i += (W + 1) * 32)
         reinterpret_cast<float4*>(tab)[i] = __ldg(reinterpret_cast<const float4*>(p.tables) + i);
     __syncthreads();
     // every wait is bounded; the first to run out sends the whole block home
@@ -655,7 +700,7 @@ __device__ __forceinline__ void sweep_tiles(const IirSweepParams& p, unsigned ch
                         X[c] = v.x;
                         X[c + 1] = v.y;
                     }
-                    tri_mad<K>(tab + G::T_PL + 4 * lane * G::BLOCKS, X, st[0], st[0]);
+                    tri_mad<K>(tab + G::T_PL + 4 * lane * G::ROW, X, st[0], st[0]);
                 }
             }
             if (!warm) {

@@ -9,6 +9,11 @@
 
 namespace iirhost {
 
+// Kernels of the recurrence on differences (compiled from this many sections on), beside the
+// realizations' own kinds.
+constexpr int SWEEP_KIND_PH_DIFF = 100;
+constexpr int SWEEP_DIFF_MIN_SECTIONS = 6;
+
 // A compiled sweep kernel: realization, sections, sub-rows of N samples, R per lane, warps per block.
 struct SweepKernel {
     int kind, K, N, R, warps;
@@ -35,5 +40,8 @@ SweepFilter sweep_filter(const SectionF32* secs, int K, double gain);
 int sweep_decay(const SweepFilter& f, int unit, int most);
 // The tables of one kernel geometry (SweepGeom's layout).
 std::vector<float> sweep_tables(const SweepFilter& f, int N, int R);
+// Relative error (2-norm, against 64 bits) of the schedule's float32 arithmetic on white noise, with pass B
+// in the direct form or on differences: the kernel's steps done on the host over 40 sub-rows, with its tables.
+double sweep_error(const SweepFilter& f, const std::vector<float>& tables, int N, bool diff);
 
 }  // namespace iirhost
