@@ -679,14 +679,71 @@ void matmul_k(const std::vector<double>& A, const std::vector<double>& B, std::v
     C.swap(R);
 }
 
+// Adds the plan's state-sweep kernels: those whose tiles cover the filter's decay.
+int plan_add_sweeps(iir_plan* p, const std::vector<SectionF32>& secs, double gain) {
+    if (tail_max_pieces() <= 0) return IIR_OK;  // the lookback everywhere
+    if (p->n_sections == 1 && (!pipeline_enabled() || std::getenv("IIR_GB300_SMALL_N"))) return IIR_OK;
+    const SweepFilter f = sweep_filter(secs.data(), p->n_sections, gain);
+    for (const SweepKernel* k : sweep_kernels(p->sweep_kind, p->n_sections)) {
+        SweepPart s;
+        s.k = k;
+        s.lanes = sweep_decay(f, k->span(), SWEEP_LANES);
+        if (s.lanes == 0) continue;
+        const std::vector<float> tab = sweep_tables(f, k->N, k->R);
+        int st = cuda_status(
+            cudaFuncSetAttribute(k->fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(k->smem)));
+        if (!st) st = cuda_status(cudaFuncSetAttribute(k->fn, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
+        int nb = 0;
+        if (!st) st = cuda_status(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k->fn, 32 * (k->warps + 1), k->smem));
+        if (!st && nb <= 0) st = IIR_ERR_UNSUPPORTED;
+        if (!st) st = cuda_status(cudaMalloc(&s.d_tab, tab.size() * sizeof(float)));
+        if (!st) st = cuda_status(cudaMemcpy(s.d_tab, tab.data(), tab.size() * sizeof(float), cudaMemcpyHostToDevice));
+        if (st) {
+            if (s.d_tab) cudaFree(s.d_tab);
+            return st;
+        }
+        s.resident = nb * p->sms;
+        p->sweeps.push_back(s);
+    }
+    IirSweepParams& q = p->sweep;
+    q.state = p->d_state;
+    q.gain = static_cast<float>(gain);
+    for (int s = 0; s < p->n_sections; ++s)
+        q.sec[s] = SweepSection{secs[s].b1, secs[s].b2, secs[s].a1, secs[s].a2,
+                                static_cast<float>(static_cast<double>(secs[s].a1) + secs[s].a2 - 1.0)};
+    // the first section's input is the raw sample: its FIR taps carry the gain
+    q.sec[0].b1 = static_cast<float>(gain * secs[0].b1);
+    q.sec[0].b2 = static_cast<float>(gain * secs[0].b2);
+    for (int s = 0; s < p->n_sections; ++s) {
+        const SweepSection& c = q.sec[s];
+        const double e = -static_cast<double>(c.a1), f = -static_cast<double>(c.a2);
+        const double e1 = 2.0 * f - e * e, f1 = f * f, e2 = 2.0 * f1 - e1 * e1;
+        q.cr[s] = SweepCr{c.b1, c.b2, c.a1, c.a2, static_cast<float>(f), static_cast<float>(-e1),
+                          static_cast<float>(-f1 / e1), static_cast<float>(f1 / e1 - e1), static_cast<float>(-e2), 0.f};
+    }
+    return IIR_OK;
+}
+
+// Largest signal that PLR filters with a block per chunk where it has a warp per chunk: the warps of a block
+// crowd a small signal onto few SMs (order 4, graph replays, block / warp: 2^16 samples 5.4 / 11.0 us, 2^20
+// 14.2 / 15.2, 3e6 33.0 / 16.1).
+constexpr size_t PLR_BLOCK_MAX_N = size_t(1) << 20;
+
 int plan_create_plr(iir_plan** out, const double* b, const double* a, int order, double gain, int B, int X,
                     size_t max_n) {
     if (order != 2 && order != 4 && order != 8 && order != 16) return IIR_ERR_UNSUPPORTED;
     int Bd = B, Xd = X;
     default_geometry(IIR_KIND_PLR, order / 2, Bd, Xd);
-    const KernelEntry* e = find_entry(IIR_KIND_PLR, Bd, Xd, order);
-    if (!e) return IIR_ERR_UNSUPPORTED;
+    // a block per chunk, and for large signals (where it is compiled) a warp per chunk
+    const KernelEntry* block = find_entry(IIR_KIND_PLR, Bd, Xd, order);
+    if (!block) return IIR_ERR_UNSUPPORTED;
+    const KernelEntry* warp = find_entry(IIR_KIND_PLR, Bd, Xd, order, 1);
+    const KernelEntry* e = warp ? warp : block;
     iir_plan* p = new iir_plan();
+    if (warp) {
+        p->small = block;
+        p->small_max_n = PLR_BLOCK_MAX_N;
+    }
     p->kind = IIR_KIND_PLR;
     p->B = Bd;
     p->N = Xd;
@@ -764,52 +821,17 @@ int plan_create_plr(iir_plan** out, const double* b, const double* a, int order,
         q.b[j] = static_cast<float>(b[j]);
         q.a[j] = static_cast<float>(a[j]);
     }
-    *out = p;
-    return IIR_OK;
-}
-
-// Adds the plan's state-sweep kernels: those whose tiles cover the filter's decay.
-int plan_add_sweeps(iir_plan* p, const std::vector<SectionF32>& secs, double gain) {
-    if (tail_max_pieces() <= 0) return IIR_OK;  // the lookback everywhere
-    if (p->n_sections == 1 && (!pipeline_enabled() || std::getenv("IIR_GB300_SMALL_N"))) return IIR_OK;
-    const SweepFilter f = sweep_filter(secs.data(), p->n_sections, gain);
-    for (const SweepKernel* k : sweep_kernels(p->sweep_kind, p->n_sections)) {
-        SweepPart s;
-        s.k = k;
-        s.lanes = sweep_decay(f, k->span(), SWEEP_LANES);
-        if (s.lanes == 0) continue;
-        const std::vector<float> tab = sweep_tables(f, k->N, k->R);
-        int st = cuda_status(
-            cudaFuncSetAttribute(k->fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(k->smem)));
-        if (!st) st = cuda_status(cudaFuncSetAttribute(k->fn, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
-        int nb = 0;
-        if (!st) st = cuda_status(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k->fn, 32 * (k->warps + 1), k->smem));
-        if (!st && nb <= 0) st = IIR_ERR_UNSUPPORTED;
-        if (!st) st = cuda_status(cudaMalloc(&s.d_tab, tab.size() * sizeof(float)));
-        if (!st) st = cuda_status(cudaMemcpy(s.d_tab, tab.data(), tab.size() * sizeof(float), cudaMemcpyHostToDevice));
+    if (order == 2) {
+        // one section: the direct form is PH's (2^25 samples: 193 us with a block per chunk, 44 on the sweep;
+        // errors against 64 bits 1.7e-7 and 1.2e-7 at a cutoff of 0.1)
+        p->sweep_kind = IIR_KIND_PH;
+        st = plan_add_sweeps(p, {SectionF32{q.b[0], q.b[1], q.a[0], q.a[1]}}, gain);
         if (st) {
-            if (s.d_tab) cudaFree(s.d_tab);
+            plan_free(p);
             return st;
         }
-        s.resident = nb * p->sms;
-        p->sweeps.push_back(s);
     }
-    IirSweepParams& q = p->sweep;
-    q.state = p->d_state;
-    q.gain = static_cast<float>(gain);
-    for (int s = 0; s < p->n_sections; ++s)
-        q.sec[s] = SweepSection{secs[s].b1, secs[s].b2, secs[s].a1, secs[s].a2,
-                                static_cast<float>(static_cast<double>(secs[s].a1) + secs[s].a2 - 1.0)};
-    // the first section's input is the raw sample: its FIR taps carry the gain
-    q.sec[0].b1 = static_cast<float>(gain * secs[0].b1);
-    q.sec[0].b2 = static_cast<float>(gain * secs[0].b2);
-    for (int s = 0; s < p->n_sections; ++s) {
-        const SweepSection& c = q.sec[s];
-        const double e = -static_cast<double>(c.a1), f = -static_cast<double>(c.a2);
-        const double e1 = 2.0 * f - e * e, f1 = f * f, e2 = 2.0 * f1 - e1 * e1;
-        q.cr[s] = SweepCr{c.b1, c.b2, c.a1, c.a2, static_cast<float>(f), static_cast<float>(-e1),
-                          static_cast<float>(-f1 / e1), static_cast<float>(f1 / e1 - e1), static_cast<float>(-e2), 0.f};
-    }
+    *out = p;
     return IIR_OK;
 }
 
@@ -1018,6 +1040,8 @@ constexpr size_t SWEEP_LARGE_PER_SM = 16384;
 
 // The sweep kernel for a signal of n samples, or null for a single section's small signal.
 const SweepPart* sweep_pick(const iir_plan* p, size_t n) {
+    // PLR's order 2 has no such kernel (2^20 samples: 8.9 us, 8.7 on the sweep; 3e6: 22.5, 9.2)
+    if (p->kind == IIR_KIND_PLR) return n > PLR_BLOCK_MAX_N ? &p->sweeps.front() : nullptr;
     if (n >= SWEEP_LARGE_PER_SM * static_cast<size_t>(p->sms)) return &p->sweeps.front();
     return p->n_sections > 1 ? &p->sweeps.back() : nullptr;
 }
@@ -1090,9 +1114,10 @@ int plan_launch(iir_plan* p, const float* x, float* y, size_t n, const float* zi
         const int st = alloc_carry(p, nchunks, stream);
         if (st) return st;
     }
-    // one block per chunk (blocks take tickets in start order; no residency assumption)
+    // one block per chunk (blocks take tickets in start order; no residency assumption), or resident
+    // blocks whose warps draw the chunks
     if (nchunks > 0x7fffffffull) return IIR_ERR_TOO_LARGE;
-    const int grid = static_cast<int>(nchunks);
+    const int grid = static_cast<int>(p->kind == IIR_KIND_PLR && ent->pipeline ? std::min<size_t>(nchunks, static_cast<size_t>(p->grid_max)) : nchunks);
     // Flags are 32-bit functions of the launch epoch: re-zero the slots and the launch state
     // long before the epoch could wrap (the reference zeroes its status buffer once).
     if (++p->launches >= (1ull << 30)) {
@@ -1114,7 +1139,7 @@ int plan_launch(iir_plan* p, const float* x, float* y, size_t n, const float* zi
         q.timeout_ns = p->timeout_ns;
         q.withhold_chunk = p->withhold;
         void* args[] = {&q};
-        err = cudaLaunchKernel(p->entry->fn, dim3(grid), dim3(p->entry->threads), args, p->entry->smem, stream);
+        err = cudaLaunchKernel(ent->fn, dim3(grid), dim3(ent->threads), args, ent->smem, stream);
     } else {
         IirParams& q = p->params;
         q.x = x;

@@ -27,7 +27,8 @@ struct KernelEntry {
     size_t smem;    // dynamic shared memory bytes
     int order;      // PLR direct-form order (0 for the cascaded realizations)
     int rows;       // rows per block (tiles x B) for the row-major realizations
-    int pipeline = 0;  // 1: single-section persistent pipeline, launched cooperatively
+    int pipeline = 0;  // 1: single-section persistent pipeline, launched cooperatively (PLR: resident blocks
+                       // whose warps draw the chunks)
     int planes = 1;    // chunk buffer layout: 1 = planes of 32-sample columns, 0 = lines (swz)
     int tail = 0;      // 1: cascade kernel on the tail-aggregate schedule (iir_tail.cuh)
     int tiny = 0;      // 1: a 32-row tail kernel that single-section plans use for short signals
