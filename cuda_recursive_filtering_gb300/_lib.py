@@ -60,7 +60,7 @@ def load(path: str | None = None):
     pp = ctypes.POINTER(ctypes.c_void_p)
     sigs = {
         "iir_sos_filter": ([vp, vp, sz, fp, i, i, vp], i),
-        "iir_sos_filter_geom": ([vp, vp, sz, fp, i, i, i, i, vp], i),
+        "iir_sos_filter_geom": ([vp, vp, sz, vp, i, i, i, i, vp], i),  # sos: an address (or a pointer object)
         "iir_sos_filter_noalloc": ([vp, vp, sz, fp, i, vp], i),
         "iir_plan_create": ([pp, fp, i, i, i, i, sz], i),
         "iir_plan_create_plr_ba": ([pp, dp, dp, i, ctypes.c_double, i, i, sz], i),
@@ -77,7 +77,7 @@ def load(path: str | None = None):
         "iir_cache_clear": ([], i),
         "iir_sos_filter_debug_withhold": ([ll, ll], i),
         "iir_batch_create": ([pp, fp, ip, i, sz, sz], i),
-        "iir_batch_execute": ([vp, ctypes.POINTER(IirSegment), i, vp], i),
+        "iir_batch_execute": ([vp, vp, i, vp], i),  # the segment table, likewise
         "iir_batch_check": ([vp, vp], i),
         "iir_batch_set_timeout_ns": ([vp, ll], i),
         "iir_batch_debug_withhold": ([vp, ll], i),

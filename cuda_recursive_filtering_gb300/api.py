@@ -31,22 +31,33 @@ def _kernel_id(kernel) -> int:
 
 
 def _sos_array(sos) -> np.ndarray:
+    if type(sos) is np.ndarray and sos.dtype == np.float32 and sos.ndim == 2 and sos.shape[1] == 6 \
+            and sos.shape[0] >= 1 and sos.flags.c_contiguous:
+        return sos
     s = np.ascontiguousarray(np.asarray(sos, dtype=np.float32).reshape(-1, 6))
     if s.shape[0] < 1:
         raise ValueError("sos needs at least one section")
     return s
 
 
-def _stream_handle(stream) -> ctypes.c_void_p:
+# The current stream's handle without a Stream object around it.
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
+# Small calls are bound by the host (GB300's Grace cores: 2^16 samples of a kept plan are 5 us of GPU time),
+# so device addresses and handles go to the C functions as plain integers.
+def _stream_handle(stream) -> int:
     if stream is None:
+        if _raw_stream is not None:
+            return _raw_stream(torch.cuda.current_device())
         stream = torch.cuda.current_stream()
-    return ctypes.c_void_p(int(stream.cuda_stream))
+    return int(stream.cuda_stream)
 
 
 def _check_tensor(x: torch.Tensor, name: str) -> None:
     if not isinstance(x, torch.Tensor) or not x.is_cuda:
         raise TypeError(f"{name} must be a CUDA tensor")
-    if x.dtype != torch.float32:
+    if x.dtype is not torch.float32:
         raise TypeError(f"{name} must be float32")
     if not x.is_contiguous():
         raise ValueError(f"{name} must be contiguous")
@@ -98,9 +109,9 @@ class Plan:
         _check_tensor(out, "out")
         if out.numel() != x.numel():
             raise ValueError("out must have as many samples as x")
-        st = self._lib.iir_plan_execute(self._ptr, ctypes.c_void_p(x.data_ptr()), ctypes.c_void_p(out.data_ptr()),
-                                        x.numel(), _stream_handle(stream))
-        check(st, "iir_plan_execute")
+        st = self._lib.iir_plan_execute(self._ptr, x.data_ptr(), out.data_ptr(), x.numel(), _stream_handle(stream))
+        if st:
+            check(st, "iir_plan_execute")
         return out
 
     def filter_host(self, x: torch.Tensor, out: torch.Tensor | None = None, piece: int = 0,
@@ -184,10 +195,10 @@ def sosfilt(sos, x: torch.Tensor, kernel="AUTO", block_size: int = 0, n_blocks: 
     if out is None:
         out = torch.empty_like(x)
     _check_tensor(out, "out")
-    st = lib.iir_sos_filter_geom(ctypes.c_void_p(x.data_ptr()), ctypes.c_void_p(out.data_ptr()), x.numel(),
-                                 s.ctypes.data_as(ctypes.POINTER(ctypes.c_float)), s.shape[0], _kernel_id(kernel),
-                                 int(block_size), int(n_blocks), _stream_handle(stream))
-    check(st, "iir_sos_filter")
+    st = lib.iir_sos_filter_geom(x.data_ptr(), out.data_ptr(), x.numel(), s.ctypes.data, s.shape[0],
+                                 _kernel_id(kernel), int(block_size), int(n_blocks), _stream_handle(stream))
+    if st:
+        check(st, "iir_sos_filter")
     return out
 
 
@@ -287,8 +298,7 @@ class Batch:
         device addresses / counts, as iir_segment)."""
         if tab.dtype != self._SEG_DTYPE or tab.size < n:
             raise ValueError("segment table of the wrong layout or size")
-        st = self._lib.iir_batch_execute(self._ptr, tab.ctypes.data_as(ctypes.POINTER(_lib.IirSegment)), int(n),
-                                         _stream_handle(stream))
+        st = self._lib.iir_batch_execute(self._ptr, tab.ctypes.data, int(n), _stream_handle(stream))
         check(st, "iir_batch_execute")
 
     def bind(self, x: torch.Tensor, y: torch.Tensor, offsets, filters, zi=None, zf=None) -> "BoundBatch":
