@@ -199,6 +199,64 @@ __device__ __forceinline__ void bsweep_run(float* buf, const float* tab, int lan
         }
     }
 }
+// The sections' states after sample m of the tile, to zf[2 s], zf[2 s + 1], s < kreal, ahead of pass B: its
+// steps once more from the start of m's sub-row, by every lane alike (bound by their latency: at most N
+// samples, about a microsecond per segment). bsweep_run's CAPTURE takes a second copy of pass B in the
+// kernel; 1024 segments of 33600 samples, order 8, with states: 99 us with it, 89 with this. The kernel of
+// up to 8 sections captures all the same: there these steps cost every tile registers (order 16, mixed
+// lengths: 506 us against 476).
+template <class G>
+__device__ __forceinline__ void bsweep_state(const float* buf, const float* tab, int lane, int m,
+                                             const float (&st)[G::R][G::D], const float (&xh)[G::R][2], float* zf,
+                                             int kreal) {
+    constexpr int K = G::K, N = G::N, R = G::R, D = G::D;
+    const int row = m / G::SPAN, sub = (m % G::SPAN) / N;
+    float S[D], h2 = 0.f, h1 = 0.f, y2[K], y1[K];
+#pragma unroll
+    for (int c = 0; c < D; ++c) S[c] = 0.f;
+#pragma unroll
+    for (int i = 0; i < R; ++i)
+        if (i == sub) {
+            h2 = xh[i][0];
+            h1 = xh[i][1];
+#pragma unroll
+            for (int c = 0; c < D; ++c) S[c] = st[i][c];
+        }
+    h2 = __shfl_sync(FULL_MASK, h2, row);
+    h1 = __shfl_sync(FULL_MASK, h1, row);
+#pragma unroll
+    for (int s = 0; s < K; ++s) {
+        const float d = __shfl_sync(FULL_MASK, S[2 * s], row), u = __shfl_sync(FULL_MASK, S[2 * s + 1], row);
+        y2[s] = u - d;
+        y1[s] = u;
+    }
+    const float gain = tab[G::T_C + 4 * K];
+#pragma unroll 1
+    for (int n = sub * N; n <= m % G::SPAN; ++n) {
+        const float xv = buf[tile_at(row, n)];
+        float w = gain * xv, g2 = h2, g1 = h1;
+        h2 = h1;
+        h1 = xv;
+#pragma unroll
+        for (int s = 0; s < K; ++s) {
+            const float4 c = *reinterpret_cast<const float4*>(tab + G::T_C + 4 * s);
+            w = fmaf(c.y, g2, fmaf(c.x, g1, w));
+            g2 = y2[s];
+            g1 = y1[s];
+            w = fmaf(c.z, g1, fmaf(c.w, g2, w));
+            y2[s] = g1;
+            y1[s] = w;
+        }
+    }
+#pragma unroll
+    for (int s = 0; s < K; ++s)
+        if (lane == 0 && s < kreal) {
+            zf[2 * s] = y2[s];
+            zf[2 * s + 1] = y1[s];
+        }
+    __syncwarp();  // every lane has read the samples
+}
+
 __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, int x, int y, int z,
                                             unsigned long long* bar) {
     asm volatile(
@@ -379,8 +437,9 @@ __device__ __forceinline__ void bsweep_copier(const IirBatchSweepParams& p, Batc
 }
 
 // One item: the tile in `buf`, whose load has been issued. wait_tile(): it is there; wait_ready(): the item
-// before has its end state. Returns false when a wait ran out.
-template <class G, int NB, class Tile, class Ready>
+// before has its end state. Returns false when a wait ran out. CAPTURE: how the segment's states are found
+// (bsweep_state).
+template <class G, int NB, bool CAPTURE, class Tile, class Ready>
 __device__ __forceinline__ bool bsweep_item(const IirBatchSweepParams& p, BatchSweepAux<NB>& aux, float* buf,
                                             const float* tab, const BatchRun& run, unsigned i, unsigned rec,
                                             Tile&& wait_tile, Ready&& wait_ready) {
@@ -505,9 +564,18 @@ __device__ __forceinline__ bool bsweep_item(const IirBatchSweepParams& p, BatchS
 #pragma unroll
     for (int j = 1; j < R; ++j) tri_mad<K>(tab + G::T_PN, st[j - 1], e[j - 1], st[j]);
     __syncwarp();  // every lane has read its neighbour's last samples
-    if (run.zf && left <= TILE) {
-        const int m = have - 1;  // the segment's last sample
-        bsweep_run<G, true>(buf, tab, lane, st, xh, m >= 0 && m / SPAN == lane ? m % SPAN : -1, run.zf + 2, run.K);
+    const int m = have - 1;  // the segment's last sample, if it is here
+    const bool ends = run.zf && left <= TILE;
+    if constexpr (CAPTURE) {
+        if (ends)
+            bsweep_run<G, true>(buf, tab, lane, st, xh, m >= 0 && m / SPAN == lane ? m % SPAN : -1, run.zf + 2, run.K);
+        else
+            bsweep_run<G, false>(buf, tab, lane, st, xh);
+    } else {
+        if (ends && m >= 0) bsweep_state<G>(buf, tab, lane, m, st, xh, run.zf + 2, run.K);
+        bsweep_run<G, false>(buf, tab, lane, st, xh);
+    }
+    if (ends) {
         __syncwarp();
         if (lane == 0) {
             const long long end = run.n;  // raw input history
@@ -517,8 +585,6 @@ __device__ __forceinline__ bool bsweep_item(const IirBatchSweepParams& p, BatchS
             if (m >= 0) run.zf[2 * run.K + 1] = buf[tile_at(m / SPAN, m % SPAN)];
             if (m >= 1) run.zf[2 * run.K] = buf[tile_at((m - 1) / SPAN, (m - 1) % SPAN)];
         }
-    } else {
-        bsweep_run<G, false>(buf, tab, lane, st, xh);
     }
     fence_proxy_async_smem();  // generic accesses of the buffer before the async ones to come
     __syncwarp();
@@ -611,7 +677,7 @@ __global__ void __launch_bounds__((W + 1 + BSWEEP_COPIERS) * 32) iir_batch_sweep
             switch (run.K) {
 #define IIR_BSWEEP_CASE(KP)                                                                                  \
     if constexpr (KP <= MAXK)                                                                                 \
-        ok = bsweep_item<BatchSweepGeom<KP, SPAN>, NB>(p, aux, buf, tab, run, i, rec, tile, ready);           \
+        ok = bsweep_item<BatchSweepGeom<KP, SPAN>, NB, (MAXK > 4)>(p, aux, buf, tab, run, i, rec, tile, ready);  \
     break;
                 case 1: IIR_BSWEEP_CASE(1)
                 case 2: IIR_BSWEEP_CASE(2)
