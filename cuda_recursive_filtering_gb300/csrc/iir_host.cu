@@ -517,8 +517,9 @@ int resolve_auto(const std::vector<SectionF32>& secs, double gain, int& sweep_ki
     sweep_kind = IIR_KIND_PH;
     if (K < SWEEP_DIFF_MIN_SECTIONS) return IIR_KERNEL_PH;
     if (tail_max_pieces() <= 0) return IIR_KERNEL_TC;  // the lookback schedules are asked for
-    const SweepFilter f = sweep_filter(secs.data(), K, gain);
     const SweepKernel* k = sweep_kernels(SWEEP_KIND_PH_DIFF, K).front();
+    if (sweep_too_slow(secs.data(), K, SWEEP_LANES * k->span())) return IIR_KERNEL_TC;
+    const SweepFilter f = sweep_filter(secs.data(), K, gain);
     if (sweep_decay(f, k->span(), SWEEP_LANES) == 0) return IIR_KERNEL_TC;
     constexpr double limit = 3e-7;
     const std::vector<float> tables = sweep_tables(f, k->N, k->R);
@@ -683,8 +684,10 @@ void matmul_k(const std::vector<double>& A, const std::vector<double>& B, std::v
 int plan_add_sweeps(iir_plan* p, const std::vector<SectionF32>& secs, double gain) {
     if (tail_max_pieces() <= 0) return IIR_OK;  // the lookback everywhere
     if (p->n_sections == 1 && (!pipeline_enabled() || std::getenv("IIR_GB300_SMALL_N"))) return IIR_OK;
+    const std::vector<const SweepKernel*> kernels = sweep_kernels(p->sweep_kind, p->n_sections);
+    if (sweep_too_slow(secs.data(), p->n_sections, SWEEP_LANES * kernels.front()->span())) return IIR_OK;
     const SweepFilter f = sweep_filter(secs.data(), p->n_sections, gain);
-    for (const SweepKernel* k : sweep_kernels(p->sweep_kind, p->n_sections)) {
+    for (const SweepKernel* k : kernels) {
         SweepPart s;
         s.k = k;
         s.lanes = sweep_decay(f, k->span(), SWEEP_LANES);

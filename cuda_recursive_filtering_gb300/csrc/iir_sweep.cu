@@ -236,6 +236,15 @@ SweepFilter sweep_filter(const SectionF32* secs, int K, double gain) {
     return f;
 }
 
+bool sweep_too_slow(const SectionF32* secs, int K, int samples) {
+    double r = 0.0;
+    for (int s = 0; s < K; ++s) {
+        const double a1 = secs[s].a1, a2 = secs[s].a2, disc = a1 * a1 + 4.0 * a2;
+        r = std::max(r, disc < 0.0 ? std::sqrt(-a2) : 0.5 * (std::fabs(a1) + std::sqrt(disc)));
+    }
+    return !(samples * std::log(r) <= std::log(1.0000001e-10));
+}
+
 int sweep_decay(const SweepFilter& f, int unit, int most) {
     const int D = 2 * f.K;
     for (double s : f.scale)
@@ -356,6 +365,8 @@ double sweep_error(const SweepFilter& f, const std::vector<float>& t, int N, boo
 }
 
 BatchSweepFilter bsweep_filter(const SectionF32* secs, int K, double gain, int span) {
+    BatchSweepFilter out;
+    if (sweep_too_slow(secs, K, 32 * span)) return out;
     // the compiled number of sections: those past the filter's own pass their input on
     const int KP = bsweep_sections(K);
     std::vector<SectionF32> padded(secs, secs + K);
@@ -393,7 +404,6 @@ BatchSweepFilter bsweep_filter(const SectionF32* secs, int K, double gain, int s
         }
         return true;
     };
-    BatchSweepFilter out;
     const int ls = log2i(span);
     int k = 0;
     while (k <= 5 && !decayed(power(ls + k))) ++k;

@@ -35,6 +35,9 @@ struct SweepFilter {
     std::vector<double> scale;  // each section's output for white noise (the states' own scale)
 };
 SweepFilter sweep_filter(const SectionF32* secs, int K, double gain);
+// Whether a pole alone takes longer than `samples` to fall to 1e-10 (no norm of the transition is below it):
+// then the filter does not decay within them, and its tables need not be worked out.
+bool sweep_too_slow(const SectionF32* secs, int K, int samples);
 // Steps of `unit` samples after which older state is below 1e-10 of the states' own scale, 0 if more
 // than `most` are needed.
 int sweep_decay(const SweepFilter& f, int unit, int most);
