@@ -721,7 +721,7 @@ int plan_add_sweeps(iir_plan* p, const std::vector<SectionF32>& secs, double gai
         const SweepSection& c = q.sec[s];
         const double e = -static_cast<double>(c.a1), f = -static_cast<double>(c.a2);
         const double e1 = 2.0 * f - e * e, f1 = f * f, e2 = 2.0 * f1 - e1 * e1;
-        q.cr[s] = SweepCr{c.b1, c.b2, c.a1, c.k, static_cast<float>(f), static_cast<float>(-e1),
+        q.cr[s] = SweepCr{c.b1, c.b2, c.a1, c.a2, static_cast<float>(f), static_cast<float>(-e1),
                           static_cast<float>(-f1 / e1), static_cast<float>(f1 / e1 - e1), static_cast<float>(-e2), 0.f};
     }
     return IIR_OK;

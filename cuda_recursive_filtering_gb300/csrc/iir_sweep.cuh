@@ -9,7 +9,7 @@
 //   scan    the sub-rows' states are joined inside the lane with Phi^N (Phi is the cascade's state
 //           transition, block lower triangular), then across the lanes with powers of Phi^SPAN;
 //   pass B  every sub-row runs the whole cascade once from its true state, all K sections in
-//           registers (4K multiply-adds per sample; 7.3K as cyclic reduction), and its output
+//           registers (4K multiply-adds per sample; 5.25K as cyclic reduction), and its output
 //           replaces the input.
 // One pass per section (iir_ph.cuh: zero-state filter, scan, correction folded into the next pass)
 // takes 7K operations per sample and a read and a write of shared memory per section; this takes
@@ -363,34 +363,32 @@ __device__ __forceinline__ void sweep_run_ph(float* buf, const SweepSection* sec
 // ------------------------------------------------------------------------------------
 // pass B, cyclic reduction: sub-rows in packed pairs, blocks of 8 samples
 // ------------------------------------------------------------------------------------
-// One section of the cyclic reduction (iir_cr.cuh) on a block of 8 samples whose incoming pair is known. It
-// solves for u[n] = y[n] - Y1, the outputs less the one before the block: its right-hand sides get the
-// constant (a1 + a2 - 1) Y1, and the first one -a2 (Y1 - Y2), so the block starts from rest and rounds by the
-// size of what changes within 8 samples. The double-sided round (1 - e z^-1 + f z^-2) splits it into halves of
-// 4, two levels reduce each half to its last sample, and the dropped samples follow by back-substitution (from
-// rest most terms vanish):
-//   w'[n] = w[n] + k Y1 (n = 0: + f (Y1 - Y2));   v[n] = w'[n] + a1 w'[n-1] + f w'[n-2]
-//   half (v0..v3):  u0 = v0,  u1 = v1 - e1 v0,  s2 = v2 - r1 v1,  s3 = v3 - e1 s2,
-//                   u3 = s3 - e2 u1,  u2 = s2 - c1 u1        (r1 = f1/e1, c1 = e1 - r1)
-// 7.3 operations per sample. Folding the pair in whole (y itself for u) takes 5.3, and its rounding enters
-// the recurrence at full gain: error against 64 bits 3.2e-7 / 1.47e-6 at orders 2 / 16, cutoff 0.05, where this
-// has 1.5e-7 / 3.8e-7 and the row solvers of iir_cr.cuh 9.4e-8 / 3.9e-7.
+// One section of the cyclic reduction (iir_cr.cuh) on a block of 8 samples whose incoming pair is known.
+// The pair is folded into the block's first two right-hand sides, so the block starts from rest; the
+// double-sided round (1 - e z^-1 + f z^-2) splits it into halves of 4, two levels reduce each half to its
+// last sample, and the dropped samples follow by back-substitution (from rest most terms vanish):
+//   w'[0] = w[0] + a1 Y1 + a2 Y2, w'[1] = w[1] + a2 Y1;   v[n] = w'[n] + a1 w'[n-1] + f w'[n-2]
+//   half (v0..v3):  y0 = v0,  y1 = v1 - e1 v0,  u2 = v2 - r1 v1,  u3 = v3 - e1 u2,
+//                   y3 = u3 - e2 y1,  y2 = u2 - c1 y1        (r1 = f1/e1, c1 = e1 - r1)
+// 5.25 multiply-adds per sample, of which 5 in a row depend on one another per 8 samples (the plain
+// recurrence has 4, and 8 in a row). Blocks of 16 take 6.1, of 4 take 4.5 with 6 in a row per 4 samples.
+// Error against 64 bits as the plain recurrence's (order 2, cutoff 0.1: 1.2e-7 of the output's RMS).
 //
 // Bound by memory at one section, by issue above. Measured on GB300, butter(order, 0.1), CUDA graph
-// replays, against those row solvers, which filters that decay more slowly keep (us):
+// replays, against the row solvers of iir_cr.cuh, which filters that decay more slowly keep (us):
 //   order            2              4              8               16
-//   STCR  3e6   10.1 ->  9.6   12.4 -> 11.6   18.2 -> 14.9    31.7 ->  23.5
-//   STCR  2^25  55.9 -> 43.9   82.0 -> 48.4  128.6 -> 69.2   240.6 -> 124.9
-//   STCR  2^27 189.1 ->157.9  292.6 ->163.8  473.2 ->242.4   909.3 -> 460.6
-//   DTCR  2^25  57.0 -> 43.9  107.6 -> 48.4  187.1 -> 69.2   367.4 -> 124.9
-//   DTCR  2^27 200.1 ->157.9  403.1 ->163.8  719.8 ->242.4  1428   -> 460.6
+//   STCR  3e6   10.1 ->  9.4   12.4 -> 11.2   18.2 -> 14.1    31.7 ->  21.8
+//   STCR  2^25  55.9 -> 44.0   82.0 -> 47.1  128.6 -> 63.0   240.6 -> 117.2
+//   STCR  2^27 189.1 ->157.8  292.6 ->160.9  473.2 ->216.9   909.3 -> 428.0
+//   DTCR  2^25  57.0 -> 44.0  107.6 -> 47.1  187.1 -> 63.0   367.4 -> 117.2
+//   DTCR  2^27 200.1 ->157.8  403.1 ->160.9  719.8 ->219.0  1428   -> 428.1
 struct SweepCr {
-    float b1, b2, a1, k, f, ne1, nr1, nc1, ne2, pad;  // k = a1 + a2 - 1, f = -a2; "n": negated; section 0: b1, b2 carry the gain
+    float b1, b2, a1, a2, f, ne1, nr1, nc1, ne2, pad;  // "n": negated; section 0: b1, b2 carry the gain
 };
 static_assert(sizeof(SweepCr) == 40, "five 16-byte loads of packed pairs");
 
 struct SweepCrPairs {
-    f32x2 b1, b2, a1, k, f, ne1, nr1, nc1, ne2;
+    f32x2 b1, b2, a1, a2, f, ne1, nr1, nc1, ne2;
 };
 // The coefficients as pairs, from a table of pairs (SweepCr's order).
 __device__ __forceinline__ SweepCrPairs cr_pairs(const f32x2* t) {
@@ -424,12 +422,6 @@ __device__ __forceinline__ void sweep_run_cr(float* buf, const f32x2* pairs, flo
                 h[p][s + 1][t] = t == 0 ? pack2(u[1] - u[0], v[1] - v[0]) : pack2(u[1], v[1]);
             }
         }
-    f32x2 dl[P][K];  // the sections' last differences
-#pragma unroll
-    for (int p = 0; p < P; ++p)
-#pragma unroll
-        for (int s = 0; s < K; ++s) dl[p][s] = pack2(st[2 * p][2 * s], st[2 * p + 1][2 * s]);
-    const f32x2 minus = pack2(-1.f, -1.f);
     float* row = buf + (lane << 5);
     const int l7 = lane & 7;
 #pragma unroll 1
@@ -459,16 +451,17 @@ __device__ __forceinline__ void sweep_run_cr(float* buf, const f32x2* pairs, flo
 #pragma unroll
             for (int p = 0; p < P; ++p) {
                 f32x2* v = z[p];
-                const f32x2 Y1 = h[p][s + 1][1], c0 = mul2(c.k, Y1);
+                const f32x2 Y2 = h[p][s + 1][0], Y1 = h[p][s + 1][1];
                 f32x2 w[8];
 #pragma unroll
                 for (int t = 0; t < 8; ++t) {
                     const f32x2 x1 = t >= 1 ? v[t - 1] : h[p][s][1], x2 = t >= 2 ? v[t - 2] : h[p][s][t];
-                    w[t] = fma2(c.b2, x2, fma2(c.b1, x1, s == 0 ? fma2(g, v[t], c0) : add2(v[t], c0)));
+                    w[t] = fma2(c.b2, x2, fma2(c.b1, x1, s == 0 ? mul2(g, v[t]) : v[t]));
                 }
                 h[p][s][0] = v[6];
                 h[p][s][1] = v[7];
-                w[0] = fma2(c.f, dl[p][s], w[0]);
+                w[0] = fma2(c.a1, Y1, fma2(c.a2, Y2, w[0]));
+                w[1] = fma2(c.a2, Y1, w[1]);
                 v[0] = w[0];
                 v[1] = fma2(c.a1, w[0], w[1]);
 #pragma unroll
@@ -481,9 +474,6 @@ __device__ __forceinline__ void sweep_run_cr(float* buf, const f32x2* pairs, flo
                     v[6 + e] = fma2(c.ne2, v[2 + e], u3);
                     v[4 + e] = fma2(c.nc1, v[2 + e], u2);
                 }
-                dl[p][s] = fma2(minus, v[6], v[7]);
-#pragma unroll
-                for (int t = 0; t < 8; ++t) v[t] = add2(Y1, v[t]);
             }
         }
 #pragma unroll
