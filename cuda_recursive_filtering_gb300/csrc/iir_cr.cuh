@@ -33,10 +33,6 @@
 // level loop dispatches each iteration to that level's body, whose indices are compile-time
 // constants. Both execute the same operations in the same order, so they are bit-identical.
 //
-// Filters that decay within a tile are run by the state sweep instead (iir_sweep.cuh, sweep_run_cr: the
-// same reduction on blocks of 8 samples); these solvers take the others, single sections up to a few
-// million samples, and launches that start from a carried state.
-//
 // With TAIL (iir_tail.cuh) the cascade kernel resolves every section's incoming state once per
 // chunk from the predecessor's tail aggregate, before the first section's join; the row warps
 // then join tiles with one barrier among themselves per section instead of two around a lookback.

@@ -685,6 +685,7 @@ int plan_add_sweeps(iir_plan* p, const std::vector<SectionF32>& secs, double gai
     if (tail_max_pieces() <= 0) return IIR_OK;  // the lookback everywhere
     if (p->n_sections == 1 && (!pipeline_enabled() || std::getenv("IIR_GB300_SMALL_N"))) return IIR_OK;
     const std::vector<const SweepKernel*> kernels = sweep_kernels(p->sweep_kind, p->n_sections);
+    if (kernels.empty()) return IIR_OK;  // another realization
     if (sweep_too_slow(secs.data(), p->n_sections, SWEEP_LANES * kernels.front()->span())) return IIR_OK;
     const SweepFilter f = sweep_filter(secs.data(), p->n_sections, gain);
     for (const SweepKernel* k : kernels) {
@@ -717,13 +718,6 @@ int plan_add_sweeps(iir_plan* p, const std::vector<SectionF32>& secs, double gai
     // the first section's input is the raw sample: its FIR taps carry the gain
     q.sec[0].b1 = static_cast<float>(gain * secs[0].b1);
     q.sec[0].b2 = static_cast<float>(gain * secs[0].b2);
-    for (int s = 0; s < p->n_sections; ++s) {
-        const SweepSection& c = q.sec[s];
-        const double e = -static_cast<double>(c.a1), f = -static_cast<double>(c.a2);
-        const double e1 = 2.0 * f - e * e, f1 = f * f, e2 = 2.0 * f1 - e1 * e1;
-        q.cr[s] = SweepCr{c.b1, c.b2, c.a1, c.a2, static_cast<float>(f), static_cast<float>(-e1),
-                          static_cast<float>(-f1 / e1), static_cast<float>(f1 / e1 - e1), static_cast<float>(-e2), 0.f};
-    }
     return IIR_OK;
 }
 

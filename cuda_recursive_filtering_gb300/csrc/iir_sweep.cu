@@ -1,4 +1,4 @@
-// iir_sweep.cu — PH and CR kernels on the state-sweep schedule (iir_sweep.cuh) and the host's side of
+// iir_sweep.cu — PH kernels on the state-sweep schedule (iir_sweep.cuh) and the host's side of
 // that schedule: the tables of a filter, computed in FP64 from its float32 sections.
 #include "iir_sweep.cuh"
 
@@ -30,24 +30,6 @@ __global__ void __launch_bounds__((W + 1) * 32) iir_ph_diff_sweep_kernel(const _
     });
 }
 
-// STCR and DTCR, both forms: whether a row's parity halves belong to one thread or two, and whether the
-// levels are looped over, is a matter of the row solvers in iir_cr.cuh. Here a lane holds both halves of
-// its sub-rows and a block's two levels are one body, so the four kinds are one kernel.
-template <int K, int N, int R, int W, int NB>
-__global__ void __launch_bounds__((W + 1) * 32) iir_cr_sweep_kernel(const __grid_constant__ IirSweepParams p) {
-    extern __shared__ __align__(1024) unsigned char smem[];
-    using G = SweepGeom<K, N, R>;
-    // the sections' coefficients as pairs (sweep_tiles' first barrier comes before their first use)
-    f32x2* pairs = reinterpret_cast<f32x2*>(smem + sweep_smem<K, N, R>(NB, sizeof(SweepAux<NB, 2 * K>)));
-    for (int i = threadIdx.x; i < 10 * K; i += (W + 1) * 32) {
-        const float c = reinterpret_cast<const float*>(p.cr)[i];
-        pairs[i] = pack2(c, c);
-    }
-    sweep_tiles<G, W, NB>(p, smem, [&](float* buf, int lane, auto& st, auto& xh) {
-        sweep_run_cr<G>(buf, pairs, p.gain, lane, st, xh);
-    });
-}
-
 }  // namespace iirgb
 
 using namespace iirgb;
@@ -64,8 +46,6 @@ void add(std::vector<SweepKernel>& v) {
         v.push_back(SweepKernel{SWEEP_KIND_PH_DIFF, K, N, R, W,
                                 reinterpret_cast<const void*>(iir_ph_diff_sweep_kernel<K, N, R, W, NB>),
                                 sweep_smem<K, N, R>(NB, sizeof(SweepAux<NB, 2 * K>))});
-    v.push_back(SweepKernel{IIR_KIND_STCR, K, N, R, W, reinterpret_cast<const void*>(iir_cr_sweep_kernel<K, N, R, W, NB>),
-                            sweep_smem<K, N, R>(NB, sizeof(SweepAux<NB, 2 * K>)) + 10 * K * sizeof(f32x2)});
 }
 
 template <int K>
@@ -186,7 +166,6 @@ void put_dots(std::vector<float>& t, const SweepFilter& f, int N, size_t t_h) {
 }  // namespace
 
 std::vector<const SweepKernel*> sweep_kernels(int kind, int K) {
-    if (kind == IIR_KIND_STCR_UNROLL || kind == IIR_KIND_DTCR || kind == IIR_KIND_DTCR_UNROLL) kind = IIR_KIND_STCR;
     std::vector<const SweepKernel*> r;
     for (const SweepKernel& k : kernels())
         if (k.kind == kind && k.K == K) r.push_back(&k);

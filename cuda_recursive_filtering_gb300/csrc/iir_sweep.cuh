@@ -9,8 +9,7 @@
 //   scan    the sub-rows' states are joined inside the lane with Phi^N (Phi is the cascade's state
 //           transition, block lower triangular), then across the lanes with powers of Phi^SPAN;
 //   pass B  every sub-row runs the whole cascade once from its true state, all K sections in
-//           registers (4K multiply-adds per sample; 5.25K as cyclic reduction), and its output
-//           replaces the input.
+//           registers (4K multiply-adds per sample), and its output replaces the input.
 // One pass per section (iir_ph.cuh: zero-state filter, scan, correction folded into the next pass)
 // takes 7K operations per sample and a read and a write of shared memory per section; this takes
 // 6K, two reads and one write.
@@ -361,143 +360,6 @@ __device__ __forceinline__ void sweep_run_ph(float* buf, const SweepSection* sec
 }
 
 // ------------------------------------------------------------------------------------
-// pass B, cyclic reduction: sub-rows in packed pairs, blocks of 8 samples
-// ------------------------------------------------------------------------------------
-// One section of the cyclic reduction (iir_cr.cuh) on a block of 8 samples whose incoming pair is known.
-// The pair is folded into the block's first two right-hand sides, so the block starts from rest; the
-// double-sided round (1 - e z^-1 + f z^-2) splits it into halves of 4, two levels reduce each half to its
-// last sample, and the dropped samples follow by back-substitution (from rest most terms vanish):
-//   w'[0] = w[0] + a1 Y1 + a2 Y2, w'[1] = w[1] + a2 Y1;   v[n] = w'[n] + a1 w'[n-1] + f w'[n-2]
-//   half (v0..v3):  y0 = v0,  y1 = v1 - e1 v0,  u2 = v2 - r1 v1,  u3 = v3 - e1 u2,
-//                   y3 = u3 - e2 y1,  y2 = u2 - c1 y1        (r1 = f1/e1, c1 = e1 - r1)
-// 5.25 multiply-adds per sample, of which 5 in a row depend on one another per 8 samples (the plain
-// recurrence has 4, and 8 in a row). Blocks of 16 take 6.1, of 4 take 4.5 with 6 in a row per 4 samples.
-// Error against 64 bits as the plain recurrence's (order 2, cutoff 0.1: 1.2e-7 of the output's RMS).
-//
-// Bound by memory at one section, by issue above. Measured on GB300, butter(order, 0.1), CUDA graph
-// replays, against the row solvers of iir_cr.cuh, which filters that decay more slowly keep (us):
-//   order            2              4              8               16
-//   STCR  3e6   10.1 ->  9.4   12.4 -> 11.2   18.2 -> 14.1    31.7 ->  21.8
-//   STCR  2^25  55.9 -> 44.0   82.0 -> 47.1  128.6 -> 63.0   240.6 -> 117.2
-//   STCR  2^27 189.1 ->157.8  292.6 ->160.9  473.2 ->216.9   909.3 -> 428.0
-//   DTCR  2^25  57.0 -> 44.0  107.6 -> 47.1  187.1 -> 63.0   367.4 -> 117.2
-//   DTCR  2^27 200.1 ->157.8  403.1 ->160.9  719.8 ->219.0  1428   -> 428.1
-struct SweepCr {
-    float b1, b2, a1, a2, f, ne1, nr1, nc1, ne2, pad;  // "n": negated; section 0: b1, b2 carry the gain
-};
-static_assert(sizeof(SweepCr) == 40, "five 16-byte loads of packed pairs");
-
-struct SweepCrPairs {
-    f32x2 b1, b2, a1, a2, f, ne1, nr1, nc1, ne2;
-};
-// The coefficients as pairs, from a table of pairs (SweepCr's order).
-__device__ __forceinline__ SweepCrPairs cr_pairs(const f32x2* t) {
-    const ulonglong2* q = reinterpret_cast<const ulonglong2*>(t);
-    const ulonglong2 c0 = q[0], c1 = q[1], c2 = q[2], c3 = q[3];
-    return SweepCrPairs{c0.x, c0.y, c1.x, c1.y, c2.x, c2.y, c3.x, c3.y, t[8]};
-}
-
-template <class G>
-__device__ __forceinline__ void sweep_run_cr(float* buf, const f32x2* pairs, float gain, int lane,
-                                             const float (&st)[G::R][G::D], const float (&xh)[G::R][2]) {
-    constexpr int K = G::K, N = G::N, R = G::R, P = R / 2;
-    constexpr bool HELD = K <= 2;  // coefficients in registers; else from shared memory for every block
-    SweepCrPairs held[HELD ? K : 1];
-    if constexpr (HELD)
-#pragma unroll
-        for (int s = 0; s < K; ++s) held[s] = cr_pairs(pairs + 10 * s);
-    const f32x2 g = pack2(gain, gain);
-    // h[p][0]: input history; h[p][s + 1]: section s's output history; [..][0] = n - 2, [..][1] = n - 1
-    f32x2 h[P][K + 1][2];
-#pragma unroll
-    for (int p = 0; p < P; ++p)
-#pragma unroll
-        for (int t = 0; t < 2; ++t) {
-            h[p][0][t] = pack2(xh[2 * p][t], xh[2 * p + 1][t]);
-#pragma unroll
-            for (int s = 0; s < K; ++s) {
-                // state pairs are (y[-1] - y[-2], y[-1])
-                const float* u = st[2 * p] + 2 * s;
-                const float* v = st[2 * p + 1] + 2 * s;
-                h[p][s + 1][t] = t == 0 ? pack2(u[1] - u[0], v[1] - v[0]) : pack2(u[1], v[1]);
-            }
-        }
-    float* row = buf + (lane << 5);
-    const int l7 = lane & 7;
-#pragma unroll 1
-    for (int j = 0; j < N / 4; j += 2) {
-        float* at0 = row + ((j >> 3) << 10) + (((j & 7) ^ l7) << 2);
-        float* at1 = row + ((j >> 3) << 10) + ((((j & 7) + 1) ^ l7) << 2);
-        f32x2 z[P][8];
-#pragma unroll
-        for (int p = 0; p < P; ++p) {
-            const float4 a = *reinterpret_cast<const float4*>(at0 + 2 * p * (N / 32) * 1024);
-            const float4 b = *reinterpret_cast<const float4*>(at0 + (2 * p + 1) * (N / 32) * 1024);
-            const float4 c = *reinterpret_cast<const float4*>(at1 + 2 * p * (N / 32) * 1024);
-            const float4 d = *reinterpret_cast<const float4*>(at1 + (2 * p + 1) * (N / 32) * 1024);
-            z[p][0] = pack2(a.x, b.x);
-            z[p][1] = pack2(a.y, b.y);
-            z[p][2] = pack2(a.z, b.z);
-            z[p][3] = pack2(a.w, b.w);
-            z[p][4] = pack2(c.x, d.x);
-            z[p][5] = pack2(c.y, d.y);
-            z[p][6] = pack2(c.z, d.z);
-            z[p][7] = pack2(c.w, d.w);
-        }
-#pragma unroll
-        for (int s = 0; s < K; ++s) {
-            if constexpr (K > 4) asm volatile("" ::: "memory");  // one section's coefficients at a time: no spills
-            const SweepCrPairs c = HELD ? held[HELD ? s : 0] : cr_pairs(pairs + 10 * s);
-#pragma unroll
-            for (int p = 0; p < P; ++p) {
-                f32x2* v = z[p];
-                const f32x2 Y2 = h[p][s + 1][0], Y1 = h[p][s + 1][1];
-                f32x2 w[8];
-#pragma unroll
-                for (int t = 0; t < 8; ++t) {
-                    const f32x2 x1 = t >= 1 ? v[t - 1] : h[p][s][1], x2 = t >= 2 ? v[t - 2] : h[p][s][t];
-                    w[t] = fma2(c.b2, x2, fma2(c.b1, x1, s == 0 ? mul2(g, v[t]) : v[t]));
-                }
-                h[p][s][0] = v[6];
-                h[p][s][1] = v[7];
-                w[0] = fma2(c.a1, Y1, fma2(c.a2, Y2, w[0]));
-                w[1] = fma2(c.a2, Y1, w[1]);
-                v[0] = w[0];
-                v[1] = fma2(c.a1, w[0], w[1]);
-#pragma unroll
-                for (int t = 2; t < 8; ++t) v[t] = fma2(c.a1, w[t - 1], fma2(c.f, w[t - 2], w[t]));
-#pragma unroll
-                for (int e = 0; e < 2; ++e) {  // the halves: samples 0 2 4 6 and 1 3 5 7
-                    const f32x2 u2 = fma2(c.nr1, v[2 + e], v[4 + e]);
-                    v[2 + e] = fma2(c.ne1, v[e], v[2 + e]);
-                    const f32x2 u3 = fma2(c.ne1, u2, v[6 + e]);
-                    v[6 + e] = fma2(c.ne2, v[2 + e], u3);
-                    v[4 + e] = fma2(c.nc1, v[2 + e], u2);
-                }
-            }
-        }
-#pragma unroll
-        for (int p = 0; p < P; ++p) {
-            h[p][K][0] = z[p][6];
-            h[p][K][1] = z[p][7];
-            float4 a, b, c, d;
-            unpack2(z[p][0], a.x, b.x);
-            unpack2(z[p][1], a.y, b.y);
-            unpack2(z[p][2], a.z, b.z);
-            unpack2(z[p][3], a.w, b.w);
-            unpack2(z[p][4], c.x, d.x);
-            unpack2(z[p][5], c.y, d.y);
-            unpack2(z[p][6], c.z, d.z);
-            unpack2(z[p][7], c.w, d.w);
-            *reinterpret_cast<float4*>(at0 + 2 * p * (N / 32) * 1024) = a;
-            *reinterpret_cast<float4*>(at0 + (2 * p + 1) * (N / 32) * 1024) = b;
-            *reinterpret_cast<float4*>(at1 + 2 * p * (N / 32) * 1024) = c;
-            *reinterpret_cast<float4*>(at1 + (2 * p + 1) * (N / 32) * 1024) = d;
-        }
-    }
-}
-
-// ------------------------------------------------------------------------------------
 // launch parameters and the tile loop
 // ------------------------------------------------------------------------------------
 struct IirSweepParams {
@@ -515,7 +377,6 @@ struct IirSweepParams {
     int use_tma;              // tensor maps valid (x, y 16-byte aligned, at least one row)
     float gain;
     SweepSection sec[IIR_MAX_SECTIONS];
-    SweepCr cr[IIR_MAX_SECTIONS];
 };
 
 constexpr unsigned SWEEP_RING = 64;  // item records and end states kept of the last items

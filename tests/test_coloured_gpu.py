@@ -1,0 +1,61 @@
+"""Signals that a filter takes nearly all away from: a tone in the stop band 40 dB over the noise, and an
+offset or a slow tone through a high pass. What is left is small beside what a section's state is made of,
+so a schedule that forms the states of later sections from the raw samples loses digits that filtering
+section by section keeps.
+
+Tolerance: the reference's gate max|err| <= 1e-4 * max|ref| (src/test_accuracy.cu:178-188), and no more than
+twice the error of the per-section lookback schedule (IIR_GB300_TAIL=0, read when a plan is created) plus
+one float32 rounding of the peak, 2^-24 * max|ref|.
+"""
+import numpy as np
+import pytest
+import torch
+from scipy import signal
+
+import oracle
+from cuda_recursive_filtering_gb300 import Plan
+
+pytestmark = pytest.mark.gpu
+
+LARGE = 152 * 16384  # samples from which PH's large-signal sweep kernel runs
+CASES = [("cheby1", 10, 0.1, "low", "stop"), ("cheby1", 12, 0.5, "low", "stop"), ("butter", 8, 0.05, "low", "stop"),
+         ("butter", 8, 0.8, "high", "slow"), ("butter", 4, 0.8, "high", "offset")]
+
+
+def design(kind, order, cutoff, btype):
+    return signal.butter(order, cutoff, btype, output="sos") if kind == "butter" else \
+        signal.cheby1(order, 1.0, cutoff, btype, output="sos")
+
+
+def coloured(n, what, seed=3):
+    t = np.arange(n)
+    x = np.random.default_rng(seed).uniform(-1, 1, n)
+    x += {"stop": 100 * np.sin(0.97 * np.pi * t), "slow": 100 * np.sin(0.0011 * np.pi * t), "offset": 1000.0}[what]
+    return x.astype(np.float32)
+
+
+def error(plan, xt, ref):
+    y = plan(xt)
+    plan.check()
+    assert bool(torch.isfinite(y).all())
+    return np.max(np.abs(y.cpu().numpy().astype(np.float64) - ref))
+
+
+def check(case, kernel, n, monkeypatch):
+    sos = design(*case[:4])
+    x = coloured(n, case[4])
+    xt = torch.from_numpy(x).cuda()
+    _, ref = oracle.reference_golden(sos, x)
+    peak = np.max(np.abs(ref))
+    got = error(Plan(sos, kernel, max_n=n), xt, ref)
+    monkeypatch.setenv("IIR_GB300_TAIL", "0")
+    lookback = error(Plan(sos, kernel, max_n=n), xt, ref)
+    assert got <= 1e-4 * peak, (got / peak, lookback / peak)
+    assert got <= 2 * lookback + 2.0 ** -24 * peak, (got / peak, lookback / peak)
+
+
+@pytest.mark.parametrize("n", (100_003, LARGE + 5000))
+@pytest.mark.parametrize("kernel", ("STCR", "STCR_UNROLL", "DTCR", "DTCR_UNROLL"))
+@pytest.mark.parametrize("case", CASES, ids=lambda c: "-".join(map(str, c)))
+def test_cyclic_reduction(case, kernel, n, monkeypatch, cuda_device):
+    check(case, kernel, n, monkeypatch)
