@@ -15,8 +15,8 @@ template <int K, int N, int R, int W, int NB>
 __global__ void __launch_bounds__((W + 1) * 32) iir_ph_sweep_kernel(const __grid_constant__ IirSweepParams p) {
     extern __shared__ __align__(1024) unsigned char smem[];
     using G = SweepGeom<K, N, R>;
-    sweep_tiles<G, W, NB>(p, smem, [&](float* buf, int lane, auto& st, auto& xh) {
-        sweep_run_ph<G, false>(buf, p.sec, p.gain, lane, st, xh);
+    sweep_tiles<G, W, NB>(p, smem, [&](float* buf, int lane, auto& st, auto& xh, auto& end) {
+        sweep_run_ph<G, false>(buf, p.sec, p.gain, lane, st, xh, end);
     });
 }
 
@@ -25,8 +25,8 @@ template <int K, int N, int R, int W, int NB>
 __global__ void __launch_bounds__((W + 1) * 32) iir_ph_diff_sweep_kernel(const __grid_constant__ IirSweepParams p) {
     extern __shared__ __align__(1024) unsigned char smem[];
     using G = SweepGeom<K, N, R>;
-    sweep_tiles<G, W, NB>(p, smem, [&](float* buf, int lane, auto& st, auto& xh) {
-        sweep_run_ph<G, true>(buf, p.sec, p.gain, lane, st, xh);
+    sweep_tiles<G, W, NB>(p, smem, [&](float* buf, int lane, auto& st, auto& xh, auto& end) {
+        sweep_run_ph<G, true>(buf, p.sec, p.gain, lane, st, xh, end);
     });
 }
 
@@ -264,6 +264,16 @@ std::vector<float> sweep_tables(const SweepFilter& f, int N, int R) {
         pl = mat_mul(pl, step, D);
     }
     return t;
+}
+
+SweepLimits sweep_limits(const SectionF32& s) {
+    const double a1 = s.a1, a2 = s.a2;
+    // power gain of 1 / (1 - a1 z^-1 - a2 z^-2): white noise that enters the recurrence comes out by it
+    const double noise = (1.0 - a2) / ((1.0 + a2) * ((1.0 - a2) * (1.0 - a2) - a1 * a1));
+    // an error of the difference grows to about 1 / (the pole's angle) of the output, its square k's size
+    const double angle = std::sqrt(std::fabs(a1 + a2 - 1.0));
+    return SweepLimits{static_cast<float>(angle < 1.0 ? 1.0 / std::max(angle, 1e-6) : 1.0),
+                       static_cast<float>(4.0 * 0x1p-24 * (1.0 + (noise > 0.0 ? std::sqrt(noise) : 0.0)))};
 }
 
 double sweep_error(const SweepFilter& f, const std::vector<float>& t, int N, bool diff) {

@@ -9,7 +9,8 @@
 //   scan    the sub-rows' states are joined inside the lane with Phi^N (Phi is the cascade's state
 //           transition, block lower triangular), then across the lanes with powers of Phi^SPAN;
 //   pass B  every sub-row runs the whole cascade once from its true state, all K sections in
-//           registers (4K multiply-adds per sample), and its output replaces the input.
+//           registers (4K multiply-adds per sample), and its output replaces the input. Its own end
+//           states check the ones that the next sub-rows started from (sweep_agree).
 // One pass per section (iir_ph.cuh: zero-state filter, scan, correction folded into the next pass)
 // takes 7K operations per sample and a read and a write of shared memory per section; this takes
 // 6K, two reads and one write.
@@ -244,6 +245,7 @@ __host__ __device__ constexpr int sweep_step_granules(int K) { return K <= 2 || 
 struct SweepSection {
     float b1, b2, a1, a2;  // section 0: b1, b2 carry the input gain (its input is the raw sample)
     float k;               // a1 + a2 - 1, rounded once: the difference form's coefficient
+    float wd, tol;         // sweep_agree: weight of a difference's residual, and the largest ratio to the output
 };
 
 // DIFF: the recurrence on the outputs' differences,
@@ -256,7 +258,8 @@ struct SweepSection {
 // against 259 / 330 direct and 443 / 399 in the precision form.
 template <class G, bool DIFF>
 __device__ __forceinline__ void sweep_run_ph(float* buf, const SweepSection* sec, float gain, int lane,
-                                             const float (&st)[G::R][G::D], const float (&xh)[G::R][2]) {
+                                             const float (&st)[G::R][G::D], const float (&xh)[G::R][2],
+                                             float (&end)[G::R][G::D]) {
     constexpr int K = G::K, N = G::N, R = G::R, P = R / 2;
     f32x2 b1[K], b2[K], a1[K], a2[K];
 #pragma unroll
@@ -357,6 +360,118 @@ __device__ __forceinline__ void sweep_run_ph(float* buf, const SweepSection* sec
 #pragma unroll
             for (int i = 0; i < R; ++i) *reinterpret_cast<float4*>(at[b] + i * (N / 32) * 1024) = x[b][i];
     }
+#pragma unroll
+    for (int p = 0; p < P; ++p)
+#pragma unroll
+        for (int s = 0; s < K; ++s) {
+            float ya, yb;
+            unpack2(h[p][s + 1][1], ya, yb);
+            end[2 * p][2 * s + 1] = ya;
+            end[2 * p + 1][2 * s + 1] = yb;
+            if constexpr (DIFF) {
+                unpack2(dl[p][s], end[2 * p][2 * s], end[2 * p + 1][2 * s]);
+            } else {
+                float za, zb;
+                unpack2(h[p][s + 1][0], za, zb);
+                end[2 * p][2 * s] = ya - za;
+                end[2 * p + 1][2 * s] = yb - zb;
+            }
+        }
+}
+
+// ------------------------------------------------------------------------------------
+// the states checked and corrected
+// ------------------------------------------------------------------------------------
+// Pass A forms a later section's state from the raw samples. Where the cascade takes nearly all of the signal
+// away (a tone in the stop band, an offset through a high pass), that sum cancels: its rounding is of the
+// samples' size, the state is not. Pass B runs the sections one after another and does not have this, so the
+// state that it leaves behind a sub-row tells how far the next one's start was off:
+//     r[j+1] = (pass B's end of sub-row j) - (start of sub-row j+1),   error of a start = -g,
+//     g[j+1] = Phi^N g[j] + r[j+1].
+// Where r stands out of the recurrence's own rounding, g is found by the same join and scan as the states, and
+// the response to g is added to the outputs (4K operations per sample). Elsewhere the check is all there is: about
+// 4% of a tile's instructions. Error against 64 bits, cheby1(16, 1, 0.3), noise and a tone 40 dB above it in
+// the stop band: 2.0e-3 without, 2.7e-5 with (section by section, iir_ph.cuh: 3.1e-5).
+
+// Residuals r of the lane's sub-rows (r[i]: at its end), from pass B's end states, the states st that it started
+// from and the tile's end state `last`. True if all are within a section's rounding: tol = 4 x 2^-24 x (1 + the
+// noise gain of 1 / A) of its largest output in the tile, a difference weighed by what it grows to. (With 12
+// for 4, up to 2.7 times the lookback's error gets by; with 2, white noise is corrected too.)
+template <class G>
+__device__ __forceinline__ bool sweep_agree(const SweepSection* sec, int lane, const float (&end)[G::R][G::D],
+                                            const float (&st)[G::R][G::D], const float* last, float (&r)[G::R][G::D]) {
+    constexpr int R = G::R, K = G::K, D = G::D;
+#pragma unroll
+    for (int c = 0; c < D; ++c) {
+        float next = __shfl_down_sync(FULL_MASK, st[0][c], 1);
+        if (lane == 31) next = last[c];
+#pragma unroll
+        for (int i = 0; i < R; ++i) r[i][c] = end[i][c] - (i + 1 < R ? st[i + 1 < R ? i + 1 : 0][c] : next);
+    }
+    bool ok = true;
+#pragma unroll
+    for (int s = 0; s < K; ++s) {
+        float top = 0.f, off = 0.f;
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+            top = fmaxf(top, fabsf(end[i][2 * s + 1]));
+            off = fmaxf(off, fmaxf(fabsf(r[i][2 * s + 1]), sec[s].wd * fabsf(r[i][2 * s])));
+        }
+        top = __uint_as_float(__reduce_max_sync(FULL_MASK, __float_as_uint(top)));
+        ok = ok && off <= sec[s].tol * top;
+    }
+    return __all_sync(FULL_MASK, ok);
+}
+
+// Adds the cascade's response to the states g before the lane's sub-rows to the outputs in the buffer.
+template <class G>
+__device__ __forceinline__ void sweep_respond(float* buf, const SweepSection* sec, int lane,
+                                              const float (&g)[G::R][G::D]) {
+    constexpr int K = G::K, N = G::N, R = G::R, P = R / 2;
+    f32x2 b1[K], b2[K], a1[K], a2[K], h[P][K][2];  // h: the sections' last two outputs
+#pragma unroll
+    for (int s = 0; s < K; ++s) {
+        b1[s] = pack2(sec[s].b1, sec[s].b1);
+        b2[s] = pack2(sec[s].b2, sec[s].b2);
+        a1[s] = pack2(sec[s].a1, sec[s].a1);
+        a2[s] = pack2(sec[s].a2, sec[s].a2);
+#pragma unroll
+        for (int p = 0; p < P; ++p) {
+            const float *u = g[2 * p] + 2 * s, *v = g[2 * p + 1] + 2 * s;
+            h[p][s][0] = pack2(u[1] - u[0], v[1] - v[0]);
+            h[p][s][1] = pack2(u[1], v[1]);
+        }
+    }
+    float* row = buf + (lane << 5);
+    const int l7 = lane & 7;
+#pragma unroll 1
+    for (int j = 0; j < N / 4; ++j) {
+        float* at = row + sub_granule_at<N>(0, j, l7);
+#pragma unroll
+        for (int p = 0; p < P; ++p) {
+            float y[2][4];
+#pragma unroll
+            for (int t = 0; t < 4; ++t) {
+                f32x2 in = 0ull, x2 = 0ull, x1 = 0ull;
+#pragma unroll
+                for (int s = 0; s < K; ++s) {
+                    const f32x2 w = s == 0 ? 0ull : fma2(b2[s], x2, fma2(b1[s], x1, in));
+                    x2 = h[p][s][0];
+                    x1 = h[p][s][1];
+                    in = fma2(a1[s], x1, fma2(a2[s], x2, w));
+                    h[p][s][0] = x1;
+                    h[p][s][1] = in;
+                }
+                unpack2(in, y[0][t], y[1][t]);
+            }
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                float4* q = reinterpret_cast<float4*>(at + (2 * p + i) * (N / 32) * 1024);
+                const float4 x = *q;
+                *q = make_float4(x.x + y[i][0], x.y + y[i][1], x.z + y[i][2], x.w + y[i][3]);
+            }
+        }
+    }
 }
 
 // ------------------------------------------------------------------------------------
@@ -379,15 +494,17 @@ struct IirSweepParams {
     SweepSection sec[IIR_MAX_SECTIONS];
 };
 
-constexpr unsigned SWEEP_RING = 64;  // item records and end states kept of the last items
+constexpr unsigned SWEEP_RING = 32;  // item records and end states kept of the last items
 constexpr unsigned SWEEP_WARM = 0x80000000u;
 
 template <int NB, int D>
 struct SweepAux {
     unsigned long long full[NB], empty[NB];
     float ends[SWEEP_RING][D];           // items' end states
+    float fix[SWEEP_RING][D];            // what they lack, where it matters
     unsigned int item[SWEEP_RING];       // the item's tile, SWEEP_WARM if only its end state is wanted
     volatile unsigned int ready[SWEEP_RING];  // i + 1 once item i's end state is in `ends`
+    volatile unsigned int checked[SWEEP_RING];  // 2 (i + 1) once it has been checked, plus 1 if `fix` is to be added
     volatile unsigned int issued[NB];    // items put into the buffer so far
     volatile unsigned int total;         // items of the block, once known
     volatile unsigned int abandon;       // a wait ran out: everybody leaves
@@ -398,8 +515,8 @@ struct SweepAux {
 // runs of consecutive tiles: block b starts with run b of run0 tiles, then draws runs of run1 tiles
 // from a ticket counter until they are gone. SMs differ in the bandwidth they get (a copy kernel
 // that splits a signal evenly among blocks reaches 6.2 TB/s, one that draws its tiles 7.0), so the
-// last part is drawn. Ahead of a run goes the tile before it, of which only the end state is
-// computed: no block needs anything from another.
+// last part is drawn. Ahead of a run goes the tile before it, which is filtered for its end state and
+// not stored: no block needs anything from another.
 //
 // Inside a block the items (tiles of its runs, one after another) are taken by the warps in order,
 // and item i's end state goes to item i + 1 through shared memory. It is the end state from rest:
@@ -427,7 +544,7 @@ __device__ __forceinline__ void sweep_tiles(const IirSweepParams& p, unsigned ch
             mbar_init(aux.empty + b, 1);
             aux.issued[b] = 0u;
         }
-        for (unsigned i = 0; i < SWEEP_RING; ++i) aux.ready[i] = 0u;
+        for (unsigned i = 0; i < SWEEP_RING; ++i) aux.ready[i] = aux.checked[i] = 0u;
         aux.next = 0u;
         aux.total = 0xffffffffu;
         aux.abandon = 0u;
@@ -564,11 +681,57 @@ __device__ __forceinline__ void sweep_tiles(const IirSweepParams& p, unsigned ch
                     tri_mad<K>(tab + G::T_PL + 4 * lane * G::ROW, X, st[0], st[0]);
                 }
             }
-            if (!warm) {
 #pragma unroll
-                for (int j = 1; j < R; ++j) tri_mad<K>(tab + G::T_PN, st[j - 1], e[j - 1], st[j]);
-                __syncwarp();  // every lane has read its neighbour's last samples
-                run(buf, lane, st, xh);
+            for (int j = 1; j < R; ++j) tri_mad<K>(tab + G::T_PN, st[j - 1], e[j - 1], st[j]);
+            __syncwarp();  // every lane has read its neighbour's last samples
+            float end[R][D];
+            run(buf, lane, st, xh, end);
+            {
+                float r[R][D], g[R][D], last[D];
+                const bool off = !sweep_agree<G>(p.sec, lane, end, st, aux.ends[i % SWEEP_RING], r);
+#pragma unroll
+                for (int c = 0; c < D; ++c) g[0][c] = 0.f;
+                if (off) {
+                    float f[D];
+                    sweep_join<G>(tab, r, f);
+                    sweep_scan<G>(tab, p.rounds, lane, f, g[0], last);
+                    if (lane == 31) {
+#pragma unroll
+                        for (int c = 0; c < D; c += 2)
+                            *reinterpret_cast<float2*>(&aux.fix[i % SWEEP_RING][c]) = make_float2(last[c], last[c + 1]);
+                    }
+                }
+                if (lane == 31) {
+                    __threadfence_block();
+                    aux.checked[i % SWEEP_RING] = 2u * (i + 1u) + (off ? 1u : 0u);
+                }
+                bool before = false;  // the state before the tile lacked something
+                if (!warm && t > 0) {
+                    const bool got = wait_for([&] { return aux.checked[(i - 1u) % SWEEP_RING] >> 1 == i; });
+                    if (__any_sync(FULL_MASK, !got)) break;
+                    __threadfence_block();
+                    before = (aux.checked[(i - 1u) % SWEEP_RING] & 1u) != 0u;
+                }
+                if (before && lane < p.lanes) {
+                    float X[D];
+#pragma unroll
+                    for (int c = 0; c < D; c += 2) {
+                        const float2 v = *reinterpret_cast<const float2*>(&aux.fix[(i - 1u) % SWEEP_RING][c]);
+                        X[c] = v.x;
+                        X[c + 1] = v.y;
+                    }
+                    tri_mad<K>(tab + G::T_PL + 4 * lane * G::ROW, X, g[0], g[0]);
+                }
+                if (!warm && (off || before)) {
+#pragma unroll
+                    for (int j = 1; j < R; ++j) {
+                        if (!off)
+#pragma unroll
+                            for (int c = 0; c < D; ++c) r[j - 1][c] = 0.f;
+                        tri_mad<K>(tab + G::T_PN, g[j - 1], r[j - 1], g[j]);
+                    }
+                    sweep_respond<G>(buf, p.sec, lane, g);
+                }
             }
             if (p.use_tma) {
                 fence_proxy_async_smem();  // generic accesses of the buffer before the async ones to come

@@ -59,3 +59,29 @@ def check(case, kernel, n, monkeypatch):
 @pytest.mark.parametrize("case", CASES, ids=lambda c: "-".join(map(str, c)))
 def test_cyclic_reduction(case, kernel, n, monkeypatch, cuda_device):
     check(case, kernel, n, monkeypatch)
+
+
+@pytest.mark.parametrize("n", (100_003, LARGE + 5000))
+@pytest.mark.parametrize("case", CASES, ids=lambda c: "-".join(map(str, c)))
+def test_state_sweep(case, n, monkeypatch, cuda_device):
+    check(case, "PH", n, monkeypatch)
+
+
+def test_state_sweep_burst(monkeypatch, cuda_device):
+    """A stop-band tone that comes and goes anywhere in a tile: the tile after it starts from a corrected
+    state although it has nothing to correct itself."""
+    n = LARGE + 40 * 4096
+    sos = design("cheby1", 10, 0.1, "low")
+    rng = np.random.default_rng(1)
+    x = rng.uniform(-1, 1, n)
+    t = np.arange(n)
+    for at, end in zip(rng.integers(0, n, 60), rng.integers(1, 9000, 60)):
+        x[at:at + end] += 100 * np.sin(0.97 * np.pi * t[at:at + end])
+    x[7 * 4096:9 * 4096] += 100 * np.sin(0.97 * np.pi * t[7 * 4096:9 * 4096])  # ends with a tile
+    x = x.astype(np.float32)
+    xt = torch.from_numpy(x).cuda()
+    _, ref = oracle.reference_golden(sos, x)
+    got = error(Plan(sos, "PH", max_n=n), xt, ref)
+    monkeypatch.setenv("IIR_GB300_TAIL", "0")
+    lookback = error(Plan(sos, "PH", max_n=n), xt, ref)
+    assert got <= 2 * lookback + 2.0 ** -24 * np.max(np.abs(ref)), (got, lookback)
