@@ -29,7 +29,7 @@ struct BatchSweepGeom {
     static constexpr int BLOCKS = K * (K + 1) / 2;
     static constexpr int T_A = 0;                             // [D][N] pass A
     static constexpr int T_H = T_A + D * N;                   // [D][2] response to (x[-2], x[-1])
-    static constexpr int T_C = T_H + 2 * D;                   // [K][4] b1, b2, a1, a2 (section 0: b g), then g
+    static constexpr int T_C = T_H + 2 * D;                   // [K][4] b1, b2, a1, a2, then the input gain
     static constexpr int T_PN = T_C + 4 * K + 4;              // [BLOCKS] Phi^N
     static constexpr int T_PS = T_PN + 4 * BLOCKS;            // [BSWEEP_STEPS][BLOCKS] Phi^(SPAN 2^k)
     static constexpr int T_PL = T_PS + 4 * BSWEEP_STEPS * BLOCKS;  // [BSWEEP_NEAR][BLOCKS] Phi^(SPAN l), if not chained
@@ -115,7 +115,7 @@ __device__ __forceinline__ void bsweep_run(float* buf, const float* tab, int lan
     for (int p = 0; p < P; ++p)
 #pragma unroll
         for (int t = 0; t < 2; ++t) {
-            h[p][0][t] = pack2(xh[2 * p][t], xh[2 * p + 1][t]);
+            h[p][0][t] = mul2(g, pack2(xh[2 * p][t], xh[2 * p + 1][t]));
 #pragma unroll
             for (int s = 0; s < K; ++s) {
                 const float* u = st[2 * p] + 2 * s;
@@ -139,10 +139,10 @@ __device__ __forceinline__ void bsweep_run(float* buf, const float* tab, int lan
                 v[p][s][0] = h[p][s][0];
                 v[p][s][1] = h[p][s][1];
             }
-            v[p][0][2] = pack2(x[2 * p].x, x[2 * p + 1].x);
-            v[p][0][3] = pack2(x[2 * p].y, x[2 * p + 1].y);
-            v[p][0][4] = pack2(x[2 * p].z, x[2 * p + 1].z);
-            v[p][0][5] = pack2(x[2 * p].w, x[2 * p + 1].w);
+            v[p][0][2] = mul2(g, pack2(x[2 * p].x, x[2 * p + 1].x));
+            v[p][0][3] = mul2(g, pack2(x[2 * p].y, x[2 * p + 1].y));
+            v[p][0][4] = mul2(g, pack2(x[2 * p].z, x[2 * p + 1].z));
+            v[p][0][5] = mul2(g, pack2(x[2 * p].w, x[2 * p + 1].w));
         }
 #pragma unroll
         for (int d = 0; d < K + 3; ++d) {
@@ -152,8 +152,7 @@ __device__ __forceinline__ void bsweep_run(float* buf, const float* tab, int lan
                 if (t < 2 || t > 5) continue;
 #pragma unroll
                 for (int p = 0; p < P; ++p) {
-                    const f32x2 in = s == 0 ? mul2(g, v[p][0][t]) : v[p][s][t];
-                    const f32x2 w = fma2(b2[s], v[p][s][t - 2], fma2(b1[s], v[p][s][t - 1], in));
+                    const f32x2 w = fma2(b2[s], v[p][s][t - 2], fma2(b1[s], v[p][s][t - 1], v[p][s][t]));
                     v[p][s + 1][t] = fma2(a1[s], v[p][s + 1][t - 1], fma2(a2[s], v[p][s + 1][t - 2], w));
                 }
             }
@@ -231,12 +230,13 @@ __device__ __forceinline__ void bsweep_state(const float* buf, const float* tab,
         y1[s] = u;
     }
     const float gain = tab[G::T_C + 4 * K];
+    h2 *= gain;
+    h1 *= gain;
 #pragma unroll 1
     for (int n = sub * N; n <= m % G::SPAN; ++n) {
-        const float xv = buf[tile_at(row, n)];
-        float w = gain * xv, g2 = h2, g1 = h1;
+        float w = gain * buf[tile_at(row, n)], g2 = h2, g1 = h1;
         h2 = h1;
-        h1 = xv;
+        h1 = w;
 #pragma unroll
         for (int s = 0; s < K; ++s) {
             const float4 c = *reinterpret_cast<const float4*>(tab + G::T_C + 4 * s);
@@ -488,8 +488,8 @@ __device__ __forceinline__ bool bsweep_item(const IirBatchSweepParams& p, BatchS
         }
         // the samples before the 16-byte grid, one by one
         for (int k = -static_cast<int>(run.peel); k < 0; ++k) {
-            const float xv = __ldg(x + k);
-            float w = tab[G::T_C + 4 * K] * xv, h2 = g2, h1 = g1;
+            const float xv = __ldg(x + k), gain = tab[G::T_C + 4 * K];
+            float w = gain * xv, h2 = gain * g2, h1 = gain * g1;
 #pragma unroll
             for (int s = 0; s < K; ++s) {
                 const float4 c = *reinterpret_cast<const float4*>(tab + G::T_C + 4 * s);

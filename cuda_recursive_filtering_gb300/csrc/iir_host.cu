@@ -717,9 +717,6 @@ int plan_add_sweeps(iir_plan* p, const std::vector<SectionF32>& secs, double gai
         const SweepLimits lim = sweep_limits(secs[s]);
         q.sec[s] = SweepSection{secs[s].b1, secs[s].b2, secs[s].a1, secs[s].a2, static_cast<float>(k), lim.wd, lim.tol};
     }
-    // the first section's input is the raw sample: its FIR taps carry the gain
-    q.sec[0].b1 = static_cast<float>(gain * secs[0].b1);
-    q.sec[0].b2 = static_cast<float>(gain * secs[0].b2);
     return IIR_OK;
 }
 

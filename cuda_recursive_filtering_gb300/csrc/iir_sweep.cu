@@ -295,21 +295,19 @@ double sweep_error(const SweepFilter& f, const std::vector<float>& t, int N, boo
             for (int n = 0; n < N; ++n) a[n & 1] = std::fmaf(t[static_cast<size_t>(c) * N + n], x[n], a[n & 1]);
             e[c] = std::fmaf(th[2 * c + 1], x1, std::fmaf(th[2 * c], x2, a[0] + a[1]));
         }
-        h[0] = x2;
-        h[1] = x1;
+        h[0] = g * x2;
+        h[1] = g * x1;
         for (int s = 0; s < K; ++s) {
             dl[s] = st[2 * s];
             h[2 * s + 2] = st[2 * s + 1] - st[2 * s];
             h[2 * s + 3] = st[2 * s + 1];
         }
         for (int n = 0; n < N; ++n) {
-            float in = x[n];
-            double rin = in;
+            float in = g * x[n];
+            double rin = f.gain * x[n];
             for (int s = 0; s < K; ++s) {
                 const SectionF32& q = f.secs[s];
-                const float b1 = s == 0 ? static_cast<float>(f.gain * q.b1) : q.b1;
-                const float b2 = s == 0 ? static_cast<float>(f.gain * q.b2) : q.b2;
-                const float w = std::fmaf(b2, h[2 * s], std::fmaf(b1, h[2 * s + 1], s == 0 ? g * in : in));
+                const float w = std::fmaf(q.b2, h[2 * s], std::fmaf(q.b1, h[2 * s + 1], in));
                 float y;
                 if (diff) {
                     const float k = static_cast<float>(static_cast<double>(q.a1) + q.a2 - 1.0);
@@ -321,8 +319,7 @@ double sweep_error(const SweepFilter& f, const std::vector<float>& t, int N, boo
                 h[2 * s] = h[2 * s + 1];
                 h[2 * s + 1] = in;
                 in = y;
-                const double gs = s == 0 ? f.gain : 1.0;
-                const double rw = gs * (rin + q.b1 * r[2 * s + 1] + q.b2 * r[2 * s]);
+                const double rw = rin + q.b1 * r[2 * s + 1] + q.b2 * r[2 * s];
                 const double ry = rw + q.a1 * r[2 * s + 3] + q.a2 * r[2 * s + 2];
                 r[2 * s] = r[2 * s + 1];
                 r[2 * s + 1] = rin;
@@ -405,10 +402,9 @@ BatchSweepFilter bsweep_filter(const SectionF32* secs, int K, double gain, int s
     t.assign(static_cast<size_t>(bsweep_table_floats(KP, span)), 0.f);
     put_dots(t, f, N, t_h);
     for (int s = 0; s < KP; ++s) {
-        // the first section's input is the raw sample: its FIR taps carry the gain
         float* c = t.data() + t_c + 4 * s;
-        c[0] = static_cast<float>(s == 0 ? gain * padded[0].b1 : padded[static_cast<size_t>(s)].b1);
-        c[1] = static_cast<float>(s == 0 ? gain * padded[0].b2 : padded[static_cast<size_t>(s)].b2);
+        c[0] = padded[static_cast<size_t>(s)].b1;
+        c[1] = padded[static_cast<size_t>(s)].b2;
         c[2] = padded[static_cast<size_t>(s)].a1;
         c[3] = padded[static_cast<size_t>(s)].a2;
     }

@@ -243,11 +243,14 @@ __device__ __forceinline__ void sweep_scan(const float* tab, int rounds, int lan
 __host__ __device__ constexpr int sweep_step_granules(int K) { return K <= 2 || K == 5 ? 4 : K == 8 ? 2 : 1; }
 
 struct SweepSection {
-    float b1, b2, a1, a2;  // section 0: b1, b2 carry the input gain (its input is the raw sample)
+    float b1, b2, a1, a2;
     float k;               // a1 + a2 - 1, rounded once: the difference form's coefficient
     float wd, tol;         // sweep_agree: weight of a difference's residual, and the largest ratio to the output
 };
 
+// The gain goes on the samples, not on the first section's taps: taps of 1, -2, 1 (a high pass) then cancel an
+// offset without rounding it.
+//
 // DIFF: the recurrence on the outputs' differences,
 //     d[n] = w[n] + (a1 + a2 - 1) y[n-1] - a2 d[n-1],   y[n] = y[n-1] + d[n],
 // one addition more per sample and section. A rounding of y[n] in the direct form enters its recurrence at
@@ -281,7 +284,7 @@ __device__ __forceinline__ void sweep_run_ph(float* buf, const SweepSection* sec
     for (int p = 0; p < P; ++p)
 #pragma unroll
         for (int t = 0; t < 2; ++t) {
-            h[p][0][t] = pack2(xh[2 * p][t], xh[2 * p + 1][t]);
+            h[p][0][t] = mul2(g, pack2(xh[2 * p][t], xh[2 * p + 1][t]));
 #pragma unroll
             for (int s = 0; s < K; ++s) {
                 // state pairs are (y[-1] - y[-2], y[-1])
@@ -315,10 +318,10 @@ __device__ __forceinline__ void sweep_run_ph(float* buf, const SweepSection* sec
             }
 #pragma unroll
             for (int b = 0; b < GB; ++b) {
-                v[p][0][4 * b + 2] = pack2(x[b][2 * p].x, x[b][2 * p + 1].x);
-                v[p][0][4 * b + 3] = pack2(x[b][2 * p].y, x[b][2 * p + 1].y);
-                v[p][0][4 * b + 4] = pack2(x[b][2 * p].z, x[b][2 * p + 1].z);
-                v[p][0][4 * b + 5] = pack2(x[b][2 * p].w, x[b][2 * p + 1].w);
+                v[p][0][4 * b + 2] = mul2(g, pack2(x[b][2 * p].x, x[b][2 * p + 1].x));
+                v[p][0][4 * b + 3] = mul2(g, pack2(x[b][2 * p].y, x[b][2 * p + 1].y));
+                v[p][0][4 * b + 4] = mul2(g, pack2(x[b][2 * p].z, x[b][2 * p + 1].z));
+                v[p][0][4 * b + 5] = mul2(g, pack2(x[b][2 * p].w, x[b][2 * p + 1].w));
             }
         }
 #pragma unroll
@@ -329,8 +332,7 @@ __device__ __forceinline__ void sweep_run_ph(float* buf, const SweepSection* sec
                 if (t < 2 || t > S + 1) continue;
 #pragma unroll
                 for (int p = 0; p < P; ++p) {
-                    const f32x2 in = s == 0 ? mul2(g, v[p][0][t]) : v[p][s][t];
-                    const f32x2 w = fma2(b2[s], v[p][s][t - 2], fma2(b1[s], v[p][s][t - 1], in));
+                    const f32x2 w = fma2(b2[s], v[p][s][t - 2], fma2(b1[s], v[p][s][t - 1], v[p][s][t]));
                     if constexpr (DIFF) {
                         dl[p][s] = fma2(a1[s], v[p][s + 1][t - 1], fma2(a2[s], dl[p][s], w));
                         v[p][s + 1][t] = add2(v[p][s + 1][t - 1], dl[p][s]);

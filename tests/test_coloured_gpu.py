@@ -85,3 +85,23 @@ def test_state_sweep_burst(monkeypatch, cuda_device):
     monkeypatch.setenv("IIR_GB300_TAIL", "0")
     lookback = error(Plan(sos, "PH", max_n=n), xt, ref)
     assert got <= 2 * lookback + 2.0 ** -24 * np.max(np.abs(ref)), (got, lookback)
+
+
+@pytest.mark.parametrize("n", (100_003, LARGE + 5000))
+@pytest.mark.parametrize("case", [("butter", 4, 0.02, "high", "offset"), ("butter", 6, 0.02, "high", "slow")],
+                         ids=lambda c: "-".join(map(str, c)))
+def test_high_pass_takes_an_offset_away(case, n, monkeypatch, cuda_device):
+    """A high pass whose taps, 1, -2, 1, cancel an offset exactly if the gain is not in them. The onset of the
+    offset is the output's peak, so the error is compared after it has rung out."""
+    sos = design(*case[:4])
+    x = coloured(n, case[4])
+    xt = torch.from_numpy(x).cuda()
+    _, ref = oracle.reference_golden(sos, x)
+    skip = 4096
+    plans = [Plan(sos, "PH", max_n=n)]
+    monkeypatch.setenv("IIR_GB300_TAIL", "0")
+    plans.append(Plan(sos, "PH", max_n=n))
+    got, lookback = [np.max(np.abs(p(xt).cpu().numpy().astype(np.float64) - ref)[skip:]) for p in plans]
+    for p in plans:
+        p.check()
+    assert got <= 2 * lookback + 2.0 ** -24 * np.max(np.abs(ref[skip:])), (got, lookback)
