@@ -88,9 +88,7 @@ __device__ __forceinline__ void bsweep_respond(const float* tab, int rounds, int
     }
 }
 
-// Pass B. State pairs are (y[-1] - y[-2], y[-1]): a low cutoff's two outputs
-// differ by little, and it is the difference that the recurrence amplifies. With CAPTURE, the sections'
-// outputs at sample `at` of this lane's row (-1: not here) and the one before it go to zf[2 s],
+// Pass B (states as in iir_sweep.cuh, sweep_sign). With CAPTURE, the sections' outputs at sample `at` of this lane's row (-1: not here) and the one before it go to zf[2 s],
 // zf[2 s + 1], s < kreal.
 template <class G, bool CAPTURE>
 __device__ __forceinline__ void bsweep_run(float* buf, const float* tab, int lane, const float (&st)[G::R][G::D],
@@ -99,9 +97,11 @@ __device__ __forceinline__ void bsweep_run(float* buf, const float* tab, int lan
     float* line = buf + (lane << 5);
     const int l7 = lane & 7;
     f32x2 b1[K], b2[K], a1[K], a2[K];
+    float sg[K];
 #pragma unroll
     for (int s = 0; s < K; ++s) {
         const float4 c = *reinterpret_cast<const float4*>(tab + G::T_C + 4 * s);
+        sg[s] = sweep_sign(c.z);
         b1[s] = pack2(c.x, c.x);
         b2[s] = pack2(c.y, c.y);
         a1[s] = pack2(c.z, c.z);
@@ -120,7 +120,7 @@ __device__ __forceinline__ void bsweep_run(float* buf, const float* tab, int lan
             for (int s = 0; s < K; ++s) {
                 const float* u = st[2 * p] + 2 * s;
                 const float* w = st[2 * p + 1] + 2 * s;
-                h[p][s + 1][t] = t == 0 ? pack2(u[1] - u[0], w[1] - w[0]) : pack2(u[1], w[1]);
+                h[p][s + 1][t] = t == 0 ? pack2(sg[s] * (u[1] - u[0]), sg[s] * (w[1] - w[0])) : pack2(u[1], w[1]);
             }
         }
 #pragma unroll(K > 4 ? 1 : 2)
@@ -226,7 +226,7 @@ __device__ __forceinline__ void bsweep_state(const float* buf, const float* tab,
 #pragma unroll
     for (int s = 0; s < K; ++s) {
         const float d = __shfl_sync(FULL_MASK, S[2 * s], row), u = __shfl_sync(FULL_MASK, S[2 * s + 1], row);
-        y2[s] = u - d;
+        y2[s] = sweep_sign(tab[G::T_C + 4 * s + 2]) * (u - d);
         y1[s] = u;
     }
     const float gain = tab[G::T_C + 4 * K];
@@ -506,7 +506,7 @@ __device__ __forceinline__ bool bsweep_item(const IirBatchSweepParams& p, BatchS
         }
 #pragma unroll
         for (int s = 0; s < K; ++s) {
-            X[2 * s] = y1[s] - y2[s];
+            X[2 * s] = fmaf(-sweep_sign(tab[G::T_C + 4 * s + 2]), y2[s], y1[s]);
             X[2 * s + 1] = y1[s];
             if (run.zf && have == 0 && lane == 0 && s < kreal) {  // nothing but the peeled samples
                 run.zf[2 + 2 * s] = y2[s];

@@ -713,7 +713,7 @@ int plan_add_sweeps(iir_plan* p, const std::vector<SectionF32>& secs, double gai
     q.state = p->d_state;
     q.gain = static_cast<float>(gain);
     for (int s = 0; s < p->n_sections; ++s) {
-        const double k = static_cast<double>(secs[s].a1) + secs[s].a2 - 1.0;
+        const double k = secs[s].a1 + sweep_sign(secs[s].a1) * (static_cast<double>(secs[s].a2) - 1.0);
         const SweepLimits lim = sweep_limits(secs[s]);
         q.sec[s] = SweepSection{secs[s].b1, secs[s].b2, secs[s].a1, secs[s].a2, static_cast<float>(k), lim.wd, lim.tol};
     }

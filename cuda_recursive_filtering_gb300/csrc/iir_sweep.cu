@@ -100,17 +100,17 @@ Mat mat_pow(Mat x, int e, int D) {
     return r;
 }
 
-// The kernels carry a section's state as (y[-1] - y[-2], y[-1]): a low cutoff's two outputs differ
-// by little, and it is the difference that the recurrence amplifies. 2x2 block (s, q) of a transition
-// of (y[-2], y[-1]) pairs, in that basis and in the kernels' column order.
-void put_block(std::vector<float>& t, size_t at, const Mat& m, int D, int s, int q) {
+// 2x2 block (s, q) of a transition of (y[-2], y[-1]) pairs, in the kernels' basis (sweep_sign) and column order.
+void put_block(std::vector<float>& t, size_t at, const Mat& m, const std::vector<SectionF32>& secs, int s, int q) {
+    const int D = 2 * static_cast<int>(secs.size());
+    const double ss = sweep_sign(secs[static_cast<size_t>(s)].a1), sq = sweep_sign(secs[static_cast<size_t>(q)].a1);
     const double* r0 = m.data() + static_cast<size_t>(2 * s) * D + 2 * q;
     const double* r1 = r0 + D;
-    // columns: a unit difference is (y[-2], y[-1]) = (-1, 0), a unit y[-1] is (1, 1)
-    const double d0 = -r0[0], d1 = -r1[0], u0 = r0[0] + r0[1], u1 = r1[0] + r1[1];
-    t[at] = static_cast<float>(d1 - d0);
+    // columns: a unit difference is (y[-2], y[-1]) = (-sq, 0), a unit y[-1] is (sq, 1)
+    const double d0 = -sq * r0[0], d1 = -sq * r1[0], u0 = sq * r0[0] + r0[1], u1 = sq * r1[0] + r1[1];
+    t[at] = static_cast<float>(d1 - ss * d0);
     t[at + 1] = static_cast<float>(d1);
-    t[at + 2] = static_cast<float>(u1 - u0);
+    t[at + 2] = static_cast<float>(u1 - ss * u0);
     t[at + 3] = static_cast<float>(u1);
 }
 
@@ -144,20 +144,21 @@ void put_dots(std::vector<float>& t, const SweepFilter& f, int N, size_t t_h) {
     auto ps = [&](int s, int n) { return n >= 0 ? p[static_cast<size_t>(s)][static_cast<size_t>(n)] : 0.0; };
     const double b1 = f.secs[0].b1, b2 = f.secs[0].b2, g = f.gain;
     for (int s = 0; s < K; ++s) {
-        float* t0 = t.data() + static_cast<size_t>(2 * s) * N;  // y[N-1] - y[N-2]
+        const double sg = sweep_sign(f.secs[static_cast<size_t>(s)].a1);
+        float* t0 = t.data() + static_cast<size_t>(2 * s) * N;  // y[N-1] - sg y[N-2]
         float* t1 = t0 + N;                                      // y[N-1]
         auto h = [&](int m) { return g * (ps(s, m) + b1 * ps(s, m - 1) + b2 * ps(s, m - 2)); };  // impulse response
         for (int n = 0; n < N; ++n) {
             const double y1 = h(N - 1 - n), y2 = h(N - 2 - n);
-            t0[n] = static_cast<float>(y1 - y2);
+            t0[n] = static_cast<float>(y1 - sg * y2);
             t1[n] = static_cast<float>(y1);
         }
         // (x[-2], x[-1]) reach the sub-row through section 0's FIR taps
         auto h2 = [&](int m) { return g * b2 * ps(s, m); };
         auto h1 = [&](int m) { return g * (b1 * ps(s, m) + b2 * ps(s, m - 1)); };
         float* th = t.data() + t_h + 4 * s;
-        th[0] = static_cast<float>(h2(N - 1) - h2(N - 2));
-        th[1] = static_cast<float>(h1(N - 1) - h1(N - 2));
+        th[0] = static_cast<float>(h2(N - 1) - sg * h2(N - 2));
+        th[1] = static_cast<float>(h1(N - 1) - sg * h1(N - 2));
         th[2] = static_cast<float>(h2(N - 1));
         th[3] = static_cast<float>(h1(N - 1));
     }
@@ -254,7 +255,7 @@ std::vector<float> sweep_tables(const SweepFilter& f, int N, int R) {
     put_dots(t, f, N, t_h);
     auto put = [&](size_t at, const Mat& m) {
         for (int s = 0; s < K; ++s)
-            for (int q = 0; q <= s; ++q) put_block(t, at + 4 * static_cast<size_t>(s * (s + 1) / 2 + q), m, D, s, q);
+            for (int q = 0; q <= s; ++q) put_block(t, at + 4 * static_cast<size_t>(s * (s + 1) / 2 + q), m, f.secs, s, q);
     };
     put(t_pn, mat_pow(f.phi, N, D));
     const Mat step = mat_pow(f.phi, span, D);
@@ -270,8 +271,8 @@ SweepLimits sweep_limits(const SectionF32& s) {
     const double a1 = s.a1, a2 = s.a2;
     // power gain of 1 / (1 - a1 z^-1 - a2 z^-2): white noise that enters the recurrence comes out by it
     const double noise = (1.0 - a2) / ((1.0 + a2) * ((1.0 - a2) * (1.0 - a2) - a1 * a1));
-    // an error of the difference grows to about 1 / (the pole's angle) of the output, its square k's size
-    const double angle = std::sqrt(std::fabs(a1 + a2 - 1.0));
+    // an error of the difference grows to about 1 / (the pole's angle from sg) in the output, its square k's size
+    const double angle = std::sqrt(std::fabs(a1 + sweep_sign(s.a1) * (a2 - 1.0)));
     return SweepLimits{static_cast<float>(angle < 1.0 ? 1.0 / std::max(angle, 1e-6) : 1.0),
                        static_cast<float>(4.0 * 0x1p-24 * (1.0 + (noise > 0.0 ? std::sqrt(noise) : 0.0)))};
 }
@@ -299,7 +300,7 @@ double sweep_error(const SweepFilter& f, const std::vector<float>& t, int N, boo
         h[1] = g * x1;
         for (int s = 0; s < K; ++s) {
             dl[s] = st[2 * s];
-            h[2 * s + 2] = st[2 * s + 1] - st[2 * s];
+            h[2 * s + 2] = sweep_sign(f.secs[static_cast<size_t>(s)].a1) * (st[2 * s + 1] - st[2 * s]);
             h[2 * s + 3] = st[2 * s + 1];
         }
         for (int n = 0; n < N; ++n) {
@@ -310,9 +311,9 @@ double sweep_error(const SweepFilter& f, const std::vector<float>& t, int N, boo
                 const float w = std::fmaf(q.b2, h[2 * s], std::fmaf(q.b1, h[2 * s + 1], in));
                 float y;
                 if (diff) {
-                    const float k = static_cast<float>(static_cast<double>(q.a1) + q.a2 - 1.0);
-                    dl[s] = std::fmaf(k, h[2 * s + 3], std::fmaf(-q.a2, dl[s], w));
-                    y = h[2 * s + 3] + dl[s];
+                    const float sg = sweep_sign(q.a1), k = static_cast<float>(q.a1 + sg * (static_cast<double>(q.a2) - 1.0));
+                    dl[s] = std::fmaf(k, h[2 * s + 3], std::fmaf(-sg * q.a2, dl[s], w));
+                    y = std::fmaf(sg, h[2 * s + 3], dl[s]);
                 } else {
                     y = std::fmaf(q.a1, h[2 * s + 3], std::fmaf(q.a2, h[2 * s + 2], w));
                 }
@@ -411,7 +412,7 @@ BatchSweepFilter bsweep_filter(const SectionF32* secs, int K, double gain, int s
     t[t_c + 4 * static_cast<size_t>(KP)] = static_cast<float>(gain);
     auto put = [&](size_t at, const Mat& m) {
         for (int s = 0; s < KP; ++s)
-            for (int q = 0; q <= s; ++q) put_block(t, at + 4 * static_cast<size_t>(s * (s + 1) / 2 + q), m, D, s, q);
+            for (int q = 0; q <= s; ++q) put_block(t, at + 4 * static_cast<size_t>(s * (s + 1) / 2 + q), m, f.secs, s, q);
     };
     put(t_pn, power(log2i(N)));
     for (int j = 0; j < BSWEEP_STEPS; ++j) put(t_ps + 4 * static_cast<size_t>(j) * blocks, power(ls + j));

@@ -242,9 +242,14 @@ __device__ __forceinline__ void sweep_scan(const float* tab, int rounds, int lan
 // / 380).
 __host__ __device__ constexpr int sweep_step_granules(int K) { return K <= 2 || K == 5 ? 4 : K == 8 ? 2 : 1; }
 
+// A section's state is carried as (y[-1] - sg y[-2], y[-1]), sg = 1 for poles on the right of the circle and -1 on
+// the left: two outputs near a slow pole differ by little (near a pole at -1, from the negative), and it is that
+// difference that the recurrence amplifies.
+__host__ __device__ constexpr float sweep_sign(float a1) { return a1 < 0.f ? -1.f : 1.f; }
+
 struct SweepSection {
     float b1, b2, a1, a2;
-    float k;               // a1 + a2 - 1, rounded once: the difference form's coefficient
+    float k;               // a1 + sg (a2 - 1), rounded once: the difference form's coefficient
     float wd, tol;         // sweep_agree: weight of a difference's residual, and the largest ratio to the output
 };
 
@@ -252,10 +257,10 @@ struct SweepSection {
 // offset without rounding it.
 //
 // DIFF: the recurrence on the outputs' differences,
-//     d[n] = w[n] + (a1 + a2 - 1) y[n-1] - a2 d[n-1],   y[n] = y[n-1] + d[n],
+//     d[n] = w[n] + (a1 + sg (a2 - 1)) y[n-1] - sg a2 d[n-1],   y[n] = sg y[n-1] + d[n],
 // one addition more per sample and section. A rounding of y[n] in the direct form enters its recurrence at
 // full gain, 1 / A(z), which a low cutoff makes large; here the rounding of y[n] is the only one of y's own
-// size, and it meets (1 + a2 z^-1) / A(z), smaller by the cutoff's angle. Error against 64 bits (2-norm,
+// size, and it meets (1 + sg a2 z^-1) / A(z), smaller by the pole's angle. Error against 64 bits (2-norm,
 // butter(16, .)): cutoff 0.05 3.0e-7 (direct form 1.11e-6, precision form 7.4e-7), 0.1 2.6e-7 (5.8e-7,
 // 6.5e-7), 0.4 3.0e-7 (2.3e-7, 5.3e-7). Time at 2^27 samples, cutoff 0.1, orders 12 / 16: 291 / 357 us
 // against 259 / 330 direct and 443 / 399 in the precision form.
@@ -264,13 +269,15 @@ __device__ __forceinline__ void sweep_run_ph(float* buf, const SweepSection* sec
                                              const float (&st)[G::R][G::D], const float (&xh)[G::R][2],
                                              float (&end)[G::R][G::D]) {
     constexpr int K = G::K, N = G::N, R = G::R, P = R / 2;
-    f32x2 b1[K], b2[K], a1[K], a2[K];
+    f32x2 b1[K], b2[K], a1[K], a2[K], sg[DIFF ? K : 1];
 #pragma unroll
     for (int s = 0; s < K; ++s) {
+        const float sign = sweep_sign(sec[s].a1);
         b1[s] = pack2(sec[s].b1, sec[s].b1);
         b2[s] = pack2(sec[s].b2, sec[s].b2);
         a1[s] = DIFF ? pack2(sec[s].k, sec[s].k) : pack2(sec[s].a1, sec[s].a1);
-        a2[s] = DIFF ? pack2(-sec[s].a2, -sec[s].a2) : pack2(sec[s].a2, sec[s].a2);
+        a2[s] = DIFF ? pack2(-sign * sec[s].a2, -sign * sec[s].a2) : pack2(sec[s].a2, sec[s].a2);
+        if constexpr (DIFF) sg[s] = pack2(sign, sign);
     }
     f32x2 dl[P][K];  // DIFF: the sections' last differences
 #pragma unroll
@@ -287,10 +294,10 @@ __device__ __forceinline__ void sweep_run_ph(float* buf, const SweepSection* sec
             h[p][0][t] = mul2(g, pack2(xh[2 * p][t], xh[2 * p + 1][t]));
 #pragma unroll
             for (int s = 0; s < K; ++s) {
-                // state pairs are (y[-1] - y[-2], y[-1])
                 const float* u = st[2 * p] + 2 * s;
                 const float* v = st[2 * p + 1] + 2 * s;
-                h[p][s + 1][t] = t == 0 ? pack2(u[1] - u[0], v[1] - v[0]) : pack2(u[1], v[1]);
+                const float sign = sweep_sign(sec[s].a1);
+                h[p][s + 1][t] = t == 0 ? pack2(sign * (u[1] - u[0]), sign * (v[1] - v[0])) : pack2(u[1], v[1]);
             }
         }
     float* row = buf + (lane << 5);
@@ -335,7 +342,7 @@ __device__ __forceinline__ void sweep_run_ph(float* buf, const SweepSection* sec
                     const f32x2 w = fma2(b2[s], v[p][s][t - 2], fma2(b1[s], v[p][s][t - 1], v[p][s][t]));
                     if constexpr (DIFF) {
                         dl[p][s] = fma2(a1[s], v[p][s + 1][t - 1], fma2(a2[s], dl[p][s], w));
-                        v[p][s + 1][t] = add2(v[p][s + 1][t - 1], dl[p][s]);
+                        v[p][s + 1][t] = fma2(sg[s], v[p][s + 1][t - 1], dl[p][s]);
                     } else {
                         v[p][s + 1][t] = fma2(a1[s], v[p][s + 1][t - 1], fma2(a2[s], v[p][s + 1][t - 2], w));
                     }
@@ -375,8 +382,9 @@ __device__ __forceinline__ void sweep_run_ph(float* buf, const SweepSection* sec
             } else {
                 float za, zb;
                 unpack2(h[p][s + 1][0], za, zb);
-                end[2 * p][2 * s] = ya - za;
-                end[2 * p + 1][2 * s] = yb - zb;
+                const float sign = sweep_sign(sec[s].a1);
+                end[2 * p][2 * s] = fmaf(-sign, za, ya);
+                end[2 * p + 1][2 * s] = fmaf(-sign, zb, yb);
             }
         }
 }
@@ -440,7 +448,8 @@ __device__ __forceinline__ void sweep_respond(float* buf, const SweepSection* se
 #pragma unroll
         for (int p = 0; p < P; ++p) {
             const float *u = g[2 * p] + 2 * s, *v = g[2 * p + 1] + 2 * s;
-            h[p][s][0] = pack2(u[1] - u[0], v[1] - v[0]);
+            const float sign = sweep_sign(sec[s].a1);
+            h[p][s][0] = pack2(sign * (u[1] - u[0]), sign * (v[1] - v[0]));
             h[p][s][1] = pack2(u[1], v[1]);
         }
     }

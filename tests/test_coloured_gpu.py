@@ -105,3 +105,22 @@ def test_high_pass_takes_an_offset_away(case, n, monkeypatch, cuda_device):
     for p in plans:
         p.check()
     assert got <= 2 * lookback + 2.0 ** -24 * np.max(np.abs(ref[skip:])), (got, lookback)
+
+
+@pytest.mark.parametrize("kernel,order", [("PH", 8), ("AUTO", 12)])
+@pytest.mark.parametrize("cutoff", (0.8, 0.9))
+def test_poles_near_minus_one(cutoff, kernel, order, monkeypatch, cuda_device):
+    """Outputs near a slow pole at -1 alternate. Mean square error against the lookback schedule's, with a
+    tenth more for the order of the sums."""
+    sos = design("butter", order, cutoff, "high")
+    n = LARGE + 5000
+    x = np.random.default_rng(order).uniform(-1, 1, n).astype(np.float32)
+    xt = torch.from_numpy(x).cuda()
+    ref = torch.from_numpy(oracle.reference_golden(sos, x)[1]).cuda()
+    plans = [Plan(sos, kernel, max_n=n)]
+    monkeypatch.setenv("IIR_GB300_TAIL", "0")
+    plans.append(Plan(sos, "PH", max_n=n))
+    got, lookback = [float((p(xt).double() - ref).square().mean().sqrt()) for p in plans]
+    for p in plans:
+        p.check()
+    assert got <= 1.1 * lookback, (got, lookback)
