@@ -444,6 +444,7 @@ struct SweepPart {
     float* d_tab = nullptr;
     int lanes = 0;  // lanes that a state reaches
     int resident = 0;
+    float tol[IIR_MAX_SECTIONS];  // SweepSection::tol for its sub-rows
 };
 
 struct iir_plan {
@@ -707,6 +708,7 @@ int plan_add_sweeps(iir_plan* p, const std::vector<SectionF32>& secs, double gai
             return st;
         }
         s.resident = nb * p->sms;
+        for (int j = 0; j < p->n_sections; ++j) s.tol[j] = sweep_limits(secs[j], k->N).tol;
         p->sweeps.push_back(s);
     }
     IirSweepParams& q = p->sweep;
@@ -714,8 +716,8 @@ int plan_add_sweeps(iir_plan* p, const std::vector<SectionF32>& secs, double gai
     q.gain = static_cast<float>(gain);
     for (int s = 0; s < p->n_sections; ++s) {
         const double k = secs[s].a1 + sweep_sign(secs[s].a1) * (static_cast<double>(secs[s].a2) - 1.0);
-        const SweepLimits lim = sweep_limits(secs[s]);
-        q.sec[s] = SweepSection{secs[s].b1, secs[s].b2, secs[s].a1, secs[s].a2, static_cast<float>(k), lim.wd, lim.tol};
+        q.sec[s] = SweepSection{secs[s].b1, secs[s].b2, secs[s].a1, secs[s].a2, static_cast<float>(k),
+                                sweep_limits(secs[s], 1).wd, 0.f};
     }
     return IIR_OK;
 }
@@ -1055,6 +1057,7 @@ int sweep_launch(iir_plan* p, const SweepPart& s, const float* x, float* y, size
     q.timeout_ns = p->timeout_ns;
     q.ntiles = static_cast<unsigned>(tiles);
     q.lanes = s.lanes;
+    for (int j = 0; j < p->n_sections; ++j) q.sec[j].tol = s.tol[j];
     q.rounds = 0;
     while ((1 << q.rounds) < s.lanes) ++q.rounds;
     const bool aligned = ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) & 15u) == 0;

@@ -267,14 +267,20 @@ std::vector<float> sweep_tables(const SweepFilter& f, int N, int R) {
     return t;
 }
 
-SweepLimits sweep_limits(const SectionF32& s) {
+SweepLimits sweep_limits(const SectionF32& s, int N) {
     const double a1 = s.a1, a2 = s.a2;
-    // power gain of 1 / (1 - a1 z^-1 - a2 z^-2): white noise that enters the recurrence comes out by it
-    const double noise = (1.0 - a2) / ((1.0 + a2) * ((1.0 - a2) * (1.0 - a2) - a1 * a1));
+    // power gain of 1 / (1 - a1 z^-1 - a2 z^-2) over a sub-row: roundings that enter the recurrence come out by it
+    double noise = 0.0, y1 = 0.0, y2 = 0.0;
+    for (int n = 0; n < N; ++n) {
+        const double y = (n == 0 ? 1.0 : 0.0) + a1 * y1 + a2 * y2;
+        noise += y * y;
+        y2 = y1;
+        y1 = y;
+    }
     // an error of the difference grows to about 1 / (the pole's angle from sg) in the output, its square k's size
     const double angle = std::sqrt(std::fabs(a1 + sweep_sign(s.a1) * (a2 - 1.0)));
     return SweepLimits{static_cast<float>(angle < 1.0 ? 1.0 / std::max(angle, 1e-6) : 1.0),
-                       static_cast<float>(4.0 * 0x1p-24 * (1.0 + (noise > 0.0 ? std::sqrt(noise) : 0.0)))};
+                       static_cast<float>(4.0 * 0x1p-24 * (1.0 + std::sqrt(noise)))};
 }
 
 double sweep_error(const SweepFilter& f, const std::vector<float>& t, int N, bool diff) {

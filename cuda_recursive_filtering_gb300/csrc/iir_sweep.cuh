@@ -405,8 +405,9 @@ __device__ __forceinline__ void sweep_run_ph(float* buf, const SweepSection* sec
 
 // Residuals r of the lane's sub-rows (r[i]: at its end), from pass B's end states, the states st that it started
 // from and the tile's end state `last`. True if all are within a section's rounding: tol = 4 x 2^-24 x (1 + the
-// noise gain of 1 / A) of its largest output in the tile, a difference weighed by what it grows to. (With 12
-// for 4, up to 2.7 times the lookback's error gets by; with 2, white noise is corrected too.)
+// noise gain of 1 / A over a sub-row) of its largest output in the tile, a difference weighed by what it grows
+// to. (With 6 for 4, up to twice the lookback's error gets by: a tone in the stop band of cheby1(4, 1, 0.02); with
+// 3, white noise is corrected by half as many filters more.)
 template <class G>
 __device__ __forceinline__ bool sweep_agree(const SweepSection* sec, int lane, const float (&end)[G::R][G::D],
                                             const float (&st)[G::R][G::D], const float* last, float (&r)[G::R][G::D]) {

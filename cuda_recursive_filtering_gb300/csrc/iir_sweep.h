@@ -43,11 +43,11 @@ bool sweep_too_slow(const SectionF32* secs, int K, int samples);
 int sweep_decay(const SweepFilter& f, int unit, int most);
 // The tables of one kernel geometry (SweepGeom's layout).
 std::vector<float> sweep_tables(const SweepFilter& f, int N, int R);
-// What a section's residuals are held to (sweep_agree).
+// What a section's residuals at the end of a sub-row of N samples are held to (sweep_agree).
 struct SweepLimits {
     float wd, tol;
 };
-SweepLimits sweep_limits(const SectionF32& s);
+SweepLimits sweep_limits(const SectionF32& s, int N);
 // Relative error (2-norm, against 64 bits) of the schedule's float32 arithmetic on white noise, with pass B
 // in the direct form or on differences: the kernel's steps done on the host over 40 sub-rows, with its tables.
 double sweep_error(const SweepFilter& f, const std::vector<float>& tables, int N, bool diff);

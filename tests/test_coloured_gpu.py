@@ -19,7 +19,8 @@ pytestmark = pytest.mark.gpu
 
 LARGE = 152 * 16384  # samples from which PH's large-signal sweep kernel runs
 CASES = [("cheby1", 10, 0.1, "low", "stop"), ("cheby1", 12, 0.5, "low", "stop"), ("butter", 8, 0.05, "low", "stop"),
-         ("butter", 8, 0.8, "high", "slow"), ("butter", 4, 0.8, "high", "offset")]
+         ("butter", 8, 0.8, "high", "slow"), ("butter", 4, 0.8, "high", "offset"), ("cheby1", 4, 0.02, "low", "stop"),
+         ("cheby1", 6, 0.04, "low", "stop")]
 
 
 def design(kind, order, cutoff, btype):
