@@ -488,6 +488,7 @@ struct iir_plan {
     // signals first; empty: the lookback kernels above filter every signal.
     std::vector<SweepPart> sweeps;
     int sweep_kind = 0;  // which of the sweep kernels: the plan's kind, or SWEEP_KIND_PH_DIFF
+    size_t sweep_min_n = 0;  // signals below it keep the lookback kernels (sweep_pick)
     IirSweepParams sweep{};
 };
 
@@ -508,8 +509,9 @@ int default_geometry(int kind, int n_sections, int& B, int& N) {
 // The realization that AUTO stands for: PH up to 5 sections (at 6 and more PH's direct form rounds more than
 // the precision form for many filters). From 6 on, PH on the state sweep, in the direct form or on
 // differences (`sweep_kind`), for filters whose float32 error there is below the precision form's: it is
-// found by doing the sweep's arithmetic on the host (within a fifth of the device's error for 40 designs of
-// orders 12 and 16), and the precision form's is 3.7e-7 to 7.4e-7 for all of them. Orders 12 / 16 at 2^27
+// found by doing the sweep's arithmetic on the host, on noise and, where the filter passes it, an offset (within a
+// fifth of the device's error for 40 designs of orders 12 and 16), and the precision form's is 2.8e-7 to 7.4e-7 for all
+// of them. Nor may the sweep have to correct white noise (order 16 at 2^20 samples: 23 us, precision form 15). Orders 12 / 16 at 2^27
 // samples: direct 259 / 330 us, differences 291 / 357, precision form 443 / 399; at 2^20: 11 / 13, 12 / 14,
 // 15 / 15. Low passes up to half of the band qualify, the direct form from a cutoff of about 0.2 on;
 // Chebyshev filters, high passes near zero and filters that do not decay within a tile do not.
@@ -518,15 +520,24 @@ int resolve_auto(const std::vector<SectionF32>& secs, double gain, int& sweep_ki
     sweep_kind = IIR_KIND_PH;
     if (K < SWEEP_DIFF_MIN_SECTIONS) return IIR_KERNEL_PH;
     if (tail_max_pieces() <= 0) return IIR_KERNEL_TC;  // the lookback schedules are asked for
-    const SweepKernel* k = sweep_kernels(SWEEP_KIND_PH_DIFF, K).front();
-    if (sweep_too_slow(secs.data(), K, SWEEP_LANES * k->span())) return IIR_KERNEL_TC;
+    // both kernels have to cover the filter: with the large one alone, small signals lie on few SMs (order 16,
+    // cutoff 0.025, 2^16 samples: 19 us, precision form 14)
+    const SweepKernel *large = sweep_kernels(SWEEP_KIND_PH_DIFF, K).front(), *small = sweep_kernels(SWEEP_KIND_PH_DIFF, K).back();
+    if (sweep_too_slow(secs.data(), K, SWEEP_LANES * small->span())) return IIR_KERNEL_TC;
     const SweepFilter f = sweep_filter(secs.data(), K, gain);
-    if (sweep_decay(f, k->span(), SWEEP_LANES) == 0) return IIR_KERNEL_TC;
-    constexpr double limit = 3e-7;
-    const std::vector<float> tables = sweep_tables(f, k->N, k->R);
-    if (sweep_error(f, tables, k->N, false) <= limit) return IIR_KERNEL_PH;
+    if (sweep_decay(f, small->span(), SWEEP_LANES) == 0) return IIR_KERNEL_TC;
+    const std::vector<float> tables = sweep_tables(f, large->N, large->R), short_rows = sweep_tables(f, small->N, small->R);
+    double dc = gain;
+    for (const SectionF32& s : secs) dc *= (1.0 + s.b1 + s.b2) / (1.0 - s.a1 - s.a2);
+    const float offset = std::fabs(dc) > 0.5 ? 1000.f : 0.f;
+    auto fits = [&](bool diff) {
+        const SweepTrial t = sweep_trial(f, tables, large->N, diff, 40);
+        return t.error <= 3e-7 && t.residual <= 0.7 && sweep_trial(f, tables, large->N, diff, 40, offset).error <= 3e-7 &&
+               sweep_trial(f, short_rows, small->N, diff, 40).residual <= 0.7;
+    };
+    if (fits(false)) return IIR_KERNEL_PH;
     sweep_kind = SWEEP_KIND_PH_DIFF;
-    return sweep_error(f, tables, k->N, true) <= limit ? IIR_KERNEL_PH : IIR_KERNEL_TC;
+    return fits(true) ? IIR_KERNEL_PH : IIR_KERNEL_TC;
 }
 
 // samples per block (= per lookback unit) of the plan's large-signal kernel, or of kernel e
@@ -681,8 +692,25 @@ void matmul_k(const std::vector<double>& A, const std::vector<double>& B, std::v
     C.swap(R);
 }
 
-// Adds the plan's state-sweep kernels: those whose tiles cover the filter's decay.
-int plan_add_sweeps(iir_plan* p, const std::vector<SectionF32>& secs, double gain) {
+// Largest signal that PLR filters with a block per chunk where it has a warp per chunk: the warps of a block
+// crowd a small signal onto few SMs (order 4, graph replays, block / warp: 2^16 samples 5.4 / 11.0 us, 2^20
+// 14.2 / 15.2, 3e6 33.0 / 16.1).
+constexpr size_t PLR_BLOCK_MAX_N = size_t(1) << 20;
+
+// From this many samples per SM on, a signal takes the large-signal sweep kernel (GB300, CUDA graph replays, large /
+// small kernel: order 8 13.1 / 9.4 us at 1e6 samples, 13.4 / 11.5 at 2.4e6, 13.1 / 15.5 at 3e6). The small kernel of
+// 8 sections has room for two blocks per SM, not three (order 16: 18.9 / 13.6 at 1.6e6, 18.9 / 20.3 at 2e6).
+constexpr size_t sweep_large_per_sm(int K) { return K == 8 ? 12288 : 16384; }
+
+// Below sweep_large_per_sm the lookback kernels filter
+//   * single sections, which have one-block-per-chunk kernels there (order 2: 8.7 us against 6.9 at 2^20, 9.5
+//     against 10.7 at 3e6; PLR's order 2 has none: 2^20 samples 8.9 us, 8.7 on the sweep; 3e6 22.5, 9.2);
+//   * from 4 sections on, filters for which the sweep has to correct white noise (cheby1(12, 1, 0.3), sweep /
+//     lookback: 2^18 samples 21.2 / 16.8 us, 2.4e6 21.6 / 20.9; butter(6, 0.02, high): 9.0 / 10.6);
+//   * below half of it, filters that decay within a large tile but not within a small one (butter(4, 0.01): 2^18
+//     samples 10.1 / 8.5 us, 2^20 10.2 / 9.2, 2.4e6 10.6 / 12.9).
+// Adds the plan's state-sweep kernels: those whose tiles cover the filter's decay. automatic: AUTO chose them.
+int plan_add_sweeps(iir_plan* p, const std::vector<SectionF32>& secs, double gain, bool automatic) {
     if (tail_max_pieces() <= 0) return IIR_OK;  // the lookback everywhere
     if (p->n_sections == 1 && (!pipeline_enabled() || std::getenv("IIR_GB300_SMALL_N"))) return IIR_OK;
     const std::vector<const SweepKernel*> kernels = sweep_kernels(p->sweep_kind, p->n_sections);
@@ -711,6 +739,16 @@ int plan_add_sweeps(iir_plan* p, const std::vector<SectionF32>& secs, double gai
         for (int j = 0; j < p->n_sections; ++j) s.tol[j] = sweep_limits(secs[j], k->N).tol;
         p->sweeps.push_back(s);
     }
+    if (!p->sweeps.empty()) {
+        const SweepPart& last = p->sweeps.back();
+        // (AUTO's choice from 6 sections on holds for every size)
+        const bool chosen = p->n_sections >= SWEEP_DIFF_MIN_SECTIONS && automatic;
+        const size_t large = sweep_large_per_sm(p->n_sections) * static_cast<size_t>(p->sms);
+        if (p->n_sections == 1) p->sweep_min_n = p->kind == IIR_KIND_PLR ? PLR_BLOCK_MAX_N + 1 : large;
+        else if (!chosen && p->n_sections >= 4 && sweep_trial(f, sweep_tables(f, last.k->N, last.k->R), last.k->N, false, 24).residual > 0.7)
+            p->sweep_min_n = large;
+        else if (!chosen && last.k == kernels.front()) p->sweep_min_n = large / 2;
+    }
     IirSweepParams& q = p->sweep;
     q.state = p->d_state;
     q.gain = static_cast<float>(gain);
@@ -721,11 +759,6 @@ int plan_add_sweeps(iir_plan* p, const std::vector<SectionF32>& secs, double gai
     }
     return IIR_OK;
 }
-
-// Largest signal that PLR filters with a block per chunk where it has a warp per chunk: the warps of a block
-// crowd a small signal onto few SMs (order 4, graph replays, block / warp: 2^16 samples 5.4 / 11.0 us, 2^20
-// 14.2 / 15.2, 3e6 33.0 / 16.1).
-constexpr size_t PLR_BLOCK_MAX_N = size_t(1) << 20;
 
 int plan_create_plr(iir_plan** out, const double* b, const double* a, int order, double gain, int B, int X,
                     size_t max_n) {
@@ -823,7 +856,7 @@ int plan_create_plr(iir_plan** out, const double* b, const double* a, int order,
         // one section: the direct form is PH's (2^25 samples: 193 us with a block per chunk, 44 on the sweep;
         // errors against 64 bits 1.7e-7 and 1.2e-7 at a cutoff of 0.1)
         p->sweep_kind = IIR_KIND_PH;
-        st = plan_add_sweeps(p, {SectionF32{q.b[0], q.b[1], q.a[0], q.a[1]}}, gain);
+        st = plan_add_sweeps(p, {SectionF32{q.b[0], q.b[1], q.a[0], q.a[1]}}, gain, false);
         if (st) {
             plan_free(p);
             return st;
@@ -882,7 +915,8 @@ int iir_plan_create(iir_plan** out, const float* sos, int n_sections, int kernel
     int st = normalise_sos(sos, n_sections, secs, gain);
     if (st) return st;
     int sweep_kind = kernel;
-    if (kernel == IIR_KERNEL_AUTO) {
+    const bool automatic = kernel == IIR_KERNEL_AUTO;
+    if (automatic) {
         kernel = resolve_auto(secs, gain, sweep_kind);
         // (the precision form takes no geometry, so from 6 sections on AUTO takes none)
         if (n_sections >= SWEEP_DIFF_MIN_SECTIONS) block_size = n_blocks = 0;
@@ -1004,7 +1038,7 @@ int iir_plan_create(iir_plan** out, const float* sos, int n_sections, int kernel
     q.gain = static_cast<float>(gain);
     q.tail_pieces = pieces;
     p->sweep_kind = sweep_kind;
-    st = plan_add_sweeps(p, secs, gain);
+    st = plan_add_sweeps(p, secs, gain, automatic);
     if (st) {
         plan_free(p);
         return st;
@@ -1030,18 +1064,10 @@ size_t sweep_tile_count(const SweepPart& s, size_t n) {
     return (n + tile - 1) / tile;
 }
 
-// From this many samples per SM on, a signal takes the large-signal sweep kernel (GB300, CUDA graph
-// replays, large / small kernel: order 8 11.3 / 8.9 us at 2^20 samples, 12.4 / 12.8 at 3e6, 20.1 / 22.7
-// at 2^23; order 16 17.7 / 13.2, 18.5 / 22.4, 32 / 39). Single sections below it keep their
-// one-block-per-chunk kernels (order 2: 8.7 us against 6.9 at 2^20, 9.5 against 10.7 at 3e6).
-constexpr size_t SWEEP_LARGE_PER_SM = 16384;
-
-// The sweep kernel for a signal of n samples, or null for a single section's small signal.
+// The sweep kernel for a signal of n samples, or null for the lookback kernels.
 const SweepPart* sweep_pick(const iir_plan* p, size_t n) {
-    // PLR's order 2 has no such kernel (2^20 samples: 8.9 us, 8.7 on the sweep; 3e6: 22.5, 9.2)
-    if (p->kind == IIR_KIND_PLR) return n > PLR_BLOCK_MAX_N ? &p->sweeps.front() : nullptr;
-    if (n >= SWEEP_LARGE_PER_SM * static_cast<size_t>(p->sms)) return &p->sweeps.front();
-    return p->n_sections > 1 ? &p->sweeps.back() : nullptr;
+    if (n < p->sweep_min_n) return nullptr;
+    return n >= sweep_large_per_sm(p->n_sections) * static_cast<size_t>(p->sms) ? &p->sweeps.front() : &p->sweeps.back();
 }
 
 int sweep_launch(iir_plan* p, const SweepPart& s, const float* x, float* y, size_t n, cudaStream_t stream) {

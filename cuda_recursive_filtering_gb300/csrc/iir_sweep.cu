@@ -283,8 +283,11 @@ SweepLimits sweep_limits(const SectionF32& s, int N) {
                        static_cast<float>(4.0 * 0x1p-24 * (1.0 + std::sqrt(noise)))};
 }
 
-double sweep_error(const SweepFilter& f, const std::vector<float>& t, int N, bool diff) {
-    const int K = f.K, D = 2 * K, rows = 40;
+SweepTrial sweep_trial(const SweepFilter& f, const std::vector<float>& t, int N, bool diff, int rows, float offset) {
+    const int K = f.K, D = 2 * K;
+    std::vector<float> top(static_cast<size_t>(K), 0.f), off(top);  // largest outputs and weighed residuals
+    std::vector<SweepLimits> lim;
+    for (const SectionF32& s : f.secs) lim.push_back(sweep_limits(s, N));
     const float* th = t.data() + static_cast<size_t>(D) * N;
     const float* pn = t.data() + ((static_cast<size_t>(D) * N + 2 * D + 3) & ~size_t(3));
     std::vector<float> st(static_cast<size_t>(D), 0.f), e(st), next(st);
@@ -296,7 +299,7 @@ double sweep_error(const SweepFilter& f, const std::vector<float>& t, int N, boo
     double err = 0.0, ref = 0.0;
     unsigned int lcg = 12345u;
     for (int i = 0; i < rows; ++i) {
-        for (float& v : x) v = static_cast<float>(static_cast<int>((lcg = 1664525u * lcg + 1013904223u) >> 8)) * 0x1p-23f - 1.f;
+        for (float& v : x) v = static_cast<float>(static_cast<int>((lcg = 1664525u * lcg + 1013904223u) >> 8)) * 0x1p-23f - 1.f + offset;
         for (int c = 0; c < D; ++c) {
             float a[2] = {0.f, 0.f};
             for (int n = 0; n < N; ++n) a[n & 1] = std::fmaf(t[static_cast<size_t>(c) * N + n], x[n], a[n & 1]);
@@ -348,13 +351,18 @@ double sweep_error(const SweepFilter& f, const std::vector<float>& t, int N, boo
             }
             next[2 * s] = a0;
             next[2 * s + 1] = a1;
+            const float y = h[2 * s + 3], sg = sweep_sign(f.secs[static_cast<size_t>(s)].a1);
+            top[s] = std::max(top[s], std::fabs(y));
+            off[s] = std::max(off[s], std::max(std::fabs(y - a1), lim[s].wd * std::fabs((diff ? dl[s] : y - sg * h[2 * s + 2]) - a0)));
         }
         st = next;
         x2 = x[N - 2];
         x1 = x[N - 1];
     }
     const double e2 = std::sqrt(err / ref);
-    return std::isfinite(e2) ? e2 : INFINITY;
+    double worst = 0.0;
+    for (int s = 0; s < K; ++s) worst = std::max(worst, static_cast<double>(off[s]) / (static_cast<double>(lim[s].tol) * top[s]));
+    return SweepTrial{std::isfinite(e2) ? e2 : INFINITY, std::isfinite(worst) ? worst : INFINITY};
 }
 
 BatchSweepFilter bsweep_filter(const SectionF32* secs, int K, double gain, int span) {

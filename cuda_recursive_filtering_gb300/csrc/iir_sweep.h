@@ -48,8 +48,13 @@ struct SweepLimits {
     float wd, tol;
 };
 SweepLimits sweep_limits(const SectionF32& s, int N);
-// Relative error (2-norm, against 64 bits) of the schedule's float32 arithmetic on white noise, with pass B
-// in the direct form or on differences: the kernel's steps done on the host over 40 sub-rows, with its tables.
-double sweep_error(const SweepFilter& f, const std::vector<float>& tables, int N, bool diff);
+// The schedule's float32 arithmetic on white noise on an offset, with pass B in the direct form or on differences:
+// the kernel's steps done on the host over some sub-rows, with its tables. error: against 64 bits (2-norm).
+// residual: the largest one, as a fraction of its limit; from about 0.7 on in 40 sub-rows, a tile of 128 is corrected now
+// and then on any signal.
+struct SweepTrial {
+    double error, residual;
+};
+SweepTrial sweep_trial(const SweepFilter& f, const std::vector<float>& tables, int N, bool diff, int rows, float offset = 0.f);
 
 }  // namespace iirhost

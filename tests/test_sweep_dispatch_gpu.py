@@ -1,0 +1,52 @@
+"""Which kernel filters a signal: sizes on either side of the lines between the lookback kernels and the state
+sweep's two kernels, for a filter of each class (csrc/iir_host.cu: sweep_large_per_sm, sweep_pick), and the
+realization that AUTO stands for.
+
+Tolerance: the reference's gate max|err| <= 1e-4 * max|ref| (src/test_accuracy.cu:178-188), and no more than
+twice the error of the per-section lookback (IIR_GB300_TAIL=0) plus one float32 rounding of the peak.
+"""
+import numpy as np
+import pytest
+import torch
+from scipy import signal
+
+import oracle
+from cuda_recursive_filtering_gb300 import Plan
+
+pytestmark = pytest.mark.gpu
+
+SM = 152
+# decays within the small tiles; only within the large ones; and one whose white noise the sweep corrects
+FILTERS = {"fast": signal.butter(4, 0.1, output="sos"), "slow": signal.butter(4, 0.01, output="sos"),
+           "corrected": signal.cheby1(10, 1.0, 0.1, output="sos"), "eight": signal.butter(16, 0.1, output="sos")}
+LINES = {"fast": (16384 * SM,), "slow": (8192 * SM, 16384 * SM), "corrected": (16384 * SM,), "eight": (12288 * SM,)}
+
+
+@pytest.mark.parametrize("kind", sorted(FILTERS))
+def test_either_side_of_the_lines(kind, monkeypatch, cuda_device):
+    sos = FILTERS[kind]
+    plan = Plan(sos, "PH", max_n=1 << 20)
+    monkeypatch.setenv("IIR_GB300_TAIL", "0")
+    lookback = Plan(sos, "PH", max_n=1 << 20)
+    for n in [v for line in LINES[kind] for v in (line - 1, line)]:
+        x = np.random.default_rng(n).uniform(-1, 1, n).astype(np.float32)
+        xt = torch.from_numpy(x).cuda()
+        _, ref = oracle.reference_golden(sos, x)
+        peak = np.max(np.abs(ref))
+        got, general = [np.max(np.abs(p(xt).cpu().numpy().astype(np.float64) - ref)) for p in (plan, lookback)]
+        plan.check()
+        lookback.check()
+        assert got <= 1e-4 * peak and got <= 2 * general + 2.0 ** -24 * peak, (n, got / peak, general / peak)
+
+
+@pytest.mark.parametrize("order,cutoff", [(12, 0.6), (14, 0.6), (16, 0.05), (12, 0.3)])
+def test_auto_on_an_offset(order, cutoff, cuda_device):
+    """AUTO is no further off than the precision form where the filter passes an offset (mean square, a tenth
+    more for the order of the sums)."""
+    sos = signal.butter(order, cutoff, output="sos")
+    n = 300_001
+    x = (np.random.default_rng(order).uniform(-1, 1, n) + 1000.0).astype(np.float32)
+    xt = torch.from_numpy(x).cuda()
+    ref = torch.from_numpy(oracle.reference_golden(sos, x)[1]).cuda()
+    got, precise = [float((Plan(sos, k, max_n=n)(xt).double() - ref).square().mean().sqrt()) for k in ("AUTO", "TC")]
+    assert got <= 1.1 * precise, (got, precise)
