@@ -5,7 +5,7 @@
 // leave behind, 2K dot products), scan, pass B (the whole cascade once from the true states). What a
 // batch adds:
 //   * the launch's work is a list of runs: consecutive tiles of one segment, after the tile ahead of
-//     them (only its end state is computed). A block's loader
+//     them (filtered for its end state and not stored). A block's loader
 //     warp draws a run, puts its tiles and its filter's table into the block's ring of buffers, and
 //     draws the next; the filter warps take the tiles in order. The next run's record is read and the
 //     one after it drawn while a run's tiles are waited for.
@@ -30,7 +30,8 @@ struct BatchSweepGeom {
     static constexpr int T_A = 0;                             // [D][N] pass A
     static constexpr int T_H = T_A + D * N;                   // [D][2] response to (x[-2], x[-1])
     static constexpr int T_C = T_H + 2 * D;                   // [K][4] b1, b2, a1, a2, then the input gain
-    static constexpr int T_PN = T_C + 4 * K + 4;              // [BLOCKS] Phi^N
+    static constexpr int T_W = T_C + 4 * K + 4;               // [K][2] what residuals are held to (sweep_agree)
+    static constexpr int T_PN = T_W + ((2 * K + 3) & ~3);     // [BLOCKS] Phi^N
     static constexpr int T_PS = T_PN + 4 * BLOCKS;            // [BSWEEP_STEPS][BLOCKS] Phi^(SPAN 2^k)
     static constexpr int T_PL = T_PS + 4 * BSWEEP_STEPS * BLOCKS;  // [BSWEEP_NEAR][BLOCKS] Phi^(SPAN l), if not chained
     static constexpr int T_LEN = T_PL + (bsweep_chained(K) ? 0 : 4 * BSWEEP_NEAR * BLOCKS);
@@ -92,7 +93,8 @@ __device__ __forceinline__ void bsweep_respond(const float* tab, int rounds, int
 // zf[2 s + 1], s < kreal.
 template <class G, bool CAPTURE>
 __device__ __forceinline__ void bsweep_run(float* buf, const float* tab, int lane, const float (&st)[G::R][G::D],
-                                           const float (&xh)[G::R][2], int at = -1, float* zf = nullptr, int kreal = 0) {
+                                           const float (&xh)[G::R][2], float (&end)[G::R][G::D], int at = -1,
+                                           float* zf = nullptr, int kreal = 0) {
     constexpr int K = G::K, N = G::N, R = G::R, P = R / 2;
     float* line = buf + (lane << 5);
     const int l7 = lane & 7;
@@ -197,6 +199,18 @@ __device__ __forceinline__ void bsweep_run(float* buf, const float* tab, int lan
             }
         }
     }
+#pragma unroll
+    for (int p = 0; p < P; ++p)
+#pragma unroll
+        for (int s = 0; s < K; ++s) {
+            float ya, yb, za, zb;
+            unpack2(h[p][s + 1][1], ya, yb);
+            unpack2(h[p][s + 1][0], za, zb);
+            end[2 * p][2 * s] = fmaf(-sg[s], za, ya);
+            end[2 * p + 1][2 * s] = fmaf(-sg[s], zb, yb);
+            end[2 * p][2 * s + 1] = ya;
+            end[2 * p + 1][2 * s + 1] = yb;
+        }
 }
 // The sections' states after sample m of the tile, to zf[2 s], zf[2 s + 1], s < kreal, ahead of pass B: its
 // steps once more from the start of m's sub-row, by every lane alike (bound by their latency: at most N
@@ -257,6 +271,75 @@ __device__ __forceinline__ void bsweep_state(const float* buf, const float* tab,
     __syncwarp();  // every lane has read the samples
 }
 
+// The same after the states were found to lack g: the response to g at sample m is added to zf, by lane `by`.
+template <class G>
+__device__ __forceinline__ void bsweep_state_fix(const float* tab, int lane, int m, const float (&g)[G::R][G::D], float* zf,
+                                                 int kreal, int by) {
+    constexpr int K = G::K, N = G::N, R = G::R, D = G::D;
+    const int row = m / G::SPAN, sub = (m % G::SPAN) / N;
+    float S[D], y2[K], y1[K];
+#pragma unroll
+    for (int c = 0; c < D; ++c) {
+        S[c] = 0.f;
+#pragma unroll
+        for (int i = 0; i < R; ++i)
+            if (i == sub) S[c] = g[i][c];
+        S[c] = __shfl_sync(FULL_MASK, S[c], row);
+    }
+#pragma unroll
+    for (int s = 0; s < K; ++s) {
+        y2[s] = sweep_sign(tab[G::T_C + 4 * s + 2]) * (S[2 * s + 1] - S[2 * s]);
+        y1[s] = S[2 * s + 1];
+    }
+#pragma unroll 1
+    for (int n = sub * N; n <= m % G::SPAN; ++n) {
+        float w = 0.f, g2 = 0.f, g1 = 0.f;
+#pragma unroll
+        for (int s = 0; s < K; ++s) {
+            const float4 c = *reinterpret_cast<const float4*>(tab + G::T_C + 4 * s);
+            w = fmaf(c.y, g2, fmaf(c.x, g1, w));
+            g2 = y2[s];
+            g1 = y1[s];
+            w = fmaf(c.z, g1, fmaf(c.w, g2, w));
+            y2[s] = g1;
+            y1[s] = w;
+        }
+    }
+#pragma unroll
+    for (int s = 0; s < K; ++s)
+        if (lane == by && s < kreal) {
+            zf[2 * s] += y2[s];
+            zf[2 * s + 1] += y1[s];
+        }
+}
+
+// The two steps of a correction (iir_sweep.cuh, sweep_lack and sweep_apply).
+template <class G>
+__device__ __noinline__ void bsweep_lack(const float* tab, int rounds, int lane, const float (&r)[G::R][G::D],
+                                         float (&g)[G::D], float (&last)[G::D]) {
+    float f[G::D], none[G::D] = {};
+    sweep_join<G>(tab, r, f);
+    bsweep_scan<G, false>(tab, rounds, lane, f, none, g, last);
+}
+// before: what the tile's incoming state lacks, or null; zf: the segment's states, if its last sample m is here, or null.
+template <class G>
+__device__ __noinline__ void bsweep_apply(float* buf, const float* tab, int rounds, int lane, const float (&r)[G::R][G::D],
+                                          const float (&g0)[G::D], const float* before, int m, float* zf, int kreal, int by) {
+    float g[G::R][G::D];
+#pragma unroll
+    for (int c = 0; c < G::D; ++c) g[0][c] = g0[c];
+    if (before) {
+        float X[G::D];
+#pragma unroll
+        for (int c = 0; c < G::D; ++c) X[c] = before[c];
+        bsweep_respond<G>(tab, rounds, lane, X, g[0]);
+    }
+#pragma unroll
+    for (int j = 1; j < G::R; ++j) tri_mad<G::K>(tab + G::T_PN, g[j - 1], r[j - 1], g[j]);
+    sweep_respond<G>(buf, [&](int s) { return *reinterpret_cast<const float4*>(tab + G::T_C + 4 * s); }, lane, g);
+    if (zf) bsweep_state_fix<G>(tab, lane, m, g, zf, kreal, by);
+}
+
 __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, int x, int y, int z,
                                             unsigned long long* bar) {
     asm volatile(
@@ -290,9 +373,11 @@ struct BatchSweepAux {
     BatchRun runs[RUNS];                     // the last runs begun
     unsigned long long full[NB], empty[NB];
     float ends[RING][2 * IIR_MAX_SECTIONS];  // items' end states
+    float fix[RING][2 * IIR_MAX_SECTIONS];   // what they lack, where it matters
     unsigned int item_run[RING];             // the item's run ...
     unsigned int item[RING];                 // ... and tile, BSWEEP_WARM (only its end state is wanted), BSWEEP_FIRST
     volatile unsigned int ready[RING];       // i + 1 once item i's end state is in `ends`
+    volatile unsigned int checked[RING];     // 2 (i + 1) once it has been checked, plus 1 if `fix` is to be added
     volatile unsigned int issued[NB];        // items put into the buffer so far
     unsigned int tag[NB];                    // the filter whose table the buffer holds (copiers)
     volatile unsigned int copied[BSWEEP_COPIERS];  // 1 + the last item that the copier has issued
@@ -437,12 +522,12 @@ __device__ __forceinline__ void bsweep_copier(const IirBatchSweepParams& p, Batc
 }
 
 // One item: the tile in `buf`, whose load has been issued. wait_tile(): it is there; wait_ready(): the item
-// before has its end state. Returns false when a wait ran out. CAPTURE: how the segment's states are found
+// before has its end state; wait_checked(): and it has been checked. Returns false when a wait ran out. CAPTURE: how the segment's states are found
 // (bsweep_state).
-template <class G, int NB, bool CAPTURE, class Tile, class Ready>
+template <class G, int NB, bool CAPTURE, class Tile, class Ready, class Checked>
 __device__ __forceinline__ bool bsweep_item(const IirBatchSweepParams& p, BatchSweepAux<NB>& aux, float* buf,
                                             const float* tab, const BatchRun& run, unsigned i, unsigned rec,
-                                            Tile&& wait_tile, Ready&& wait_ready) {
+                                            Tile&& wait_tile, Ready&& wait_ready, Checked&& wait_checked) {
     constexpr int SPAN = G::SPAN, TILE = G::TILE, R = G::R, K = G::K, D = G::D;
     using Aux = BatchSweepAux<NB>;
     const int lane = threadIdx.x & 31;
@@ -557,23 +642,68 @@ __device__ __forceinline__ bool bsweep_item(const IirBatchSweepParams& p, BatchS
             }
         }
     }
-    if (warm) {
-        fence_proxy_async_smem();  // generic accesses of the buffer before the async ones to come
-        return true;
-    }
 #pragma unroll
     for (int j = 1; j < R; ++j) tri_mad<K>(tab + G::T_PN, st[j - 1], e[j - 1], st[j]);
     __syncwarp();  // every lane has read its neighbour's last samples
     const int m = have - 1;  // the segment's last sample, if it is here
     const bool ends = run.zf && left <= TILE;
+    float end[R][D];
     if constexpr (CAPTURE) {
         if (ends)
-            bsweep_run<G, true>(buf, tab, lane, st, xh, m >= 0 && m / SPAN == lane ? m % SPAN : -1, run.zf + 2, run.K);
+            bsweep_run<G, true>(buf, tab, lane, st, xh, end, m >= 0 && m / SPAN == lane ? m % SPAN : -1, run.zf + 2, run.K);
         else
-            bsweep_run<G, false>(buf, tab, lane, st, xh);
+            bsweep_run<G, false>(buf, tab, lane, st, xh, end);
     } else {
         if (ends && m >= 0) bsweep_state<G>(buf, tab, lane, m, st, xh, run.zf + 2, run.K);
-        bsweep_run<G, false>(buf, tab, lane, st, xh);
+        bsweep_run<G, false>(buf, tab, lane, st, xh, end);
+    }
+    {
+        // the states checked and corrected (iir_sweep.cuh, sweep_agree)
+        float r[R][D];
+        const bool off = !sweep_agree<G, (K > 4)>([&](int s) { return *reinterpret_cast<const float2*>(tab + G::T_W + 2 * s); }, lane,
+                                         have, end, st, aux.ends[i % Aux::RING], r);
+        float gs[D];
+#pragma unroll
+        for (int c = 0; c < D; ++c) gs[c] = 0.f;
+        if (off) {
+            float rr[R][D], g0[D], last[D];  // (copies: their addresses go to a call, the others stay in registers)
+#pragma unroll
+            for (int q = 0; q < R; ++q)
+#pragma unroll
+                for (int c = 0; c < D; ++c) rr[q][c] = r[q][c];
+            bsweep_lack<G>(tab, run.rounds, lane, rr, g0, last);
+#pragma unroll
+            for (int c = 0; c < D; ++c) gs[c] = g0[c];
+            if (lane == 31) {
+#pragma unroll
+                for (int c = 0; c < D; c += 2)
+                    *reinterpret_cast<float2*>(&aux.fix[i % Aux::RING][c]) = make_float2(last[c], last[c + 1]);
+            }
+        }
+        if (lane == 31) {
+            __threadfence_block();
+            aux.checked[i % Aux::RING] = 2u * (i + 1u) + (off ? 1u : 0u);
+        }
+        if (warm) {
+            fence_proxy_async_smem();  // generic accesses of the buffer before the async ones to come
+            return true;
+        }
+        bool before = false;  // the state before the tile lacked something
+        if (!first) {
+            if (!wait_checked()) return false;
+            before = (aux.checked[(i - 1u) % Aux::RING] & 1u) != 0u;
+        }
+        if (off || before) {
+            float rr[R][D], g0[D];
+#pragma unroll
+            for (int c = 0; c < D; ++c) {
+                g0[c] = gs[c];
+#pragma unroll
+                for (int q = 0; q < R; ++q) rr[q][c] = off ? r[q][c] : 0.f;
+            }
+            bsweep_apply<G>(buf, tab, run.rounds, lane, rr, g0, before ? aux.fix[(i - 1u) % Aux::RING] : nullptr, m,
+                            ends && m >= 0 ? run.zf + 2 : nullptr, run.K, CAPTURE ? m / SPAN : 0);
+        }
     }
     if (ends) {
         __syncwarp();
@@ -634,7 +764,7 @@ __global__ void __launch_bounds__((W + 1 + BSWEEP_COPIERS) * 32) iir_batch_sweep
             aux.issued[b] = 0u;
             aux.tag[b] = 0xffffffffu;
         }
-        for (unsigned i = 0; i < Aux::RING; ++i) aux.ready[i] = 0u;
+        for (unsigned i = 0; i < Aux::RING; ++i) aux.ready[i] = aux.checked[i] = 0u;
         for (int c = 0; c < BSWEEP_COPIERS; ++c) aux.copied[c] = 0u;
         aux.next = 0u;
         aux.recorded = 0u;
@@ -673,11 +803,16 @@ __global__ void __launch_bounds__((W + 1 + BSWEEP_COPIERS) * 32) iir_batch_sweep
                 __threadfence_block();
                 return !__any_sync(FULL_MASK, !got);
             };
+            auto checked = [&] {
+                const bool got = bsweep_wait(aux, p, [&] { return aux.checked[(i - 1u) % Aux::RING] >> 1 == i; });
+                __threadfence_block();
+                return !__any_sync(FULL_MASK, !got);
+            };
             bool ok = false;
             switch (run.K) {
 #define IIR_BSWEEP_CASE(KP)                                                                                  \
     if constexpr (KP <= MAXK)                                                                                 \
-        ok = bsweep_item<BatchSweepGeom<KP, SPAN>, NB, (MAXK > 4)>(p, aux, buf, tab, run, i, rec, tile, ready);  \
+        ok = bsweep_item<BatchSweepGeom<KP, SPAN>, NB, (MAXK > 4)>(p, aux, buf, tab, run, i, rec, tile, ready, checked);  \
     break;
                 case 1: IIR_BSWEEP_CASE(1)
                 case 2: IIR_BSWEEP_CASE(2)

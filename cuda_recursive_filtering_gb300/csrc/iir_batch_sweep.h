@@ -28,7 +28,7 @@ __host__ __device__ constexpr int bsweep_subrow(int K, int span) { return span =
 __host__ __device__ constexpr bool bsweep_chained(int K) { return K > 4; }
 
 __host__ __device__ constexpr int bsweep_table_floats(int K, int span) {  // BatchSweepGeom::T_LEN
-    return 2 * K * bsweep_subrow(K, span) + 8 * K + 4 +
+    return 2 * K * bsweep_subrow(K, span) + 8 * K + 4 + ((2 * K + 3) & ~3) +
            4 * (1 + BSWEEP_STEPS + (bsweep_chained(K) ? 0 : BSWEEP_NEAR)) * (K * (K + 1) / 2);
 }
 // The largest table of up to K sections.

@@ -411,8 +411,8 @@ BatchSweepFilter bsweep_filter(const SectionF32* secs, int K, double gain, int s
     if (k > 5) return out;
     out.rounds = k;
     out.fast = true;
-    const size_t t_h = static_cast<size_t>(D) * N, t_c = t_h + 2 * D, t_pn = t_c + 4 * KP + 4,
-                 t_ps = t_pn + 4 * static_cast<size_t>(blocks);
+    const size_t t_h = static_cast<size_t>(D) * N, t_c = t_h + 2 * D, t_w = t_c + 4 * KP + 4,
+                 t_pn = t_w + static_cast<size_t>((2 * KP + 3) & ~3), t_ps = t_pn + 4 * static_cast<size_t>(blocks);
     std::vector<float>& t = out.table;
     t.assign(static_cast<size_t>(bsweep_table_floats(KP, span)), 0.f);
     put_dots(t, f, N, t_h);
@@ -422,6 +422,10 @@ BatchSweepFilter bsweep_filter(const SectionF32* secs, int K, double gain, int s
         c[1] = padded[static_cast<size_t>(s)].b2;
         c[2] = padded[static_cast<size_t>(s)].a1;
         c[3] = padded[static_cast<size_t>(s)].a2;
+        // (a section that passes its input on is held to nothing of its own)
+        const SweepLimits lim = s < K ? sweep_limits(padded[static_cast<size_t>(s)], N) : SweepLimits{0.f, 1.f};
+        t[t_w + 2 * static_cast<size_t>(s)] = lim.wd;
+        t[t_w + 2 * static_cast<size_t>(s) + 1] = lim.tol;
     }
     t[t_c + 4 * static_cast<size_t>(KP)] = static_cast<float>(gain);
     auto put = [&](size_t at, const Mat& m) {

@@ -214,9 +214,8 @@ __device__ __forceinline__ void sweep_scan(const float* tab, int rounds, int lan
     constexpr int D = G::D;
 #pragma unroll
     for (int c = 0; c < D; ++c) last[c] = f[c];
-#pragma unroll
-    for (int k = 0; (1 << k) < SWEEP_LANES; ++k) {
-        if (k >= rounds) break;
+#pragma unroll 1
+    for (int k = 0; k < rounds; ++k) {
         float o[D];
 #pragma unroll
         for (int c = 0; c < D; ++c) {
@@ -239,8 +238,10 @@ __device__ __forceinline__ void sweep_scan(const float* tab, int rounds, int lan
 // that do not depend on one another) and more code; measured with 1 / 2 / 4: order 2 at 2^23 samples
 // 15.4 / 15.0 / 14.7 us, order 4 16.9 / 16.6 / 16.2; at 2^27 order 8 174.7 / 175.0 / 184.7, order 10
 // 237.5 / 234.3 / 230.6, order 12 259 / 267 / 273, order 16 330.7 / 329.8 / 330.7 (on differences 376 / 367
-// / 380).
-__host__ __device__ constexpr int sweep_step_granules(int K) { return K <= 2 || K == 5 ? 4 : K == 8 ? 2 : 1; }
+// / 380). With the states checked, 1 / 2: order 16 at 2^25 96.8 / 100.1, on differences at 2^27 393 / 388.
+__host__ __device__ constexpr int sweep_step_granules(int K, bool diff) {
+    return K <= 2 || K == 5 ? 4 : K == 8 && diff ? 2 : 1;
+}
 
 // A section's state is carried as (y[-1] - sg y[-2], y[-1]), sg = 1 for poles on the right of the circle and -1 on
 // the left: two outputs near a slow pole differ by little (near a pole at -1, from the negative), and it is that
@@ -302,8 +303,8 @@ __device__ __forceinline__ void sweep_run_ph(float* buf, const SweepSection* sec
         }
     float* row = buf + (lane << 5);
     const int l7 = lane & 7;
-    constexpr int GB = sweep_step_granules(K), S = 4 * GB;  // granules and samples per step
-#pragma unroll (GB == 1 ? 2 : 1)
+    constexpr int GB = sweep_step_granules(K, DIFF), S = 4 * GB;  // granules and samples per step
+#pragma unroll 1
     for (int j = 0; j < N / 4; j += GB) {
         float4 x[GB][R];
         float* at[GB];
@@ -404,52 +405,64 @@ __device__ __forceinline__ void sweep_run_ph(float* buf, const SweepSection* sec
 // the stop band: 2.0e-3 without, 2.7e-5 with (section by section, iir_ph.cuh: 3.1e-5).
 
 // Residuals r of the lane's sub-rows (r[i]: at its end), from pass B's end states, the states st that it started
-// from and the tile's end state `last`. True if all are within a section's rounding: tol = 4 x 2^-24 x (1 + the
-// noise gain of 1 / A over a sub-row) of its largest output in the tile, a difference weighed by what it grows
-// to. (With 6 for 4, up to twice the lookback's error gets by: a tone in the stop band of cheby1(4, 1, 0.02); with
-// 3, white noise is corrected by half as many filters more.)
-template <class G>
-__device__ __forceinline__ bool sweep_agree(const SweepSection* sec, int lane, const float (&end)[G::R][G::D],
+// from and the tile's end state `last`. True if they are within the sections' rounding: tol = 4 x 2^-24 x (1 + the
+// noise gain of 1 / A over a sub-row) of a section's largest output in the tile, a difference weighed by what it
+// grows to. (With 6 for 4, up to twice the lookback's error gets by: a tone in the stop band of cheby1(4, 1, 0.02);
+// with 3, white noise is corrected by half as many filters more. Judging a lane by its last sub-row alone is no
+// faster, and lets three times the lookback's error by: cheby1(6, 1, 0.04).) limits(s): a section's (wd, tol).
+// The first, the middle and the last section speak for all (over 528 designs and signals, the sections in scipy's
+// order, reversed, or with zeros and poles paired at random; the last alone lets five times by). PADDED: the last one
+// may pass its input on. Sub-rows that end past the tile's first `have` samples hold nothing.
+template <class G, bool PADDED = false, class Limits>
+__device__ __forceinline__ bool sweep_agree(Limits&& limits, int lane, int have, const float (&end)[G::R][G::D],
                                             const float (&st)[G::R][G::D], const float* last, float (&r)[G::R][G::D]) {
     constexpr int R = G::R, K = G::K, D = G::D;
+    const bool whole = have >= G::TILE;
 #pragma unroll
     for (int c = 0; c < D; ++c) {
         float next = __shfl_down_sync(FULL_MASK, st[0][c], 1);
         if (lane == 31) next = last[c];
 #pragma unroll
-        for (int i = 0; i < R; ++i) r[i][c] = end[i][c] - (i + 1 < R ? st[i + 1 < R ? i + 1 : 0][c] : next);
+        for (int i = 0; i < R; ++i) {
+            r[i][c] = end[i][c] - (i + 1 < R ? st[i + 1 < R ? i + 1 : 0][c] : next);
+            if (!whole && lane * G::SPAN + (i + 1) * G::N > have) r[i][c] = 0.f;
+        }
     }
     bool ok = true;
 #pragma unroll
     for (int s = 0; s < K; ++s) {
-        float top = 0.f, off = 0.f;
+        if (s != 0 && s != K / 2 && s != K - 1 && !(PADDED && s == K - 2)) continue;
+        const float2 lim = limits(s);
+        float top = 0.f, off = 0.f, dif = 0.f;
 #pragma unroll
         for (int i = 0; i < R; ++i) {
-            top = fmaxf(top, fabsf(end[i][2 * s + 1]));
-            off = fmaxf(off, fmaxf(fabsf(r[i][2 * s + 1]), sec[s].wd * fabsf(r[i][2 * s])));
+            if (whole || lane * G::SPAN + (i + 1) * G::N <= have) top = fmaxf(top, fabsf(end[i][2 * s + 1]));
+            off = fmaxf(off, fabsf(r[i][2 * s + 1]));
+            dif = fmaxf(dif, fabsf(r[i][2 * s]));
         }
         top = __uint_as_float(__reduce_max_sync(FULL_MASK, __float_as_uint(top)));
-        ok = ok && off <= sec[s].tol * top;
+        ok = ok && fmaxf(off, lim.x * dif) <= lim.y * top;
     }
     return __all_sync(FULL_MASK, ok);
 }
 
-// Adds the cascade's response to the states g before the lane's sub-rows to the outputs in the buffer.
-template <class G>
-__device__ __forceinline__ void sweep_respond(float* buf, const SweepSection* sec, int lane,
-                                              const float (&g)[G::R][G::D]) {
+// Adds the cascade's response to the states g before the lane's sub-rows to the outputs in the buffer. taps(s): a
+// section's (b1, b2, a1, a2).
+template <class G, class Taps>
+__device__ __forceinline__ void sweep_respond(float* buf, Taps&& taps, int lane, const float (&g)[G::R][G::D]) {
     constexpr int K = G::K, N = G::N, R = G::R, P = R / 2;
     f32x2 b1[K], b2[K], a1[K], a2[K], h[P][K][2];  // h: the sections' last two outputs
 #pragma unroll
     for (int s = 0; s < K; ++s) {
-        b1[s] = pack2(sec[s].b1, sec[s].b1);
-        b2[s] = pack2(sec[s].b2, sec[s].b2);
-        a1[s] = pack2(sec[s].a1, sec[s].a1);
-        a2[s] = pack2(sec[s].a2, sec[s].a2);
+        const float4 c = taps(s);
+        const float sign = sweep_sign(c.z);
+        b1[s] = pack2(c.x, c.x);
+        b2[s] = pack2(c.y, c.y);
+        a1[s] = pack2(c.z, c.z);
+        a2[s] = pack2(c.w, c.w);
 #pragma unroll
         for (int p = 0; p < P; ++p) {
             const float *u = g[2 * p] + 2 * s, *v = g[2 * p + 1] + 2 * s;
-            const float sign = sweep_sign(sec[s].a1);
             h[p][s][0] = pack2(sign * (u[1] - u[0]), sign * (v[1] - v[0]));
             h[p][s][1] = pack2(u[1], v[1]);
         }
@@ -458,7 +471,6 @@ __device__ __forceinline__ void sweep_respond(float* buf, const SweepSection* se
     const int l7 = lane & 7;
 #pragma unroll 1
     for (int j = 0; j < N / 4; ++j) {
-        float* at = row + sub_granule_at<N>(0, j, l7);
 #pragma unroll
         for (int p = 0; p < P; ++p) {
             float y[2][4];
@@ -478,12 +490,55 @@ __device__ __forceinline__ void sweep_respond(float* buf, const SweepSection* se
             }
 #pragma unroll
             for (int i = 0; i < 2; ++i) {
-                float4* q = reinterpret_cast<float4*>(at + (2 * p + i) * (N / 32) * 1024);
+                float4* q = reinterpret_cast<float4*>(row + sub_granule_at<N>(2 * p + i, j, l7));
                 const float4 x = *q;
                 *q = make_float4(x.x + y[i][0], x.y + y[i][1], x.z + y[i][2], x.w + y[i][3]);
             }
         }
     }
+}
+
+// The two steps of a correction, and the staging of tiles off the 16-byte grid, are functions of their own: few tiles
+// need them, and the code that every tile goes through then stays in the instruction cache (order 8 at 2^27: 214 us
+// with the corrections inline, 204 as calls; and 189 with the lane scan and pass B as loops that are not unrolled).
+// g: what the state before each lane lacks, from rest before the tile; last: and the one after the tile.
+template <class G>
+__device__ __noinline__ void sweep_lack(const float* tab, int rounds, int lane, const float (&r)[G::R][G::D],
+                                        float (&g)[G::D], float (&last)[G::D]) {
+    float f[G::D];
+    sweep_join<G>(tab, r, f);
+    sweep_scan<G>(tab, rounds, lane, f, g, last);
+}
+// Corrects the tile's outputs, g0 before the lane.
+template <class G>
+__device__ __noinline__ void sweep_apply(float* buf, const float* tab, const SweepSection* sec, int lane,
+                                         const float (&r)[G::R][G::D], const float (&g0)[G::D]) {
+    float g[G::R][G::D];
+#pragma unroll
+    for (int c = 0; c < G::D; ++c) g[0][c] = g0[c];
+#pragma unroll
+    for (int j = 1; j < G::R; ++j) tri_mad<G::K>(tab + G::T_PN, g[j - 1], r[j - 1], g[j]);
+    sweep_respond<G>(buf, [&](int s) { return make_float4(sec[s].b1, sec[s].b2, sec[s].a1, sec[s].a2); }, lane, g);
+}
+
+// A tile sample by sample, samples past the signal's end zero, and back.
+template <class G>
+__device__ __noinline__ void sweep_stage(float* buf, const float* x, long long base, long long n, int lane) {
+#pragma unroll 8
+    for (int j = lane; j < G::TILE; j += 32) {
+        const bool have = base + j < n;
+        cp_async4(buf + tile_at(j / G::SPAN, j % G::SPAN), have ? x + base + j : x, have ? 4 : 0);
+    }
+    cp_async_commit();
+    cp_async_wait<0>();
+    __syncwarp();
+}
+template <class G>
+__device__ __noinline__ void sweep_unstage(const float* buf, float* y, long long base, long long n, int lane) {
+    __syncwarp();
+#pragma unroll 8
+    for (int j = lane; j < G::TILE; j += 32)
+        if (base + j < n) y[base + j] = buf[tile_at(j / G::SPAN, j % G::SPAN)];
 }
 
 // ------------------------------------------------------------------------------------
@@ -654,14 +709,7 @@ __device__ __forceinline__ void sweep_tiles(const IirSweepParams& p, unsigned ch
                     __syncwarp();
                 }
             } else {
-#pragma unroll 8
-                for (int j = lane; j < G::TILE; j += 32) {
-                    const bool have = base + j < p.n;
-                    cp_async4(buf + tile_at(j / SPAN, j % SPAN), have ? p.x + base + j : p.x, have ? 4 : 0);
-                }
-                cp_async_commit();
-                cp_async_wait<0>();
-                __syncwarp();
+                sweep_stage<G>(buf, p.x, base, p.n, lane);
             }
             float e[R][D], st[R][D], xh[R][2];
             sweep_ends<G>(buf, tab, lane, g2, g1, e, xh);
@@ -699,14 +747,22 @@ __device__ __forceinline__ void sweep_tiles(const IirSweepParams& p, unsigned ch
             float end[R][D];
             run(buf, lane, st, xh, end);
             {
-                float r[R][D], g[R][D], last[D];
-                const bool off = !sweep_agree<G>(p.sec, lane, end, st, aux.ends[i % SWEEP_RING], r);
+                float r[R][D], last[D];
+                // (past the signal's end there are zeros)
+                const bool off = !sweep_agree<G>([&](int s) { return make_float2(p.sec[s].wd, p.sec[s].tol); }, lane, G::TILE,
+                                                 end, st, aux.ends[i % SWEEP_RING], r);
+                float gs[D];
 #pragma unroll
-                for (int c = 0; c < D; ++c) g[0][c] = 0.f;
+                for (int c = 0; c < D; ++c) gs[c] = 0.f;
                 if (off) {
-                    float f[D];
-                    sweep_join<G>(tab, r, f);
-                    sweep_scan<G>(tab, p.rounds, lane, f, g[0], last);
+                    float rr[R][D], g0[D];  // (copies: their addresses go to a call, the others stay in registers)
+#pragma unroll
+                    for (int q = 0; q < R; ++q)
+#pragma unroll
+                        for (int c = 0; c < D; ++c) rr[q][c] = r[q][c];
+                    sweep_lack<G>(tab, p.rounds, lane, rr, g0, last);
+#pragma unroll
+                    for (int c = 0; c < D; ++c) gs[c] = g0[c];
                     if (lane == 31) {
 #pragma unroll
                         for (int c = 0; c < D; c += 2)
@@ -724,25 +780,21 @@ __device__ __forceinline__ void sweep_tiles(const IirSweepParams& p, unsigned ch
                     __threadfence_block();
                     before = (aux.checked[(i - 1u) % SWEEP_RING] & 1u) != 0u;
                 }
-                if (before && lane < p.lanes) {
-                    float X[D];
-#pragma unroll
-                    for (int c = 0; c < D; c += 2) {
-                        const float2 v = *reinterpret_cast<const float2*>(&aux.fix[(i - 1u) % SWEEP_RING][c]);
-                        X[c] = v.x;
-                        X[c + 1] = v.y;
-                    }
-                    tri_mad<K>(tab + G::T_PL + 4 * lane * G::ROW, X, g[0], g[0]);
-                }
                 if (!warm && (off || before)) {
+                    float rr[R][D], g0[D];
 #pragma unroll
-                    for (int j = 1; j < R; ++j) {
-                        if (!off)
+                    for (int c = 0; c < D; ++c) {
+                        g0[c] = gs[c];
 #pragma unroll
-                            for (int c = 0; c < D; ++c) r[j - 1][c] = 0.f;
-                        tri_mad<K>(tab + G::T_PN, g[j - 1], r[j - 1], g[j]);
+                        for (int q = 0; q < R; ++q) rr[q][c] = off ? r[q][c] : 0.f;
                     }
-                    sweep_respond<G>(buf, p.sec, lane, g);
+                    if (before && lane < p.lanes) {
+                        float X[D];
+#pragma unroll
+                        for (int c = 0; c < D; ++c) X[c] = aux.fix[(i - 1u) % SWEEP_RING][c];
+                        tri_mad<K>(tab + G::T_PL + 4 * lane * G::ROW, X, g0, g0);
+                    }
+                    sweep_apply<G>(buf, tab, p.sec, lane, rr, g0);
                 }
             }
             if (p.use_tma) {
@@ -757,10 +809,7 @@ __device__ __forceinline__ void sweep_tiles(const IirSweepParams& p, unsigned ch
                 if (!warm && part >= 0)
                     for (int j = lane; j < rest; j += 32) p.y[rows * SPAN + j] = buf[tile_at(part, j)];
             } else if (!warm) {
-                __syncwarp();
-#pragma unroll 8
-                for (int j = lane; j < G::TILE; j += 32)
-                    if (base + j < p.n) p.y[base + j] = buf[tile_at(j / SPAN, j % SPAN)];
+                sweep_unstage<G>(buf, p.y, base, p.n, lane);
             }
             __syncwarp();
             if (lane == 0) {

@@ -125,3 +125,47 @@ def test_poles_near_minus_one(cutoff, kernel, order, monkeypatch, cuda_device):
     for p in plans:
         p.check()
     assert got <= 1.1 * lookback, (got, lookback)
+
+
+BATCH_CASES = [("cheby1", 4, 0.1, "low", "stop"), ("butter", 8, 0.1, "low", "stop"), ("cheby1", 10, 0.1, "low", "stop"),
+               ("butter", 14, 0.2, "low", "stop"), ("cheby1", 16, 0.5, "low", "stop"), ("butter", 4, 0.8, "high", "offset")]
+
+
+@pytest.mark.parametrize("lens", ([60001, 8192, 4097, 100], [700, 33, 512, 1023] * 8), ids=("large_tiles", "small_tiles"))
+@pytest.mark.parametrize("case", BATCH_CASES, ids=lambda c: "-".join(map(str, c)))
+def test_batched_state_sweep(case, lens, monkeypatch, cuda_device):
+    """Batched segments, each in two parts with its state carried over, off the 16-byte grid; the states out
+    are held to the lookback's as the outputs are."""
+    from cuda_recursive_filtering_gb300 import Batch
+    sos = design(*case[:4]).astype(np.float32)
+    rng = np.random.default_rng(len(lens))
+    off = np.concatenate([[1], 1 + np.cumsum([n + int(rng.integers(0, 4)) for n in lens])])
+    x = np.zeros(int(off[-1]) + 4, np.float32)
+    for i, n in enumerate(lens):
+        x[off[i]:off[i] + n] = coloured(n, case[4], seed=i)
+    xt = torch.from_numpy(x).cuda()
+    cut = [int(rng.integers(1, n)) for n in lens]
+
+    def run():
+        batch = Batch([sos], max_segments=64)
+        yt = torch.zeros_like(xt)
+        mid = torch.zeros(len(lens), batch.state_size(0), device="cuda")
+        end = torch.zeros_like(mid)
+        o = off
+        batch([(xt[o[i]:o[i] + c], yt[o[i]:o[i] + c], 0, None, mid[i]) for i, c in enumerate(cut)])
+        batch([(xt[o[i] + c:o[i] + n], yt[o[i] + c:o[i] + n], 0, mid[i], end[i]) for i, (c, n) in enumerate(zip(cut, lens))])
+        batch.check()
+        return yt.cpu().numpy().astype(np.float64), end.cpu().numpy().astype(np.float64)
+
+    y, z = run()
+    monkeypatch.setenv("IIR_GB300_TAIL", "0")
+    yl, zl = run()
+    for i, n in enumerate(lens):
+        _, ref = oracle.reference_golden(sos, x[off[i]:off[i] + n])
+        peak = np.max(np.abs(ref))
+        got, lookback = [np.max(np.abs(v[off[i]:off[i] + n] - ref)) for v in (y, yl)]
+        assert got <= 1e-4 * peak, (i, n, got / peak, lookback / peak)
+        if n > 4096:  # (over a few hundred samples the largest error is a matter of chance)
+            assert got <= 2 * lookback + 2.0 ** -24 * peak, (i, n, got / peak, lookback / peak)
+        scale = np.max(np.abs(zl[i]))
+        assert np.max(np.abs(z[i] - zl[i])) <= 1e-4 * scale, (i, n)
