@@ -4,8 +4,8 @@
 // cascade (any number of sections up to IIR_MAX_SECTIONS), an optional state in (zi) and an
 // optional state out (zf). Two kernels share a call's segments:
 //   * the state sweep (iir_batch_sweep.cuh) takes every segment whose filter decays within a tile;
-//   * the lookback kernel below takes the others, and all of them when a fault is injected or the
-//     environment asks for its schedules. Where both have segments they run side by side.
+//   * the lookback kernel below takes the others, and all of them when the sweep would be small beside it, a
+//     fault is injected or the environment asks for its schedules. Where both have segments they run side by side.
 //
 // Lookback kernel: the launch's chunks are the concatenation of every segment's
 // chunks; that list is the launch's work queue. A persistent grid (every block resident: the
@@ -534,7 +534,6 @@ struct ShapeData {
     bool ready = false;    // tables and filters on the device
     bool measured = false;  // footprint and residency known
     bool tails = false;     // the filters carry their tail pieces
-    bool all = false;       // every filter's tables, not the slow ones' only
     IirSection* d_secs = nullptr;
     float4* d_tables = nullptr;
     IirBatchFilter* d_filters = nullptr;
@@ -746,11 +745,10 @@ int batch_tail_tables(iir_batch* b) {
 }
 
 // Builds shape k's lane tables and filter records (once) and its occupancy.
-// (all: of every filter; else of those that the sweep does not take).
-int shape_prepare(iir_batch* b, int k, bool all) {
+int shape_prepare(iir_batch* b, int k) {
     ShapeData& d = b->shape_data[static_cast<size_t>(k)];
     const bool tails = std::getenv("IIR_GB300_BATCH_TAIL_CHUNKS") != nullptr;
-    if (d.ready && (d.tails || !tails) && (d.all || !all)) return IIR_OK;
+    if (d.ready && (d.tails || !tails)) return IIR_OK;
     if (tails && !b->d_phi)
         if (const int r = batch_tail_tables(b)) return r;
     if (d.ready) {  // again, with more of them: bound launches (and graphs of them) keep the earlier ones
@@ -759,19 +757,11 @@ int shape_prepare(iir_batch* b, int k, bool all) {
         d = ShapeData{};
     }
     d.tails = tails;
-    d.all = all;
     const ShapeDef& sd = shapes()[static_cast<size_t>(k)];
     std::vector<float4> tabs(b->sec32.size() * IIR_BT_STRIDE, make_float4(0, 0, 0, 0));
     std::vector<IirSection> secs(b->sec32.size());
     std::vector<float4> full(IIR_TAB_STRIDE);
-    std::vector<char> wanted(b->sec32.size(), all ? 1 : 0);
-    for (size_t f = 0; f < b->filters.size() && !all; ++f) {
-        bool fast = true;
-        for (const SweepData& v : b->sweep) fast = fast && (!v.ready || v.filters[f].fast);
-        std::fill_n(wanted.begin() + b->filters[f].sec0, b->filters[f].n_sections, fast ? 0 : 1);
-    }
     for (size_t s = 0; s < b->sec32.size(); ++s) {
-        if (!wanted[s]) continue;
         IirSection& q = secs[s];
         const int st = precompute_section(b->sec32[s], IIR_KIND_PH, sd.rows, sd.n, q, full.data());
         if (st) return st;
@@ -868,7 +858,6 @@ size_t sweep_tiles(const iir_segment& s, int tile) {
 // How a call's segments are filtered: those on the state sweep, with the tile size and the length and
 // number of their runs, and those on the lookback kernel.
 struct Schedule {
-    bool sweep = false;  // some may be swept
     int v = 0;
     size_t len = 0;      // tiles per run
     size_t longest = 0;  // of the runs there are
@@ -876,6 +865,9 @@ struct Schedule {
     std::vector<int> swept;
     std::vector<iir_segment> rest;
 };
+
+// Samples per SM from which segments are swept while others are on the lookback kernel (make_schedule).
+constexpr size_t SWEEP_BESIDE_PER_SM = 8 * 4096;
 
 bool sweep_enabled() { return batch_tail_enabled() && !std::getenv("IIR_GB300_BATCH_TAIL_CHUNKS"); }
 
@@ -885,31 +877,38 @@ size_t sweep_run_capacity(const iir_batch* b, size_t segs, size_t chunks) {
 }
 
 // The sweep takes every segment whose filter decays within a tile, unless a fault is to be injected (it
-// has no carries to withhold) or the environment asks for a lookback schedule.
+// has no carries to withhold), the environment asks for a lookback schedule, or there is little of it beside others.
 int make_schedule(iir_batch* b, const iir_segment* segs, int n_segs, bool inject, cudaStream_t stream, Schedule& c) {
-    const bool sweep = c.sweep = !inject && sweep_enabled();
-    // 4096-sample tiles unless padding costs more than the shorter tiles' overhead (a 1024-sample tile
-    // scans as many lanes for a quarter of the samples)
+    const bool sweep = !inject && sweep_enabled();
+    // 4096-sample tiles unless padding costs more than the shorter tiles' overhead (a 1024-sample tile scans as many
+    // lanes for a quarter of the samples; from 5 sections on that is most of a tile's cost: order 10, 1024 segments of
+    // 1000 to 3000 samples 18.5 us in large tiles, 24.2 in small ones, of 100 to 600 21.1 and 13.0), and only if they
+    // cover the filters that the large ones do
     size_t large = 0, small = 0;
     if (sweep) {
         for (int i = 0; i < n_segs; ++i) {
             large += 4096 * sweep_tiles(segs[i], 4096);
             small += 1024 * sweep_tiles(segs[i], 1024);
         }
-        c.v = 2 * large > 3 * small ? 1 : 0;
-        if (c.v == 1 && !(b->sweep[1].ready && (b->sweep[1].covers || b->shape_data[static_cast<size_t>(b->shape)].all))) {
+        c.v = 2 * large > (b->max_sections > 4 ? 6 : 3) * small ? 1 : 0;
+        if (c.v == 1 && !b->sweep[1].ready) {
             // tables to build, which no capture allows: it gets the tiles that are there
             cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
             if (const int st = cuda_status(cudaStreamIsCapturing(stream, &cap))) return st;
             if (cap != cudaStreamCaptureStatusNone) c.v = 0;
         }
         if (const int st = sweep_prepare(b, c.v)) return st;
+        for (int i = 0; i < n_segs && c.v == 1; ++i) {
+            const size_t f = static_cast<size_t>(segs[i].filter);
+            if (segs[i].n > 0 && b->sweep[0].filters[f].fast && !b->sweep[1].filters[f].fast) c.v = 0;
+        }
     }
     const SweepData& d = b->sweep[c.v];
     const int tile = sweep ? d.kern->tile() : 1;
-    // A run costs the pass A of the tile ahead of it, so it is long, but every block should see several.
+    // A run costs the tile ahead of it, so it is long, but every block should see several.
     const size_t total = (c.v == 0 ? large : small) / static_cast<size_t>(tile);
     c.len = std::min<size_t>(16, std::max<size_t>(4, total / static_cast<size_t>(6 * b->sms)));
+    size_t samples = 0;  // swept
     for (int i = 0; i < n_segs; ++i) {
         const iir_segment& s = segs[i];
         if (s.n == 0) continue;
@@ -920,7 +919,18 @@ int make_schedule(iir_batch* b, const iir_segment* segs, int n_segs, bool inject
             c.swept.push_back(i);
             c.runs += (tiles + c.len - 1) / c.len;
             c.longest = std::max(c.longest, std::min(tiles, c.len));
+            samples += s.n;
         }
+    }
+    // Two kernels take turns on the SMs and need a fork and a join, so a small sweep beside slow segments goes to the
+    // lookback kernel with them (order 10, a quarter of the segments slow, one kernel / two: 64 of 20000 to 80000
+    // samples 25.2 / 36.2 us, 1024 of 4097 to 5000 38.5 / 46.2, of 8000 to 12000 64.5 / 60.4).
+    if (!c.rest.empty() && samples < SWEEP_BESIDE_PER_SM * static_cast<size_t>(b->sms)) {
+        c.rest.clear();
+        for (int i = 0; i < n_segs; ++i)
+            if (segs[i].n > 0) c.rest.push_back(segs[i]);
+        c.swept.clear();
+        c.runs = 0;
     }
     return c.runs > 0x7fffffffull ? IIR_ERR_TOO_LARGE : IIR_OK;
 }
@@ -988,7 +998,8 @@ IirBatchSweepParams sweep_params(const iir_batch* b, const Schedule& c, const ii
     q.tables = d.d_tables;
     q.state = b->d_sweep_state;
     q.nruns = static_cast<unsigned>(c.runs);
-    q.unit = c.longest >= 8 ? 1 : 2;  // short runs are drawn in pairs: a draw takes about a microsecond
+    // short runs are drawn in pairs (a draw takes about a microsecond), unless every block gets but one
+    q.unit = c.longest >= 8 || c.runs <= static_cast<size_t>(d.resident) ? 1 : 2;
     return q;
 }
 
@@ -1090,9 +1101,9 @@ int check_segments(const iir_batch* b, const iir_segment* segs, int n_segs) {
 }
 
 // Segments (checked) on the lookback kernel: their table to the device, and the launch.
-int lookback_execute(iir_batch* b, const iir_segment* segs, int n_segs, bool all, cudaStream_t stream) {
+int lookback_execute(iir_batch* b, const iir_segment* segs, int n_segs, cudaStream_t stream) {
     const int k = b->shape;
-    if (const int st = shape_prepare(b, k, all)) return st;
+    if (const int st = shape_prepare(b, k)) return st;
     size_t total = 0, groups = 0;
     for (int i = 0; i < n_segs; ++i) {
         const size_t ch = seg_chunks(segs[i], k);
@@ -1203,7 +1214,7 @@ int iir_batch_create(iir_batch** out, const float* sos, const int* n_sections, i
     if (!st) st = shape_measure(b, 0);
     if (!st) st = sweep_prepare(b, 0);
     // the lookback kernel's tables at once where a segment may need it, else at its first launch
-    if (!st && !(b->sweep[0].covers && sweep_enabled())) st = shape_prepare(b, 0, !sweep_enabled());
+    if (!st && !(b->sweep[0].covers && sweep_enabled())) st = shape_prepare(b, 0);
     if (st) {
         batch_free(b);
         return st;
@@ -1218,7 +1229,7 @@ int iir_batch_set_shape(iir_batch* b, int rows, int samples_per_row) {
         if (shapes()[k].rows == rows && shapes()[k].n == samples_per_row) {
             const int st = b->sweep[0].covers && sweep_enabled()
                                ? shape_measure(b, static_cast<int>(k))
-                               : shape_prepare(b, static_cast<int>(k), !sweep_enabled());
+                               : shape_prepare(b, static_cast<int>(k));
             if (st) return st;
             b->shape = static_cast<int>(k);
             return IIR_OK;
@@ -1254,7 +1265,7 @@ int iir_batch_execute(iir_batch* b, const iir_segment* segs, int n_segs, void* s
         if (st) return st;
     }
     auto lookback = [&](cudaStream_t s) {
-        return c.rest.empty() ? IIR_OK : lookback_execute(b, c.rest.data(), static_cast<int>(c.rest.size()), !c.sweep || c.v != 0, s);
+        return c.rest.empty() ? IIR_OK : lookback_execute(b, c.rest.data(), static_cast<int>(c.rest.size()), s);
     };
     auto sweep = [&](cudaStream_t s) {
         if (c.runs == 0) return static_cast<int>(IIR_OK);
@@ -1297,7 +1308,7 @@ int iir_batch_bind(iir_batch* b, const iir_segment* all, int n_all, iir_batch_bo
     if (st) return st;
     const iir_segment* segs = c.rest.data();
     const int n_segs = static_cast<int>(c.rest.size());
-    if (n_segs > 0) st = shape_prepare(b, k, !c.sweep || c.v != 0);
+    if (n_segs > 0) st = shape_prepare(b, k);
     if (!st) st = cuda_status(cudaDeviceSynchronize());
     if (st) return st;
     iir_batch_bound* h = new iir_batch_bound();
