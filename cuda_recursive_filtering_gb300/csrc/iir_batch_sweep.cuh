@@ -837,6 +837,10 @@ __global__ void __launch_bounds__((W + 1 + BSWEEP_COPIERS) * 32) iir_batch_sweep
     }
     __syncthreads();
     if (threadIdx.x == 0) {
+        // loads still in flight (a stopped block) land before the block leaves (iir_sweep.cuh, sweep_tiles)
+        if (aux.abandon)
+            for (int b = 0; b < NB; ++b)
+                if (aux.issued[b] > 0u) (void)wait_mbar_bounded(aux.full + b, (aux.issued[b] - 1u) & 1u, IIR_DRAIN_NS);
         // the last block out re-arms the run counter
         __threadfence();
         if (atomicAdd(&p.state->done, 1u) == gridDim.x - 1u) {

@@ -208,6 +208,11 @@ __device__ __forceinline__ bool wait_mbar_bounded(unsigned long long* bar, uint3
     return true;
 }
 
+// A block that gives up first waits for its own copies and matrix products in flight: they write into memory that
+// another block may have by then. They take microseconds, so this limit has nothing to do with the launch's
+// timeout, which may be short.
+constexpr long long IIR_DRAIN_NS = 1000000000ll;
+
 // ------------------------------------------------------------------------------------
 // 2x2 helpers (row-major float4 {m00, m01, m10, m11})
 // ------------------------------------------------------------------------------------
@@ -649,7 +654,10 @@ __device__ __forceinline__ bool block_acquire(const IirParams& p, float* buf, Bl
         bool arrived = true;
         if (threadIdx.x >= 32) arrived = wait_mbar_bounded(&aux->mbar, 0, p.timeout_ns);
         if (__syncthreads_or(arrived ? 0 : 1)) {
-            if (threadIdx.x == 0) raise_error(p.state, epoch, IIR_DEV_ERR_MBARRIER);
+            if (threadIdx.x == 0) {
+                raise_error(p.state, epoch, IIR_DEV_ERR_MBARRIER);
+                (void)wait_mbar_bounded(&aux->mbar, 0, IIR_DRAIN_NS);
+            }
             return false;
         }
     } else {

@@ -821,6 +821,11 @@ __device__ __forceinline__ void sweep_tiles(const IirSweepParams& p, unsigned ch
     }
     __syncthreads();
     if (threadIdx.x == 0) {
+        // Loads still in flight (a stopped block) land before the block leaves: the last one of each buffer
+        // completes its barrier's last phase, and every earlier one had been waited for before it was issued.
+        if (aux.abandon)
+            for (int b = 0; b < NB; ++b)
+                if (aux.issued[b] > 0u) (void)wait_mbar_bounded(aux.full + b, (aux.issued[b] - 1u) & 1u, IIR_DRAIN_NS);
         // the last block out re-arms the run counter
         __threadfence();
         if (atomicAdd(&p.state->done, 1u) == gridDim.x - 1u) {

@@ -631,7 +631,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) iir_tc_kernel(const __grid_cons
             // of each buffer completes its phase (tma_n - 1), and every earlier one had landed
             // before the next was issued
             for (int sb = 0; sb < 2; ++sb)
-                if (tma_n[sb] > 0) wait_mbar_bounded(&aux->mb_tma[sb], (tma_n[sb] - 1) & 1u, p.timeout_ns);
+                if (tma_n[sb] > 0) wait_mbar_bounded(&aux->mb_tma[sb], (tma_n[sb] - 1) & 1u, IIR_DRAIN_NS);
         }
         __syncwarp();
     } else if (warp < TC_CW0 + TC_CW) {
@@ -850,7 +850,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) iir_tc_kernel(const __grid_cons
         __syncthreads();
         if (ct == 0)  // GEMM 1 batches still in flight end before TMEM is freed
             while (g1_par < aux->g1_issued &&
-                   wait_mbar_bounded(&aux->mb_g1[g1_par & 1], (g1_par >> 1) & 1u, p.timeout_ns))
+                   wait_mbar_bounded(&aux->mb_g1[g1_par & 1], (g1_par >> 1) & 1u, IIR_DRAIN_NS))
                 ++g1_par;
     } else {
         // ================= back group =================
@@ -1114,7 +1114,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) iir_tc_kernel(const __grid_cons
         if (ct == 0) bulk_wait_all();  // the output tiles' TMA stores have completed
         __syncthreads();
         if (ct == 0)  // GEMM 2 batches still in flight end before TMEM is freed
-            while (g2_par < aux->g2_issued && wait_mbar_bounded(&aux->mb_g2, g2_par & 1u, p.timeout_ns)) ++g2_par;
+            while (g2_par < aux->g2_issued && wait_mbar_bounded(&aux->mb_g2, g2_par & 1u, IIR_DRAIN_NS)) ++g2_par;
     }
     if (warp < TC_CW0) __syncthreads();  // pairs with the compute groups' barrier above
     tc_fence_before();

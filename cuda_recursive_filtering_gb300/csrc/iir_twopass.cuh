@@ -266,7 +266,7 @@ __device__ __forceinline__ void run_twopass(const IirParams& p, unsigned char* s
         if (lane == 0) bulk_wait_all();
         if (*reinterpret_cast<volatile int*>(&aux->abandon) && lane == 0) {
             const uint32_t first = issued > static_cast<uint32_t>(S) ? issued - S : 0;
-            for (uint32_t q = first; q < issued; ++q) (void)wait_mbar_bounded(&aux->full[q % S], spar(q), p.timeout_ns);
+            for (uint32_t q = first; q < issued; ++q) (void)wait_mbar_bounded(&aux->full[q % S], spar(q), IIR_DRAIN_NS);
         }
     } else if (warp == 1) {
         // ------------------------------- lookback warp -------------------------------
