@@ -4,8 +4,8 @@
 // cascade (any number of sections up to IIR_MAX_SECTIONS), an optional state in (zi) and an
 // optional state out (zf). Two kernels share a call's segments:
 //   * the state sweep (iir_batch_sweep.cuh) takes every segment whose filter decays within a tile;
-//   * the lookback kernel below takes the others, and all of them when the sweep would be small beside it, a
-//     fault is injected or the environment asks for its schedules. Where both have segments they run side by side.
+//   * the lookback kernel below takes the others, and all of them when the sweep would be small beside it or
+//     the environment asks for its schedules. Where both have segments they run side by side.
 //
 // Lookback kernel: the launch's chunks are the concatenation of every segment's
 // chunks; that list is the launch's work queue. A persistent grid (every block resident: the
@@ -864,6 +864,10 @@ struct Schedule {
     size_t runs = 0;
     std::vector<int> swept;
     std::vector<iir_segment> rest;
+    // fault injection: the tile of a swept segment, or the chunk of the lookback kernel's, whose state is not passed on
+    int withhold_seg = -1;
+    unsigned int withhold_tile = BATCH_RUN_NONE;
+    long long withhold_chunk = -1;
 };
 
 // Samples per SM from which segments are swept while others are on the lookback kernel (make_schedule).
@@ -876,10 +880,10 @@ size_t sweep_run_capacity(const iir_batch* b, size_t segs, size_t chunks) {
     return 2 * segs + 6 * static_cast<size_t>(b->sms) + chunks / 2 + 8;
 }
 
-// The sweep takes every segment whose filter decays within a tile, unless a fault is to be injected (it
-// has no carries to withhold), the environment asks for a lookback schedule, or there is little of it beside others.
-int make_schedule(iir_batch* b, const iir_segment* segs, int n_segs, bool inject, cudaStream_t stream, Schedule& c) {
-    const bool sweep = !inject && sweep_enabled();
+// The sweep takes every segment whose filter decays within a tile, unless the environment asks for a lookback
+// schedule or there is little of it beside others.
+int make_schedule(iir_batch* b, const iir_segment* segs, int n_segs, cudaStream_t stream, Schedule& c) {
+    const bool sweep = sweep_enabled();
     // 4096-sample tiles unless padding costs more than the shorter tiles' overhead (a 1024-sample tile scans as many
     // lanes for a quarter of the samples; from 5 sections on that is most of a tile's cost: order 10, 1024 segments of
     // 1000 to 3000 samples 18.5 us in large tiles, 24.2 in small ones, of 100 to 600 21.1 and 13.0), and only if they
@@ -952,6 +956,7 @@ void sweep_runs(const iir_batch* b, const Schedule& c, const iir_segment* segs, 
         r.K = static_cast<unsigned char>(b->filter_sections[static_cast<size_t>(s.filter)]);
         r.rounds = static_cast<unsigned char>(f.rounds);
         r.peel = static_cast<unsigned char>(peel);
+        r.withhold = i == c.withhold_seg ? c.withhold_tile : BATCH_RUN_NONE;
         for (size_t t = 0; t < tiles; t += c.len) {
             r.tile0 = static_cast<unsigned>(t);
             r.count = static_cast<unsigned>(std::min(c.len, tiles - t));
@@ -1083,6 +1088,30 @@ int launch_both(iir_batch* b, cudaStream_t stream, bool both, Lookback&& lookbac
     return st ? st : side;
 }
 
+// The injected fault: chunk b->withhold of the call, for one launch. A swept segment withholds the tile in which the
+// chunk ends.
+void schedule_withhold(iir_batch* b, const iir_segment* segs, int n_segs, Schedule& c) {
+    long long left = b->withhold, rest = 0;
+    b->withhold = -1;
+    const ShapeDef& sd = shapes()[static_cast<size_t>(b->shape)];
+    for (int i = 0; i < n_segs; ++i) {
+        const long long chunks = static_cast<long long>(seg_chunks(segs[i], b->shape));
+        const bool swept = std::find(c.swept.begin(), c.swept.end(), i) != c.swept.end();
+        if (left < chunks) {
+            if (swept) {
+                c.withhold_seg = i;
+                c.withhold_tile =
+                    static_cast<unsigned int>(((left + 1) * sd.rows * sd.n - 1) / b->sweep[c.v].kern->tile());
+            } else {
+                c.withhold_chunk = rest + left;
+            }
+            return;
+        }
+        left -= chunks;
+        if (!swept) rest += chunks;
+    }
+}
+
 // Arguments of every segment, and the number of chunks (of the current shape) within bounds.
 int check_segments(const iir_batch* b, const iir_segment* segs, int n_segs) {
     size_t total = 0;
@@ -1101,7 +1130,7 @@ int check_segments(const iir_batch* b, const iir_segment* segs, int n_segs) {
 }
 
 // Segments (checked) on the lookback kernel: their table to the device, and the launch.
-int lookback_execute(iir_batch* b, const iir_segment* segs, int n_segs, cudaStream_t stream) {
+int lookback_execute(iir_batch* b, const iir_segment* segs, int n_segs, long long withhold, cudaStream_t stream) {
     const int k = b->shape;
     if (const int st = shape_prepare(b, k)) return st;
     size_t total = 0, groups = 0;
@@ -1152,8 +1181,7 @@ int lookback_execute(iir_batch* b, const iir_segment* segs, int n_segs, cudaStre
     if (!st) st = cuda_status(cudaEventRecord(b->stage_done[turn], stream));
     if (st) return st;
     IirBatchParams q = batch_params(b, k, b->d_segs, b->d_starts, static_cast<unsigned int>(n_segs),
-                                    static_cast<unsigned int>(total), b->withhold);
-    b->withhold = -1;
+                                    static_cast<unsigned int>(total), withhold);
     return batch_launch(b, k, q, stream);
 }
 
@@ -1257,15 +1285,16 @@ int iir_batch_execute(iir_batch* b, const iir_segment* segs, int n_segs, void* s
     cudaStream_t stream = static_cast<cudaStream_t>(stream_);
     if (const int st = check_segments(b, segs, n_segs)) return st;
     Schedule c;
-    int st = make_schedule(b, segs, n_segs, b->withhold >= 0, stream, c);
+    int st = make_schedule(b, segs, n_segs, stream, c);
     if (st) return st;
+    if (b->withhold >= 0) schedule_withhold(b, segs, n_segs, c);
     if (c.runs > b->run_cap) {
         cudaStreamSynchronize(stream);
         st = batch_alloc_runs(b, 2 * c.runs);
         if (st) return st;
     }
     auto lookback = [&](cudaStream_t s) {
-        return c.rest.empty() ? IIR_OK : lookback_execute(b, c.rest.data(), static_cast<int>(c.rest.size()), s);
+        return c.rest.empty() ? IIR_OK : lookback_execute(b, c.rest.data(), static_cast<int>(c.rest.size()), c.withhold_chunk, s);
     };
     auto sweep = [&](cudaStream_t s) {
         if (c.runs == 0) return static_cast<int>(IIR_OK);
@@ -1304,7 +1333,7 @@ int iir_batch_bind(iir_batch* b, const iir_segment* all, int n_all, iir_batch_bo
     const int k = b->shape;
     if (const int st = check_segments(b, all, n_all)) return st;
     Schedule c;
-    int st = make_schedule(b, all, n_all, false, nullptr, c);  // (a bound launch takes no injected fault)
+    int st = make_schedule(b, all, n_all, nullptr, c);  // (a bound launch takes no injected fault)
     if (st) return st;
     const iir_segment* segs = c.rest.data();
     const int n_segs = static_cast<int>(c.rest.size());

@@ -389,7 +389,8 @@ struct BatchSweepAux {
 
 // Every wait of a block is bounded; the first to run out sends the whole block home.
 template <class Aux, class Cond>
-__device__ __forceinline__ bool bsweep_wait(Aux& aux, const IirBatchSweepParams& p, Cond&& cond) {
+__device__ __forceinline__ bool bsweep_wait(Aux& aux, const IirBatchSweepParams& p, Cond&& cond,
+                                            uint32_t code = IIR_DEV_ERR_MBARRIER) {
     if (cond()) return true;
     const uint64_t start = globaltimer_ns();
     uint32_t spins = 0;
@@ -399,7 +400,7 @@ __device__ __forceinline__ bool bsweep_wait(Aux& aux, const IirBatchSweepParams&
         if (aux.abandon) return false;
         if (globaltimer_ns() - start > static_cast<uint64_t>(p.timeout_ns)) {
             aux.abandon = 1u;
-            raise_error(p.state, 0xffffffffu, IIR_DEV_ERR_MBARRIER);
+            raise_error(p.state, sweep_epoch(p.state), code);
             return false;
         }
     }
@@ -622,7 +623,7 @@ __device__ __forceinline__ bool bsweep_item(const IirBatchSweepParams& p, BatchS
                 for (int c = 0; c < D; c += 2)
                     *reinterpret_cast<float2*>(&aux.ends[i % Aux::RING][c]) = make_float2(last[c], last[c + 1]);
                 __threadfence_block();
-                aux.ready[i % Aux::RING] = i + 1u;
+                if (t != run.withhold) aux.ready[i % Aux::RING] = i + 1u;
             }
         };
         if constexpr (bsweep_chained(K)) {
@@ -799,12 +800,14 @@ __global__ void __launch_bounds__((W + 1 + BSWEEP_COPIERS) * 32) iir_batch_sweep
                 return !__any_sync(FULL_MASK, !got);
             };
             auto ready = [&] {
-                const bool got = bsweep_wait(aux, p, [&] { return aux.ready[(i - 1u) % Aux::RING] == i; });
+                const bool got =
+                    bsweep_wait(aux, p, [&] { return aux.ready[(i - 1u) % Aux::RING] == i; }, IIR_DEV_ERR_TIMEOUT);
                 __threadfence_block();
                 return !__any_sync(FULL_MASK, !got);
             };
             auto checked = [&] {
-                const bool got = bsweep_wait(aux, p, [&] { return aux.checked[(i - 1u) % Aux::RING] >> 1 == i; });
+                const bool got =
+                    bsweep_wait(aux, p, [&] { return aux.checked[(i - 1u) % Aux::RING] >> 1 == i; }, IIR_DEV_ERR_TIMEOUT);
                 __threadfence_block();
                 return !__any_sync(FULL_MASK, !got);
             };
@@ -841,13 +844,7 @@ __global__ void __launch_bounds__((W + 1 + BSWEEP_COPIERS) * 32) iir_batch_sweep
         if (aux.abandon)
             for (int b = 0; b < NB; ++b)
                 if (aux.issued[b] > 0u) (void)wait_mbar_bounded(aux.full + b, (aux.issued[b] - 1u) & 1u, IIR_DRAIN_NS);
-        // the last block out re-arms the run counter
-        __threadfence();
-        if (atomicAdd(&p.state->done, 1u) == gridDim.x - 1u) {
-            p.state->runs = 0u;
-            p.state->done = 0u;
-            __threadfence();
-        }
+        sweep_finish(p.state);
     }
 }
 

@@ -41,6 +41,8 @@ __host__ __device__ constexpr int bsweep_table_capacity(int K, int span) {
     return most;
 }
 
+constexpr unsigned BATCH_RUN_NONE = 0xffffffffu;
+
 // Consecutive tiles of one segment. x is on the 16-byte grid; `peel` samples (0..3) lie before it.
 struct __align__(16) BatchRun {
     const float* x;
@@ -53,7 +55,8 @@ struct __align__(16) BatchRun {
     unsigned int table;    // the filter's table, in 16-byte units from the launch's tables
     unsigned char K, rounds, peel;
     unsigned char warm;    // 1: the tile before tile0 leads up to it
-    unsigned char pad[8];
+    unsigned int withhold; // fault injection: the tile whose end state is not passed on (BATCH_RUN_NONE: none)
+    unsigned char pad[4];
 };
 static_assert(sizeof(BatchRun) == 64, "copied as 16 words");
 

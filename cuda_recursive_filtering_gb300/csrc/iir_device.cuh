@@ -167,6 +167,21 @@ __device__ __forceinline__ void raise_error(IirLaunchState* st, uint32_t epoch, 
     if (h) *reinterpret_cast<volatile unsigned long long*>(h) = w;  // seen by the host without a sync
 }
 
+// The state-sweep kernels draw no tickets, but each launch takes an epoch of the same count: the last block out
+// moves it on, so a block reads its launch's until it leaves.
+__device__ __forceinline__ uint32_t sweep_epoch(const IirLaunchState* st) {
+    return static_cast<uint32_t>(ld_relaxed_u64(&st->ticket) >> 32);
+}
+__device__ __forceinline__ void sweep_finish(IirLaunchState* st) {
+    __threadfence();
+    if (atomicAdd(&st->done, 1u) == gridDim.x - 1u) {
+        st->runs = 0u;  // re-arms the run counter
+        st->done = 0u;
+        atomicAdd(&st->ticket, 1ull << 32);
+        __threadfence();
+    }
+}
+
 // Takes the block's ticket: one atomic returns the launch epoch (high word) and the chunk
 // id (low word). The block that draws the last chunk re-arms the counter for the next
 // launch on the stream (every other block of this launch has already drawn its ticket).

@@ -1070,10 +1070,28 @@ const SweepPart* sweep_pick(const iir_plan* p, size_t n) {
     return n >= sweep_large_per_sm(p->n_sections) * static_cast<size_t>(p->sms) ? &p->sweeps.front() : &p->sweeps.back();
 }
 
-int sweep_launch(iir_plan* p, const SweepPart& s, const float* x, float* y, size_t n, cudaStream_t stream) {
+// Counts a launch of the plan. Flags are 32-bit functions of the launch epoch: the slots and the launch state are
+// zeroed long before the epoch could wrap (the reference zeroes its status buffer once).
+int count_launch(iir_plan* p, cudaStream_t stream) {
+    if (++p->launches < (1ull << 30)) return IIR_OK;
+    int st = cuda_status(cudaMemsetAsync(p->d_carry, 0, p->carry_bytes, stream));
+    if (!st) st = cuda_status(cudaMemsetAsync(p->d_state, 0, IIR_STATE_RESET_BYTES, stream));
+    if (!st) p->launches = 1;
+    return st;
+}
+
+// withhold: the chunk (of `chunk` samples) whose state is not passed on, or -1.
+int sweep_launch(iir_plan* p, const SweepPart& s, const float* x, float* y, size_t n, long long withhold, size_t chunk,
+                 cudaStream_t stream) {
     const size_t tiles = sweep_tile_count(s, n);
     if (tiles > 0x7fffffffull) return IIR_ERR_TOO_LARGE;
+    if (const int st = count_launch(p, stream)) return st;
     IirSweepParams& q = p->sweep;
+    q.withhold = SWEEP_NONE;
+    if (withhold >= 0 && static_cast<size_t>(withhold) < (n + chunk - 1) / chunk) {
+        const size_t w = ((static_cast<size_t>(withhold) + 1) * chunk - 1) / (32 * static_cast<size_t>(s.k->span()));
+        if (w < tiles) q.withhold = static_cast<unsigned>(w);  // the tile in which the chunk ends
+    }
     const int span = s.k->span();
     const size_t rows = n / static_cast<size_t>(span);
     q.x = x;
@@ -1123,16 +1141,19 @@ int plan_launch(iir_plan* p, const float* x, float* y, size_t n, const float* zi
         p->withhold = -1;
         return st;
     }
-    // filters that decay within a tile's halo (a launch with an injected fault takes the lookback,
-    // whose carries it withholds)
-    if (!p->sweeps.empty() && !zi && p->withhold < 0)
-        if (const SweepPart* s = sweep_pick(p, n)) return sweep_launch(p, *s, x, y, n, stream);
     // the kernel for this signal: a single-section plan's small-signal kernel up to its limit
     // (a piece that starts from a carried state always takes the persistent schedule)
     const bool use_tiny = p->tiny && !zi && n <= p->tiny_max_n;
     const bool use_small = !use_tiny && p->small && !zi && n <= p->small_max_n;
     const KernelEntry* ent = use_tiny ? p->tiny : use_small ? p->small : p->entry;
     const size_t chunk = chunk_samples(p, ent);
+    // filters that decay within a tile
+    if (!p->sweeps.empty() && !zi)
+        if (const SweepPart* s = sweep_pick(p, n)) {
+            const int st = sweep_launch(p, *s, x, y, n, p->withhold, chunk, stream);
+            p->withhold = -1;
+            return st;
+        }
     const size_t nchunks = (n + chunk - 1) / chunk;
     if (nchunks > 0xffffffffull) return IIR_ERR_TOO_LARGE;
     if (nchunks > p->carry_cap) {
@@ -1143,14 +1164,7 @@ int plan_launch(iir_plan* p, const float* x, float* y, size_t n, const float* zi
     // blocks whose warps draw the chunks
     if (nchunks > 0x7fffffffull) return IIR_ERR_TOO_LARGE;
     const int grid = static_cast<int>(p->kind == IIR_KIND_PLR && ent->pipeline ? std::min<size_t>(nchunks, static_cast<size_t>(p->grid_max)) : nchunks);
-    // Flags are 32-bit functions of the launch epoch: re-zero the slots and the launch state
-    // long before the epoch could wrap (the reference zeroes its status buffer once).
-    if (++p->launches >= (1ull << 30)) {
-        int st = cuda_status(cudaMemsetAsync(p->d_carry, 0, p->carry_bytes, stream));
-        if (!st) st = cuda_status(cudaMemsetAsync(p->d_state, 0, IIR_STATE_RESET_BYTES, stream));
-        if (st) return st;
-        p->launches = 1;
-    }
+    if (const int st = count_launch(p, stream)) return st;
     const bool aligned = ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) & 15u) == 0;
     cudaError_t err;
     if (p->kind == IIR_KIND_PLR) {

@@ -51,7 +51,7 @@
 // earlier launch without synchronising (the one-shot entry points report it on their next call).
 // Periodic re-zeroing covers the first IIR_STATE_RESET_BYTES only, never host_error.
 struct IirLaunchState {
-    unsigned long long ticket;       // (epoch << 32) | ticket
+    unsigned long long ticket;       // (epoch << 32) | ticket (state-sweep kernels: the epoch alone)
     unsigned long long error;        // (epoch << 32) | status code of the first failure
     unsigned int done;               // persistent kernels: blocks of the launch that have exited
     unsigned int runs;               // state-sweep kernels: runs drawn in this launch (iir_sweep.cuh)

@@ -544,6 +544,8 @@ __device__ __noinline__ void sweep_unstage(const float* buf, float* y, long long
 // ------------------------------------------------------------------------------------
 // launch parameters and the tile loop
 // ------------------------------------------------------------------------------------
+constexpr unsigned SWEEP_NONE = 0xffffffffu;
+
 struct IirSweepParams {
     CUtensorMap tmap_x;  // x as rows of SPAN samples, box {32, 32}, 128-byte swizzle
     CUtensorMap tmap_y;  // y likewise
@@ -555,6 +557,7 @@ struct IirSweepParams {
     long long timeout_ns;
     unsigned int ntiles;
     unsigned int run0, run1;  // tiles of a block's first run, and of the runs drawn after it
+    unsigned int withhold;    // fault injection: the tile whose end state is not passed on (SWEEP_NONE: none)
     int lanes, rounds;        // lanes that a state reaches; scan steps that cover them
     int use_tma;              // tensor maps valid (x, y 16-byte aligned, at least one row)
     float gain;
@@ -623,7 +626,7 @@ __device__ __forceinline__ void sweep_tiles(const IirSweepParams& p, unsigned ch
         reinterpret_cast<float4*>(tab)[i] = __ldg(reinterpret_cast<const float4*>(p.tables) + i);
     __syncthreads();
     // every wait is bounded; the first to run out sends the whole block home
-    auto wait_for = [&](auto&& cond) {
+    auto wait_for = [&](auto&& cond, uint32_t code = IIR_DEV_ERR_MBARRIER) {
         if (cond()) return true;
         const uint64_t start = globaltimer_ns();
         uint32_t spins = 0;
@@ -632,7 +635,7 @@ __device__ __forceinline__ void sweep_tiles(const IirSweepParams& p, unsigned ch
             if (aux.abandon) return false;
             if (globaltimer_ns() - start > static_cast<uint64_t>(p.timeout_ns)) {
                 aux.abandon = 1u;
-                raise_error(p.state, 0xffffffffu, IIR_DEV_ERR_MBARRIER);
+                raise_error(p.state, sweep_epoch(p.state), code);
                 return false;
             }
         }
@@ -723,11 +726,11 @@ __device__ __forceinline__ void sweep_tiles(const IirSweepParams& p, unsigned ch
                     for (int c = 0; c < D; c += 2)
                         *reinterpret_cast<float2*>(&aux.ends[i % SWEEP_RING][c]) = make_float2(last[c], last[c + 1]);
                     __threadfence_block();
-                    aux.ready[i % SWEEP_RING] = i + 1u;
+                    if (t != p.withhold) aux.ready[i % SWEEP_RING] = i + 1u;
                 }
             }
             if (!warm && t > 0) {
-                const bool got = wait_for([&] { return aux.ready[(i - 1u) % SWEEP_RING] == i; });
+                const bool got = wait_for([&] { return aux.ready[(i - 1u) % SWEEP_RING] == i; }, IIR_DEV_ERR_TIMEOUT);
                 if (__any_sync(FULL_MASK, !got)) break;
                 __threadfence_block();
                 if (lane < p.lanes) {
@@ -775,7 +778,8 @@ __device__ __forceinline__ void sweep_tiles(const IirSweepParams& p, unsigned ch
                 }
                 bool before = false;  // the state before the tile lacked something
                 if (!warm && t > 0) {
-                    const bool got = wait_for([&] { return aux.checked[(i - 1u) % SWEEP_RING] >> 1 == i; });
+                    const bool got =
+                        wait_for([&] { return aux.checked[(i - 1u) % SWEEP_RING] >> 1 == i; }, IIR_DEV_ERR_TIMEOUT);
                     if (__any_sync(FULL_MASK, !got)) break;
                     __threadfence_block();
                     before = (aux.checked[(i - 1u) % SWEEP_RING] & 1u) != 0u;
@@ -826,13 +830,7 @@ __device__ __forceinline__ void sweep_tiles(const IirSweepParams& p, unsigned ch
         if (aux.abandon)
             for (int b = 0; b < NB; ++b)
                 if (aux.issued[b] > 0u) (void)wait_mbar_bounded(aux.full + b, (aux.issued[b] - 1u) & 1u, IIR_DRAIN_NS);
-        // the last block out re-arms the run counter
-        __threadfence();
-        if (atomicAdd(&p.state->done, 1u) == gridDim.x - 1u) {
-            p.state->runs = 0u;
-            p.state->done = 0u;
-            __threadfence();
-        }
+        sweep_finish(p.state);
     }
 }
 
