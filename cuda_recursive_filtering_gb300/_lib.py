@@ -70,6 +70,7 @@ def load(path: str | None = None):
         "iir_plan_set_timeout_ns": ([vp, ll], i),
         "iir_plan_debug_withhold": ([vp, ll], i),
         "iir_plan_info": ([vp, ip, ip, ip, ip, ip], i),
+        "iir_plan_uses_geometry": ([vp, sz], i),
         "iir_plan_launches_per_execute": ([vp], i),
         "iir_plan_destroy": ([vp], i),
         "iir_status_string": ([i], ctypes.c_char_p),

@@ -135,6 +135,10 @@ class Plan:
         check(st, "iir_plan_execute_host")
         return out
 
+    def uses_geometry(self, n: int) -> bool:
+        """Whether a launch over ``n`` samples runs a kernel of the plan's block_size and n_blocks."""
+        return bool(self._lib.iir_plan_uses_geometry(self._ptr, int(n)))
+
     def launches_per_execute(self) -> int:
         return int(self._lib.iir_plan_launches_per_execute(self._ptr))
 

@@ -2,9 +2,9 @@
 for a filter and signal length by timing the candidates on this GPU (CUDA events, device-
 resident data) and checking each against the FP64 reference filter on a prefix.
 
-The candidate order is a prior taken from measurements on GB300: at order 2 the two-pass
-single-section kernels, PH first; for cascades the precision form (TC) first, then PH with 64
-samples per row. (The reference
+The candidate order is a prior taken from measurements on GB300: PH with 64 samples per row first, whose
+state sweep is the fastest where it applies, then the other realizations. Where a realization's launch takes
+no notice of the geometry (Plan.uses_geometry), it is timed once for all of them. (The reference
 picks its launch shape from an occupancy model, gpu_specs.hpp:57-116; here the resident-block
 count comes from the CUDA occupancy query and the rest is measured.) Results are cached per
 (device, order, filter, signal-length bucket) in memory and, optionally, in a JSON file.
@@ -24,7 +24,7 @@ __all__ = ["tune", "tuned_plan", "GB300", "supply_blocks_per_sm", "demand_blocks
 
 _CANDIDATES_ORDER2 = [("PH", 32, 64), ("PH", 32, 32), ("STCR_UNROLL", 32, 64), ("STCR_UNROLL", 32, 32),
                       ("DTCR_UNROLL", 32, 128), ("DTCR_UNROLL", 32, 64), ("PH", 32, 128), ("PLR", 0, 0)]
-_CANDIDATES_CASCADE = [("TC", 0, 0), ("PH", 32, 64), ("PH", 32, 32), ("STCR_UNROLL", 32, 64), ("DTCR_UNROLL", 32, 64),
+_CANDIDATES_CASCADE = [("PH", 32, 64), ("TC", 0, 0), ("PH", 32, 32), ("STCR_UNROLL", 32, 64), ("DTCR_UNROLL", 32, 64),
                        ("PH", 32, 128), ("STCR_UNROLL", 32, 32)]
 _memo: dict = {}
 
@@ -68,10 +68,16 @@ def tune(sos, n: int, candidates=None, reps: int = 5, device=None, cache_path: s
     ref = _reference_check(sos, prefix)
     scale = float(np.max(np.abs(ref))) or 1.0
     table = []
+    timed_once = {}  # realization -> its row, where the geometry makes no difference
     for kernel, b, nb in candidates:
         try:
             plan = Plan(sos, kernel, b, nb, max_n=m, device=dev)
         except Exception:
+            continue
+        same = timed_once.get(kernel)
+        if same is not None and not plan.uses_geometry(m):
+            table.append(dict(same, block_size=b, n_blocks=nb))
+            plan.close()
             continue
         plan(x, y)
         plan.check()
@@ -91,6 +97,8 @@ def tune(sos, n: int, candidates=None, reps: int = 5, device=None, cache_path: s
         torch.cuda.synchronize()
         ms = s.elapsed_time(e) / reps
         table.append({"kernel": kernel, "block_size": b, "n_blocks": nb, "gsps": m / (ms * 1e-3) / 1e9})
+        if not plan.uses_geometry(m):
+            timed_once[kernel] = table[-1]
         plan.close()
     timed = [t for t in table if t["gsps"] is not None]
     if not timed:

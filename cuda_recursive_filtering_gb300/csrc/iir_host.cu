@@ -1348,9 +1348,13 @@ int iir_plan_info(const iir_plan* p, int* kernel, int* block_size, int* n_blocks
     if (kernel) *kernel = p->kind;
     if (block_size) *block_size = p->B;
     if (n_blocks) *n_blocks = p->N;
-    if (grid) *grid = p->grid_max;
+    if (grid) *grid = p->sweeps.empty() ? p->grid_max : p->sweeps.front().resident;
     if (n_sections) *n_sections = p->n_sections;
     return IIR_OK;
+}
+
+int iir_plan_uses_geometry(const iir_plan* p, size_t n) {
+    return p && p->kind != IIR_KIND_TC && (p->sweeps.empty() || !sweep_pick(p, n)) ? 1 : 0;
 }
 
 int iir_plan_launches_per_execute(const iir_plan* p) { return p ? 1 : 0; }

@@ -96,6 +96,8 @@ int iir_sos_filter(const float* x, float* y, size_t n, const float* sos, int n_s
  *     alike (ph_kernels.cuh:208, 501).
  *   - A block filters a chunk of whole tiles (32 to 256 rows); the chunk, not one tile, is
  *     the unit of the lookback.
+ *   - PH's state sweep takes no notice of the geometry: cascades whose state decays within a tile
+ *     (4096 samples) and, from about 2.5e6 samples, single sections (iir_plan_uses_geometry).
  * For PLR, block_size is the thread-block size and n_blocks the values per thread (PLR_X,
  * plr_kernels.cuh:94-101). */
 int iir_sos_filter_geom(const float* x, float* y, size_t n, const float* sos, int n_sections,
@@ -165,9 +167,15 @@ int iir_plan_set_timeout_ns(iir_plan* plan, long long timeout_ns);
  * publishing its carries (so its successors' waits run out). -1 disables. */
 int iir_plan_debug_withhold(iir_plan* plan, long long chunk);
 
-/* Resolved realization / geometry of a plan (after IIR_KERNEL_AUTO and defaults). */
+/* Resolved realization / geometry of a plan (after IIR_KERNEL_AUTO and defaults), and the resident
+ * blocks of its kernel for large signals. The geometry is the plan's even where a launch does not
+ * use it. */
 int iir_plan_info(const iir_plan* plan, int* kernel, int* block_size, int* n_blocks,
                   int* grid, int* n_sections);
+
+/* 1 if a launch over n samples runs a kernel of the plan's geometry; 0 if its work is laid out
+ * otherwise (PH's state sweep, the precision form). */
+int iir_plan_uses_geometry(const iir_plan* plan, size_t n);
 
 /* Number of kernel launches one iir_plan_execute issues (for launch accounting). */
 int iir_plan_launches_per_execute(const iir_plan* plan);

@@ -50,3 +50,58 @@ def test_auto_on_an_offset(order, cutoff, cuda_device):
     ref = torch.from_numpy(oracle.reference_golden(sos, x)[1]).cuda()
     got, precise = [float((Plan(sos, k, max_n=n)(xt).double() - ref).square().mean().sqrt()) for k in ("AUTO", "TC")]
     assert got <= 1.1 * precise, (got, precise)
+
+
+def test_geometry_is_reported_and_tuned_where_it_matters(cuda_device):
+    """Plans say whether a launch runs a kernel of their geometry, and the tuner times a realization once where
+    none does (the first maximum wins: PH keeps the geometry listed first)."""
+    from cuda_recursive_filtering_gb300 import autotune
+    fast, slow, large = FILTERS["fast"], signal.butter(4, 0.002, output="sos"), 16384 * SM
+    assert not Plan(fast, "PH").uses_geometry(1000) and not Plan(fast, "PH").uses_geometry(1 << 24)
+    assert Plan(fast, "DTCR").uses_geometry(1 << 24) and Plan(slow, "PH").uses_geometry(1 << 24)
+    assert not Plan(fast, "TC").uses_geometry(1000)
+    one = Plan(signal.butter(2, 0.1, output="sos"), "PH")
+    assert one.uses_geometry(large - 1) and not one.uses_geometry(large)
+    table = autotune.tune(fast, 1 << 22, reps=1)["table"]
+    assert len({t["gsps"] for t in table if t["kernel"] == "PH"}) == 1
+    assert len({t["gsps"] for t in autotune.tune(slow, 1 << 22, reps=1)["table"] if t["kernel"] == "PH" and t["gsps"]}) != 1
+
+
+@pytest.mark.parametrize("fast_len", (600_000, 700_000))  # swept samples on either side of 8 x 4096 per SM
+def test_batch_with_slow_segments(fast_len, cuda_device):
+    """Fast segments beside slow ones: on the lookback kernel with them below the line, on the sweep beside it
+    above, called directly, bound and from a CUDA graph."""
+    from cuda_recursive_filtering_gb300 import Batch
+    sos = [signal.butter(4, 0.1, output="sos").astype(np.float32), signal.butter(8, 0.2, output="sos").astype(np.float32),
+           signal.cheby1(8, 1.0, 0.04, output="sos").astype(np.float32)]
+    which = [0, 2, 1, 0, 2, 1, 0, 1, 0, 1]
+    lens = [100_003 if f == 2 else fast_len + i for i, f in enumerate(which)]
+    assert (sum(n for n, f in zip(lens, which) if f < 2) >= 8 * 4096 * SM) == (fast_len == 700_000)
+    off = np.concatenate([[0], np.cumsum(lens)])
+    x = np.random.default_rng(fast_len).uniform(-1, 1, int(off[-1])).astype(np.float32)
+    xt = torch.from_numpy(x).cuda()
+    yt = torch.zeros_like(xt)
+    refs = [oracle.reference_golden(sos[f], x[a:b])[1] for f, a, b in zip(which, off[:-1], off[1:])]
+
+    def verify(what):
+        torch.cuda.synchronize()
+        batch.check()
+        y = yt.cpu().numpy()
+        for i, ref in enumerate(refs):
+            assert np.max(np.abs(y[off[i]:off[i + 1]] - ref)) <= 1e-4 * np.max(np.abs(ref)), (what, i)
+        yt.zero_()
+
+    batch = Batch(sos, max_segments=16)
+    batch.packed(xt, yt, off, which)
+    verify("packed")
+    bound = batch.bind(xt, yt, off, which)
+    bound()
+    verify("bound")
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        bound()
+        bound()
+    yt.zero_()
+    graph.replay()
+    graph.replay()
+    verify("graph")
