@@ -61,3 +61,24 @@ def test_around_the_limits(order, cutoff, monkeypatch, cuda_device):
                 assert e["finite"] and e["rel_max"] <= 1e-4, e
         else:  # the same filter: two schedules' roundings apart, a hundred times below the signal's peak
             assert float((y - z).abs().max()) <= 1e-2 * float(z.abs().max())
+
+
+@pytest.mark.parametrize("order,cutoff", [(2, 0.1), (2, 0.002)])
+def test_against_rounded_taps(order, cutoff, cuda_device):
+    """FP64 filtering with the float32 direct form's own taps: what is left is rounding. A direct form rounds `order`
+    times a sample, by 2^-24 of the peak at most, and 1/A amplifies that by the sum of its impulse response.
+
+    Order 4 is not held to this: its doubling multiplies by rounded n-nacci factors, which costs more digits than the
+    taps do (1.9e-2 of the peak at cutoff 0.04). Its kernel for long signals is held to the other one's bits above."""
+    sos = signal.butter(order, cutoff, output="sos")
+    b, a = oracle.merge_sections(oracle.normalise_sos(sos)[0])
+    b, a = np.r_[1.0, np.float32(b)].astype(np.float64), np.r_[1.0, -np.float32(a)].astype(np.float64)
+    limit = order * 2.0 ** -24 * np.abs(signal.lfilter([1.0], a, np.r_[1.0, np.zeros(100000)])).sum()
+    for n in (SHORT, 3 * SHORT + 4097):
+        x = np.random.default_rng(n).uniform(-1, 1, n).astype(np.float32)
+        plan = Plan(sos, "PLR", max_n=n)
+        y = plan(torch.from_numpy(x).cuda()).cpu().numpy()
+        plan.check()
+        ref = signal.lfilter(b, a, oracle.reference_golden(sos, x)[0].astype(np.float64))
+        e = oracle.errors(y, ref)
+        assert e["finite"] and e["rel_max"] <= limit, (n, limit, e)

@@ -110,3 +110,23 @@ def test_zero_and_huge_samples_stay_where_they_are(cuda_device):
     y = plan(x)
     plan.check()
     assert bool(torch.isfinite(y[:at]).all()) and not bool(torch.isfinite(y[at]))
+
+
+@pytest.mark.parametrize("order", (4, 8, 16))
+@pytest.mark.parametrize("n", (25 * TILE + 99, 2 * LARGE + 99))
+@pytest.mark.parametrize("bad", (float("inf"), float("nan")))
+def test_what_a_non_finite_sample_spoils(bad, n, order, cuda_device):
+    """The output is not finite from the sample on for as long as sub-rows' states reach, at most to the end of the next
+    tile: tiles that a filter's memory does not reach start from rest. What comes before and after is as without it."""
+    plan = Plan(design(order), "PH", max_n=n)
+    x = torch.from_numpy(np.random.default_rng(order).uniform(-1, 1, n).astype(np.float32)).cuda()
+    clean = plan(x).clone()
+    at = 20 * TILE + 77
+    x[at] = bad
+    y = plan(x)
+    plan.check()
+    end = 22 * TILE
+    assert not bool(torch.isfinite(y[at]))
+    scale = float(clean.abs().max())
+    assert float((y[:at] - clean[:at]).abs().max()) <= 1e-6 * scale
+    assert float((y[end:] - clean[end:]).abs().max()) <= 1e-6 * scale
