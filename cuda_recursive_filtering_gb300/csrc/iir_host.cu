@@ -705,10 +705,14 @@ constexpr size_t sweep_large_per_sm(int K) { return K == 8 ? 12288 : 16384; }
 // Below sweep_large_per_sm the lookback kernels filter
 //   * single sections, which have one-block-per-chunk kernels there (order 2: 8.7 us against 6.9 at 2^20, 9.5
 //     against 10.7 at 3e6; PLR's order 2 has none: 2^20 samples 8.9 us, 8.7 on the sweep; 3e6 22.5, 9.2);
-//   * from 4 sections on, filters for which the sweep has to correct white noise (cheby1(12, 1, 0.3), sweep /
-//     lookback: 2^18 samples 21.2 / 16.8 us, 2.4e6 21.6 / 20.9; butter(6, 0.02, high): 9.0 / 10.6);
 //   * below half of it, filters that decay within a large tile but not within a small one (butter(4, 0.01): 2^18
 //     samples 10.1 / 8.5 us, 2^20 10.2 / 9.2, 2.4e6 10.6 / 12.9).
+//
+// From 4 sections on, filters for which the sweep has to correct white noise (an emulated residual above 0.7 of its
+// limit) keep the lookback kernels at every size (sweep / lookback: cheby1(12, 1, 0.3) 2^18 samples 21.2 / 16.8 us, 5e6
+// 37.5 / 25.5, 2e7 92.4 / 85.0; cheby1(8, 1, 0.3, high) 5e6 24.8 / 17.5, 2e7 61.1 / 57.2). With 2 or 3 the sweep is as
+// fast or faster but for 2.6e6 to 5e6 samples (butter(6, 0.02, high): 1e5 9.8 / 10.8, 5e6 21.0 / 15.9, 2e7 50.0 /
+// 51.5; butter(4, 0.03, high): 14.7 / 12.5, 35.8 / 43.9), where it keeps the digits that the lookback loses to an offset.
 // Adds the plan's state-sweep kernels: those whose tiles cover the filter's decay. automatic: AUTO chose them.
 int plan_add_sweeps(iir_plan* p, const std::vector<SectionF32>& secs, double gain, bool automatic) {
     if (tail_max_pieces() <= 0) return IIR_OK;  // the lookback everywhere
@@ -717,11 +721,21 @@ int plan_add_sweeps(iir_plan* p, const std::vector<SectionF32>& secs, double gai
     if (kernels.empty()) return IIR_OK;  // another realization
     if (sweep_too_slow(secs.data(), p->n_sections, SWEEP_LANES * kernels.front()->span())) return IIR_OK;
     const SweepFilter f = sweep_filter(secs.data(), p->n_sections, gain);
+    // (AUTO's choice from 6 sections on holds for every size)
+    const bool chosen = p->n_sections >= SWEEP_DIFF_MIN_SECTIONS && automatic;
+    std::vector<SweepPart> parts;
     for (const SweepKernel* k : kernels) {
         SweepPart s;
         s.k = k;
         s.lanes = sweep_decay(f, k->span(), SWEEP_LANES);
-        if (s.lanes == 0) continue;
+        if (s.lanes > 0) parts.push_back(s);
+    }
+    if (!chosen && p->n_sections >= 4 && !parts.empty()) {
+        const int N = parts.back().k->N;
+        if (sweep_trial(f, sweep_tables(f, N, parts.back().k->R), N, false, 24).residual > 0.7) return IIR_OK;
+    }
+    for (SweepPart s : parts) {
+        const SweepKernel* k = s.k;
         const std::vector<float> tab = sweep_tables(f, k->N, k->R);
         int st = cuda_status(
             cudaFuncSetAttribute(k->fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(k->smem)));
@@ -741,12 +755,8 @@ int plan_add_sweeps(iir_plan* p, const std::vector<SectionF32>& secs, double gai
     }
     if (!p->sweeps.empty()) {
         const SweepPart& last = p->sweeps.back();
-        // (AUTO's choice from 6 sections on holds for every size)
-        const bool chosen = p->n_sections >= SWEEP_DIFF_MIN_SECTIONS && automatic;
         const size_t large = sweep_large_per_sm(p->n_sections) * static_cast<size_t>(p->sms);
         if (p->n_sections == 1) p->sweep_min_n = p->kind == IIR_KIND_PLR ? PLR_BLOCK_MAX_N + 1 : large;
-        else if (!chosen && p->n_sections >= 4 && sweep_trial(f, sweep_tables(f, last.k->N, last.k->R), last.k->N, false, 24).residual > 0.7)
-            p->sweep_min_n = large;
         else if (!chosen && last.k == kernels.front()) p->sweep_min_n = large / 2;
     }
     IirSweepParams& q = p->sweep;

@@ -105,3 +105,18 @@ def test_batch_with_slow_segments(fast_len, cuda_device):
     graph.replay()
     graph.replay()
     verify("graph")
+
+
+@pytest.mark.parametrize("sos", [signal.cheby1(8, 1, 0.3, "high", output="sos"), signal.cheby1(12, 1, 0.3, output="sos")])
+def test_filters_that_correct_white_noise(sos, monkeypatch, cuda_device):
+    """From 4 sections on the lookback filters at every size what the sweep would have to correct on any signal."""
+    plan = Plan(sos, "PH", max_n=1 << 20)
+    assert all(plan.uses_geometry(n) for n in (1000, 1 << 20, 16384 * SM, 1 << 27))
+    monkeypatch.setenv("IIR_GB300_TAIL", "0")
+    lookback = Plan(sos, "PH", max_n=1 << 20)
+    n = 16384 * SM + 77
+    x = np.random.default_rng(5).uniform(-1, 1, n).astype(np.float32)
+    _, ref = oracle.reference_golden(sos, x)
+    got, general = [np.max(np.abs(p(torch.from_numpy(x).cuda()).cpu().numpy().astype(np.float64) - ref)) for p in (plan, lookback)]
+    peak = np.max(np.abs(ref))
+    assert got <= 1e-4 * peak and got <= 2 * general + 2.0 ** -24 * peak
