@@ -14,9 +14,10 @@ sample), and the error of ALL of that row's outputs against the FP64 oracle (the
 golden path, tools/ref_generate.py:89), compared on the device. The precision form is
 measured at orders 8..16 on its own workload with the same full-length error.
 
-    python bench.py [--gpus N] [--steps K] [--warmup W] [--impl ours|reference] [--no-sweep]
+    python bench.py [--gpus N] [--steps K] [--warmup W] [--impl ours|reference] [--no-sweep] [--tables FILE]
 
-Prints one JSON line (rank 0). Under torchrun every rank filters its own replica of the
+Prints one JSON line (rank 0): the headline, with the rates of the other legs in "rates". Their full tables go
+to a JSON file (--tables, bench_tables.json beside this script if not given). Under torchrun every rank filters its own replica of the
 workload on its own GPU (the path has no exchange step between GPUs: replicas only).
 """
 from __future__ import annotations
@@ -386,8 +387,8 @@ def run_reference(args, rank: int, world: int) -> None:
 # forms (batching, serving, precision)
 # ------------------------------------------------------------------------------------------
 def run_batching(dev) -> dict:
-    """Many channels of uneven length, each with its own filter, in one persistent launch; the
-    chunk shape chosen by autotune.tune_batch (every compiled shape timed, in the order the
+    """Many channels of uneven length, each with its own filter, in one call (up to two launches: the state sweep
+    for filters that decay within a tile, the lookback kernel for the rest); the lookback's chunk shape chosen by autotune.tune_batch (every compiled shape timed, in the order the
     occupancy model proposes); then the launch over a bound segment table is captured in a CUDA
     graph, and 10 replays are timed with CUDA events (device-resident); a few channels are
     checked against the oracle."""
@@ -428,8 +429,8 @@ def run_batching(dev) -> dict:
         _, ref = oracle.reference_golden(filters[i], xi)
         worst = max(worst, oracle.errors(y[off[i]:off[i + 1]].cpu().numpy(), ref)["rel_max"])
     return {"workload": "4096 channels, lengths log-uniform [2^10, 2^20], own filter each: order {2,4,8,16}, "
-                        "butter / cheby1 (1 dB), cutoff U[0.02, 0.45], seed 3; one persistent launch of the "
-                        "tuned chunk shape over a bound segment table, replayed from a captured CUDA graph",
+                        "butter / cheby1 (1 dB), cutoff U[0.02, 0.45], seed 3; one call over a bound "
+                        "segment table (lookback kernel: the tuned chunk shape), replayed from a captured CUDA graph",
             "value": round(float(off[-1]) / (ms * 1e-3) / 1e9, 1), "unit": "GS/s", "ms_per_launch": ms,
             "samples": int(off[-1]), "check_rel_max_8_channels": worst, "shape": batch.shape(),
             "tuner": tuned}
@@ -840,10 +841,40 @@ def run_ours(args, rank: int, world: int, local_rank: int) -> None:
         "clocks": clk,
         "check": {"rel_max": float(f"{chk['rel_max']:.3g}"), "rel_rms": float(f"{chk['rel_rms']:.3g}"),
                   "samples": n, "what": "all outputs of the last timed launch against the FP64 oracle"},
-        "sweep": sweep,
     }
-    out.update(forms)
+    tables = {"sweep": sweep, **forms}
+    if any(tables.values()):
+        with open(args.tables, "w") as f:
+            json.dump({**out, **tables}, f, indent=1)
+        out["rates"] = summary(tables)
+        out["tables"] = os.path.basename(args.tables)
     print(json.dumps(out), flush=True)
+
+
+def summary(tables: dict) -> dict:
+    """The rates (GS/s) of the full tables that fit a line: the realizations at the default geometry by order, the
+    precision form, batching and serving; and the worst max|err| / max|ref| of the cascades."""
+    out = {}
+    for size, rows in tables.get("sweep", {}).items():
+        if size != f"2^{LOG2N}":
+            continue
+        for kname in ("PH", "DTCR_UNROLL", "STCR_UNROLL"):
+            got = [rows.get(f"order{o}_{kname}_32x64") for o in (2, 4, 8, 16)]
+            out[kname] = [r.get("gsps") if isinstance(r, dict) else None for r in got]
+        worst = [r["rel_max"] for k, r in rows.items() if isinstance(r, dict) and "PLR" not in k]
+        out["orders"], out["worst_rel_max"] = [2, 4, 8, 16], max(worst, default=None)
+    for order in (8, 16):
+        row = tables.get("precision", {}).get(f"order{order}", {})
+        if "TC" in row:
+            out[f"TC_order{order}"] = row["TC"]["gsps"]
+    if "value" in tables.get("batching", {}):
+        out["batching"] = tables["batching"]["value"]
+    if "gsps" in tables.get("serving", {}):
+        out["serving"] = {k: round(tables["serving"][k], 3) for k in ("gsps", "p50_us", "p99_us")}
+    for leg in ("sweep", "precision", "batching", "serving"):
+        if "error" in tables.get(leg, {}):
+            out[f"{leg}_error"] = str(tables[leg]["error"])[:120]
+    return out
 
 
 def run_only_batch(args, spec: str) -> None:
@@ -924,6 +955,7 @@ def main() -> None:
     ap.add_argument("--impl", choices=("ours", "reference"), default="ours")
     ap.add_argument("--no-sweep", action="store_true")
     ap.add_argument("--no-forms", action="store_true", help="skip the precision, batching and serving legs")
+    ap.add_argument("--tables", default=os.path.join(ROOT, "bench_tables.json"), help="file for the full tables")
     ap.add_argument("--cpu-seconds", type=float, default=12.0)
     ap.add_argument("--log2n", type=int, default=LOG2N,
                     help="signal length 2^k (the bench line is quoted at 2^28; smaller k is for profiling)")

@@ -307,7 +307,8 @@ class Batch:
 
     def bind(self, x: torch.Tensor, y: torch.Tensor, offsets, filters, zi=None, zf=None) -> "BoundBatch":
         """Packed segments (as :meth:`packed`) uploaded once; the returned object launches
-        them with a single kernel launch per call, which CUDA graphs can capture."""
+        them with at most two kernel launches per call (the state sweep and the lookback kernel), which CUDA graphs can
+        capture."""
         _check_tensor(x, "x")
         _check_tensor(y, "y")
         off = np.asarray(offsets, dtype=np.int64)

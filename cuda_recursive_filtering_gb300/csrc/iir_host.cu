@@ -511,9 +511,9 @@ int default_geometry(int kind, int n_sections, int& B, int& N) {
 // differences (`sweep_kind`), for filters whose float32 error there is below the precision form's: it is
 // found by doing the sweep's arithmetic on the host, on noise and, where the filter passes it, an offset (within a
 // fifth of the device's error for 40 designs of orders 12 and 16), and the precision form's is 2.8e-7 to 7.4e-7 for all
-// of them. Nor may the sweep have to correct white noise (order 16 at 2^20 samples: 23 us, precision form 15). Orders 12 / 16 at 2^27
-// samples: direct 259 / 330 us, differences 291 / 357, precision form 443 / 399; at 2^20: 11 / 13, 12 / 14,
-// 15 / 15. Low passes up to half of the band qualify, the direct form from a cutoff of about 0.2 on;
+// of them. Nor may the sweep have to correct white noise (order 16 at 2^20 samples: 23 us, precision form 15). Orders 12
+// / 16 at 2^27 samples, cutoff 0.1: direct 280 / 343 us, differences 305 / 378, precision form 446 / 401; at 2^20: 12 /
+// 14, 12 / 14, 16 / 15. Low passes up to half of the band qualify, the direct form from a cutoff of about 0.2 on;
 // Chebyshev filters, high passes near zero and filters that do not decay within a tile do not.
 int resolve_auto(const std::vector<SectionF32>& secs, double gain, int& sweep_kind) {
     const int K = static_cast<int>(secs.size());

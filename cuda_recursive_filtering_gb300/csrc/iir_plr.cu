@@ -220,7 +220,7 @@ __global__ void __launch_bounds__(32 + BT) iir_plr_kernel(const __grid_constant_
 // A block holds one copy of the chunk's factors and W warps, which draw chunks until none is left; no
 // barrier after the start. Bound by issue and by the latency of a chunk's phases: 54 instructions per sample
 // (37 of them multiply-adds) at half of the issue slots. Measured at order 4 against a block per chunk (GB300,
-// graph replays, us): 3e6 samples 33.0 -> 16.1, 2^25 334 -> 94.8, 2^27 1320 -> 346.
+// graph replays, us): 3e6 samples 33.0 -> 16.1, 2^25 334 -> 95.3, 2^27 1320 -> 347.
 template <int X>
 struct PlrWarp {
     static constexpr int KO = 4, BT = 256, CHUNK = BT * X;

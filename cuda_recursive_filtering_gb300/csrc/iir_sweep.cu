@@ -4,7 +4,6 @@
 
 #include <algorithm>
 #include <cmath>
-#include <mutex>
 
 #include "iir_batch_sweep.h"
 #include "iir_sweep.h"
@@ -53,7 +52,8 @@ void add_sections(std::vector<SweepKernel>& v) {
     // Large signals: 16 KB tiles, two warps per scheduler (7, 9 or 10 warps leave the schedulers uneven
     // and 12 leave one buffer to load ahead: 5-10% slower), as many buffers as shared memory holds.
     // Four sub-rows per lane give pass B two independent chains; from 5 sections on the registers and
-    // the joins of four sub-rows cost more than that (order 16 at 2^27: 337 us with two, 395 with four).
+    // the joins of four sub-rows cost more than that (order 16 at 2^27, before the states were checked: 337 us with two, 395
+    // with four).
     if constexpr (K <= 4) add<K, 32, 4, 8, 13>(v);
     else add<K, 64, 2, 8, (K <= 6 ? 13 : 12)>(v);
     // Small signals: short lane rows, so that the signal spreads over more SMs. (Single sections have

@@ -25,14 +25,14 @@
 // measured either way). Pass A packs neighbouring samples (x and the tables come as pairs from
 // 16-byte loads), pass B two sub-rows.
 //
-// Bound by: memory up to 2 sections; above, by issue (27 instructions per sample at 4 sections, 17 of
-// them on the FMA pipe, which is 55% busy). Measured on GB300, butter(order, 0.1), CUDA graph replays,
-// against the kernels that this replaces (us, before -> after):
+// Bound by: memory up to 2 sections; above, by dependent steps at 2.2 warps per scheduler (28 instructions
+// per sample at 4 sections, 17.5 of them on the FMA pipe, which is 52% busy). Measured on GB300, butter(order,
+// 0.1), CUDA graph replays, against the kernels that this replaces (us, before -> after):
 //   order        2              4              8              16
-//   2^20     (small kernel kept) 8.8 -> 7.4   12.7 -> 8.9    21.0 -> 13.2
-//   2^23      18.2 -> 15.8   22.7 -> 16.9   31.4 -> 20.2   56.2 -> 34.4
-//   2^25      48.4 -> 44.4   59.3 -> 45.7   83.4 -> 51.5  152.1 -> 91.9
-//   2^27     163 -> 157.8   193 -> 158.2   284 -> 175.5   565 -> 333
+//   2^20     (small kernel kept) 8.5 -> 8.4   12.3 -> 9.9    20.6 -> 13.4
+//   2^23      14.3 -> 11.7   18.7 -> 14.1   27.0 -> 19.7   52.4 -> 31.5
+//   2^25      49.5 -> 45.3   59.9 -> 47.1   84.0 -> 57.5  153.3 -> 97.8
+//   2^27     163.7 -> 159.0  192.4 -> 159.5  284 -> 192    565 -> 344
 #pragma once
 #include "iir_pipe.cuh"
 
@@ -235,10 +235,10 @@ __device__ __forceinline__ void sweep_scan(const float* tab, int rounds, int lan
 // pass B, PH form: the cascade's own recurrences, sub-rows in packed pairs
 // ------------------------------------------------------------------------------------
 // Granules of 4 samples that go through the cascade together. More of them give longer diagonals (steps
-// that do not depend on one another) and more code; measured with 1 / 2 / 4: order 2 at 2^23 samples
-// 15.4 / 15.0 / 14.7 us, order 4 16.9 / 16.6 / 16.2; at 2^27 order 8 174.7 / 175.0 / 184.7, order 10
+// that do not depend on one another) and more code. Measured with 1 / 2 / 4 before the states were checked: order 2
+// at 2^23 samples 15.4 / 15.0 / 14.7 us, order 4 16.9 / 16.6 / 16.2; at 2^27 order 8 174.7 / 175.0 / 184.7, order 10
 // 237.5 / 234.3 / 230.6, order 12 259 / 267 / 273, order 16 330.7 / 329.8 / 330.7 (on differences 376 / 367
-// / 380). With the states checked, 1 / 2: order 16 at 2^25 96.8 / 100.1, on differences at 2^27 393 / 388.
+// / 380); and with that, 1 / 2: order 16 at 2^25 96.8 / 100.1, on differences at 2^27 393 / 388.
 __host__ __device__ constexpr int sweep_step_granules(int K, bool diff) {
     return K <= 2 || K == 5 ? 4 : K == 8 && diff ? 2 : 1;
 }
@@ -263,8 +263,8 @@ struct SweepSection {
 // full gain, 1 / A(z), which a low cutoff makes large; here the rounding of y[n] is the only one of y's own
 // size, and it meets (1 + sg a2 z^-1) / A(z), smaller by the pole's angle. Error against 64 bits (2-norm,
 // butter(16, .)): cutoff 0.05 3.0e-7 (direct form 1.11e-6, precision form 7.4e-7), 0.1 2.6e-7 (5.8e-7,
-// 6.5e-7), 0.4 3.0e-7 (2.3e-7, 5.3e-7). Time at 2^27 samples, cutoff 0.1, orders 12 / 16: 291 / 357 us
-// against 259 / 330 direct and 443 / 399 in the precision form.
+// 6.5e-7), 0.4 3.0e-7 (2.3e-7, 5.3e-7). Time at 2^27 samples, cutoff 0.1, orders 12 / 16: 305 / 378 us
+// against 280 / 343 direct and 446 / 401 in the precision form.
 template <class G, bool DIFF>
 __device__ __forceinline__ void sweep_run_ph(float* buf, const SweepSection* sec, float gain, int lane,
                                              const float (&st)[G::R][G::D], const float (&xh)[G::R][2],
@@ -401,7 +401,9 @@ __device__ __forceinline__ void sweep_run_ph(float* buf, const SweepSection* sec
 //     g[j+1] = Phi^N g[j] + r[j+1].
 // Where r stands out of the recurrence's own rounding, g is found by the same join and scan as the states, and
 // the response to g is added to the outputs (4K operations per sample). Elsewhere the check is all there is: about
-// 4% of a tile's instructions. Error against 64 bits, cheby1(16, 1, 0.3), noise and a tone 40 dB above it in
+// 4% of a tile's instructions (order 16: 49.9 -> 52.0 per sample) and 4 to 9% of the time from 4 sections on, the two
+// ends of tiles being read besides. A signal that has every tile corrected: order 8 97 us at 2^25 samples (57.5
+// otherwise; the lookback kernels 84 to 99). Error against 64 bits, cheby1(16, 1, 0.3), noise and a tone 40 dB above it in
 // the stop band: 2.0e-3 without, 2.7e-5 with (section by section, iir_ph.cuh: 3.1e-5).
 
 // Residuals r of the lane's sub-rows (r[i]: at its end), from pass B's end states, the states st that it started
@@ -596,9 +598,9 @@ struct SweepAux {
 //
 // Item i lies in buffer i % NB: the loader keeps NB - W items ahead of the warps. A warp gives its
 // buffer back when the store of its output has read it. From 3 sections on it waits for that at once,
-// so that the loads run further ahead (2^27, order 8: 177.9 -> 175.5 us, order 16: 345 -> 332.6); at 1 and
-// 2 sections, bound by memory, it looks after it during its next item (after pass A), or before it would
-// wait itself (order 4: 158.2 us, 158.7 at once).
+// so that the loads run further ahead (2^27, before the states were checked: order 8 177.9 -> 175.5 us, order 16
+// 345 -> 332.6); at 1 and 2 sections, bound by memory, it looks after it during its next item (after pass A), or
+// before it would wait itself (order 4: 158.2 us, 158.7 at once).
 template <class G, int W, int NB, class Run>
 __device__ __forceinline__ void sweep_tiles(const IirSweepParams& p, unsigned char* smem, Run&& run) {
     constexpr int SPAN = G::SPAN, R = G::R, K = G::K, D = G::D;
