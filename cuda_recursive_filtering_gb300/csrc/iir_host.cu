@@ -724,19 +724,22 @@ int plan_add_sweeps(iir_plan* p, const std::vector<SectionF32>& secs, double gai
     // (AUTO's choice from 6 sections on holds for every size)
     const bool chosen = p->n_sections >= SWEEP_DIFF_MIN_SECTIONS && automatic;
     std::vector<SweepPart> parts;
+    std::vector<std::vector<float>> tables;
     for (const SweepKernel* k : kernels) {
         SweepPart s;
         s.k = k;
         s.lanes = sweep_decay(f, k->span(), SWEEP_LANES);
-        if (s.lanes > 0) parts.push_back(s);
+        if (s.lanes == 0) continue;
+        parts.push_back(s);
+        tables.push_back(sweep_tables(f, k->N, k->R));
     }
     if (!chosen && p->n_sections >= 4 && !parts.empty()) {
-        const int N = parts.back().k->N;
-        if (sweep_trial(f, sweep_tables(f, N, parts.back().k->R), N, false, 24).residual > 0.7) return IIR_OK;
+        if (sweep_trial(f, tables.back(), parts.back().k->N, false, 24).residual > 0.7) return IIR_OK;
     }
-    for (SweepPart s : parts) {
+    for (size_t i = 0; i < parts.size(); ++i) {
+        SweepPart s = parts[i];
         const SweepKernel* k = s.k;
-        const std::vector<float> tab = sweep_tables(f, k->N, k->R);
+        const std::vector<float>& tab = tables[i];
         int st = cuda_status(
             cudaFuncSetAttribute(k->fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(k->smem)));
         if (!st) st = cuda_status(cudaFuncSetAttribute(k->fn, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
